@@ -70,7 +70,7 @@ struct Geometry {
     unsigned P = 0, R = 0, D = 0, NR = 0, L = 0, S = 0;
     std::vector<float2> shifts_f; // the reference's float shift grid
     std::vector<int2> shifts_i;   // truncated to int as the resample kernel receives them
-    std::vector<float2> tmpl;     // polar template [NR][L]
+    std::vector<float2> dirs;     // directions of a ring's sampling angles [L]
 };
 
 // Reference: generate_shift_array, cuda/gpu_aln_common.cu:64-86
@@ -88,20 +88,16 @@ std::vector<float2> shift_grid(float rx, float ry, float step)
     return v;
 }
 
-// Reference: generate_polar_sampling_points, cuda/gpu_aln_common.cu:39-62
-// (host libm, float products, same operation order)
-std::vector<float2> polar_template(unsigned ring_num, unsigned ring_len)
+// Directions (cosf, sinf) of a ring's sampling angles as
+// generate_polar_sampling_points forms them (cuda/gpu_aln_common.cu:39-62:
+// host libm); the kernels scale them to each ring's offsets (RingScale).
+std::vector<float2> polar_directions(unsigned ring_len)
 {
-    std::vector<float2> t((size_t)ring_num * ring_len);
-    for (unsigned i = 0; i < ring_num; i++)
-        for (unsigned j = 0; j < ring_len; j++) {
-            volatile float angle = (float)((double)((float)j / (float)ring_len) * 3.14159265358979 * 2);
-            volatile float cx = cosf(angle) * (float)(i + 1);
-            volatile float sy = sinf(angle) * (float)(i + 1);
-            volatile float ox = cx * (float)ring_num;
-            volatile float oy = sy * (float)ring_num;
-            t[(size_t)i * ring_len + j] = make_float2(ox / (float)ring_num, oy / (float)ring_num);
-        }
+    std::vector<float2> t(ring_len);
+    for (unsigned j = 0; j < ring_len; j++) {
+        volatile float angle = (float)((double)((float)j / (float)ring_len) * 3.14159265358979 * 2);
+        t[j] = make_float2(cosf(angle), sinf(angle));
+    }
     return t;
 }
 
@@ -149,7 +145,7 @@ int validate(const AlignConfig* cfg, Geometry& g, bool need_type, bool allow_l51
     g.shifts_i.resize(sf.size());
     for (size_t i = 0; i < sf.size(); i++)
         g.shifts_i[i] = make_int2((int)sf[i].x, (int)sf[i].y);
-    g.tmpl = polar_template(g.NR, g.L);
+    g.dirs = polar_directions(g.L);
     return 0;
 }
 
@@ -225,7 +221,7 @@ struct Workspace {
     // geometry currently uploaded (skip re-uploading an unchanged one)
     unsigned geo_D = 0, geo_NR = 0, geo_L = 0;
     std::vector<float2> geo_shifts;
-    DevBuf<float2> tmpl, tw, tw512, shifts_f, ref_sp, sbj_sp, base;
+    DevBuf<float2> dirs, tw, tw512, shifts_f, ref_sp, sbj_sp, base;
     DevBuf<int2> shifts_i, zero_shift;
     DevBuf<unsigned> err; // device-side timeout flag of the kernels' bounded waits
     DevBuf<unsigned char> sop, rop; // BF16 hi/lo operands of the tensor-core contraction
@@ -274,7 +270,7 @@ struct Workspace {
         geo_D = geo_NR = geo_L = 0;
         geo_shifts.clear();
         zero_shift.release();
-        tmpl.release();
+        dirs.release();
         tw.release();
         tw512.release();
         shifts_f.release();
@@ -299,16 +295,16 @@ std::vector<float2> twiddles(int n = kRingLen)
 int upload_geometry(const Geometry& g, Workspace& ws, cudaStream_t st)
 {
     if (ws.geo_D == g.D && ws.geo_NR == g.NR && ws.geo_L == g.L && ws.geo_shifts.size() == g.shifts_f.size() &&
-        ws.tmpl.p && std::memcmp(ws.geo_shifts.data(), g.shifts_f.data(), g.shifts_f.size() * sizeof(float2)) == 0)
+        ws.dirs.p && std::memcmp(ws.geo_shifts.data(), g.shifts_f.data(), g.shifts_f.size() * sizeof(float2)) == 0)
         return 0;
-    if (ws.tmpl.ensure(g.tmpl.size()) || ws.tw.ensure(kRingLen) || ws.tw512.ensure(kRingLen512) ||
+    if (ws.dirs.ensure(g.dirs.size()) || ws.tw.ensure(kRingLen) || ws.tw512.ensure(kRingLen512) ||
         ws.shifts_f.ensure(g.S) || ws.shifts_i.ensure(g.S) || ws.zero_shift.ensure(1))
         return E_NOMEM;
     std::vector<float2> tw = twiddles(), tw512 = twiddles(kRingLen512);
     CK(cudaMemcpyAsync(ws.tw512.p, tw512.data(), tw512.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
     const int2 zero = make_int2(0, 0);
     CK(cudaMemcpyAsync(ws.zero_shift.p, &zero, sizeof(int2), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(ws.tmpl.p, g.tmpl.data(), g.tmpl.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(ws.dirs.p, g.dirs.data(), g.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(ws.tw.p, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(ws.shifts_f.p, g.shifts_f.data(), g.S * sizeof(float2), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(ws.shifts_i.p, g.shifts_i.data(), g.S * sizeof(int2), cudaMemcpyHostToDevice, st));
@@ -488,7 +484,7 @@ int run_alignment_split(const Geometry& g, Workspace& ws, const StackDesc& refs,
     CK(cudaStreamWaitEvent(hi, ws.split_entry, 0));
     CK(cudaStreamWaitEvent(lo, ws.split_entry, 0));
     cudaEvent_t ev = g_timer.begin(hi);
-    CK(launch_polar_operands(refs, ws.tmpl.p, ws.tw.p, g.NR, ws.zero_shift.p, 1, nullptr, 0, g.R, 1,
+    CK(launch_polar_operands(refs, ws.dirs.p, ws.tw.p, g.NR, ws.zero_shift.p, 1, nullptr, 0, g.R, 1,
                              split_ref_layout(pl, ws.rop.p), hi, ref_tx));
     g_timer.end(K_SPECTRA, ev, hi);
     // particle chunk: two operand buffers and the pair spectra of a particle
@@ -522,7 +518,7 @@ int run_alignment_split(const Geometry& g, Workspace& ws, const StackDesc& refs,
         if (c >= 2)
             CK(cudaStreamWaitEvent(lo, ws.mma_done[buf], 0));
         ev = g_timer.begin(lo);
-        CK(launch_polar_operands(sbjs, ws.tmpl.p, ws.tw.p, g.NR, ws.shifts_i.p, g.S, d_base, p0, n, 0,
+        CK(launch_polar_operands(sbjs, ws.dirs.p, ws.tw.p, g.NR, ws.shifts_i.p, g.S, d_base, p0, n, 0,
                                  split_sbj_layout(pl, sop), lo, sbj_tx));
         g_timer.end(K_SPECTRA, ev, lo);
         CK(cudaEventRecord(ws.ops_done[buf], lo));
@@ -570,7 +566,7 @@ int run_alignment_l512(const Geometry& g, Workspace& ws, const StackDesc& refs, 
     if (ws.ref_sp.ensure(row_elems * std::max(g.R, 1u)))
         return E_NOMEM;
     cudaEvent_t ev = g_timer.begin(st);
-    CK(launch_polar_spectra512(refs, ws.tmpl.p, ws.tw512.p, g.NR, ws.zero_shift.p, 1, nullptr, 0, g.R, 1,
+    CK(launch_polar_spectra512(refs, ws.dirs.p, ws.tw512.p, g.NR, ws.zero_shift.p, 1, nullptr, 0, g.R, 1,
                                ws.ref_sp.p, st, ref_tx));
     g_timer.end(K_SPECTRA, ev, st);
     size_t free_b = 0, total_b = 0;
@@ -584,7 +580,7 @@ int run_alignment_l512(const Geometry& g, Workspace& ws, const StackDesc& refs, 
     for (unsigned p0 = 0; p0 < g.P; p0 += (unsigned)chunk) {
         const unsigned n = (unsigned)std::min<size_t>(chunk, g.P - p0);
         ev = g_timer.begin(st);
-        CK(launch_polar_spectra512(sbjs, ws.tmpl.p, ws.tw512.p, g.NR, ws.shifts_i.p, g.S, d_base, p0, n, 0,
+        CK(launch_polar_spectra512(sbjs, ws.dirs.p, ws.tw512.p, g.NR, ws.shifts_i.p, g.S, d_base, p0, n, 0,
                                    ws.sbj_sp.p, st, sbj_tx));
         g_timer.end(K_SPECTRA, ev, st);
         ev = g_timer.begin(st);
@@ -633,7 +629,7 @@ int run_alignment(const AlignConfig* cfg, const Geometry& g, Workspace& ws, cons
     if (ws.ref_sp.ensure(row_elems * std::max(g.R, 1u)))
         return E_NOMEM;
     cudaEvent_t ev = g_timer.begin(st);
-    CK(launch_polar_spectra(refs, ws.tmpl.p, ws.tw.p, g.NR, ws.zero_shift.p, 1, nullptr, 0,
+    CK(launch_polar_spectra(refs, ws.dirs.p, ws.tw.p, g.NR, ws.zero_shift.p, 1, nullptr, 0,
                             g.R, 1, ws.ref_sp.p, st, nullptr, ref_tx));
     g_timer.end(K_SPECTRA, ev, st);
 
@@ -675,7 +671,7 @@ int run_alignment(const AlignConfig* cfg, const Geometry& g, Workspace& ws, cons
     for (unsigned p0 = 0; p0 < g.P; p0 += (unsigned)chunk) {
         unsigned n = (unsigned)std::min<size_t>(chunk, g.P - p0);
         ev = g_timer.begin(st);
-        CK(launch_polar_spectra(sbjs, ws.tmpl.p, ws.tw.p, g.NR, ws.shifts_i.p, g.S, d_base, p0, n, 0, ws.sbj_sp.p,
+        CK(launch_polar_spectra(sbjs, ws.dirs.p, ws.tw.p, g.NR, ws.shifts_i.p, g.S, d_base, p0, n, 0, ws.sbj_sp.p,
                                 st, nullptr, sbj_tx));
         g_timer.end(K_SPECTRA, ev, st);
         ev = g_timer.begin(st);
@@ -839,7 +835,7 @@ int host_geometry(const AlignConfig* cfg, HostGeometry& out)
     out.S = g.S;
     out.shifts_f = g.shifts_f;
     out.shifts_i = g.shifts_i;
-    out.tmpl = g.tmpl;
+    out.dirs = g.dirs;
     out.tw = twiddles();
     out.sbj_batch = std::max(1u, reference_sbj_batch(cfg));
     return 0;
@@ -1062,7 +1058,7 @@ int gpuisac_spectra_device_layout(const AlignConfig* cfg, const float* imgs, uns
     const unsigned long long* tx = nullptr;
     if (texture_unit_enabled() && n_img > 0)
         tx = ws.sbj_tex.try_build(sd, st);
-    CK(launch_polar_spectra(sd, ws.tmpl.p, ws.tw.p, g.NR, is_ref ? ws.zero_shift.p : ws.shifts_i.p, is_ref ? 1 : g.S,
+    CK(launch_polar_spectra(sd, ws.dirs.p, ws.tw.p, g.NR, is_ref ? ws.zero_shift.p : ws.shifts_i.p, is_ref ? 1 : g.S,
                             reinterpret_cast<const float2*>(base_shift), 0, n_img, is_ref,
                             reinterpret_cast<float2*>(out), st, nullptr, tx));
     CK(cudaStreamSynchronize(st));

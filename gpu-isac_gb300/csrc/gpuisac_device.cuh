@@ -63,6 +63,12 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+// the same product with its rounding written out (the compiler is free in
+// which of a sum's two products it fuses)
+__device__ __forceinline__ float2 cmul_fixed(float2 a, float2 b)
+{
+    return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
 // multiply by +i (SIGN>0) or -i (SIGN<0)
 template <int SIGN>
 __device__ __forceinline__ float2 cmul_i(float2 a)
@@ -177,14 +183,14 @@ __device__ __forceinline__ void fft256_group(float2 (&x)[16], float2* ws, const 
 // with the sign of SIGN), read at fixed offsets instead of through (l j) & 255.
 // Rows of 17 float2 keep the 16 threads of a group on distinct banks.
 constexpr int kTwRow = 17;
-template <int SIGN>
+template <int SIGN, bool kPacked = true>
 __device__ __forceinline__ void fft256_group_twl(float2 (&x)[16], float2* ws, const float2* twl, unsigned mask)
 {
     const int l = threadIdx.x & 15;
-    dft16<SIGN>(x);
+    dft16<SIGN, kPacked>(x);
 #pragma unroll
     for (int j = 1; j < 16; j++)
-        x[perm16(j)] = cmul(x[perm16(j)], twl[j]);
+        x[perm16(j)] = SIGN < 0 ? cmul_fixed(x[perm16(j)], twl[j]) : cmul(x[perm16(j)], twl[j]);
     __syncwarp(mask);
 #pragma unroll
     for (int j = 0; j < 16; j++)
@@ -194,8 +200,41 @@ __device__ __forceinline__ void fft256_group_twl(float2 (&x)[16], float2* ws, co
     for (int n = 0; n < 16; n++)
         x[n] = ws[n * 17 + l];
     __syncwarp(mask);
-    dft16<SIGN>(x);
+    dft16<SIGN, kPacked>(x);
 }
+
+// ---------------------------------------------------------------------------
+// Polar sampling offsets.  The reference's template
+// (generate_polar_sampling_points, cuda/gpu_aln_common.cu:39-62) holds, for
+// ring radius R and direction (c, s) = (cosf, sinf) of the sample's angle,
+// ((c R) N) / N and ((s R) N) / N in float, N the ring count.  The kernels
+// keep only the directions in memory and redo the float operations: at 8
+// bytes a sample the template was the larger part of what the spectra kernels
+// fetched from L2 (71 KB a row at 35 rings, nearly none of it held by the L1
+// that the shared memory leaves), and its latency came before the texture's.
+// The division by N is Markstein's (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990): with y = RN(1 / N)
+// and q0 = RN(m y), the remainder e = m - q0 N is exact in an FMA and
+// RN(q0 + e y) is the correctly rounded m / N -- checked for every 24-bit m
+// and every N up to the largest ring count (tests/test_ring_offsets.py holds
+// the template's own values).
+struct RingScale {
+    float2 n, neg_n, y; // (N, N), (-N, -N), (RN(1 / N), RN(1 / N))
+    __device__ __forceinline__ explicit RingScale(unsigned ring_num)
+    {
+        const float f = (float)ring_num, r = __frcp_rn(f);
+        n = make_float2(f, f);
+        neg_n = make_float2(-f, -f);
+        y = make_float2(r, r);
+    }
+    // offset of the sample in direction dir at radius R = (R, R)
+    __device__ __forceinline__ float2 offset(float2 dir, float radius) const
+    {
+        const float2 m = __fmul2_rn(__fmul2_rn(dir, make_float2(radius, radius)), n);
+        const float2 q0 = __fmul2_rn(m, y);
+        return __ffma2_rn(__ffma2_rn(q0, neg_n, m), y, q0);
+    }
+};
 
 // ---------------------------------------------------------------------------
 // Stacked image arrays read the way the reference's 2D textures are read

@@ -16,7 +16,7 @@ constexpr unsigned kMaxShifts = 4096;   // shift grid entries supported
 
 inline size_t polar_spectra_smem_bytes(unsigned ring_num)
 {
-    return (size_t)((ring_num + 1) / 2) * kPairStride * sizeof(float2) + kRingLen * sizeof(float2) +
+    return (size_t)((ring_num + 1) / 2) * kPairStride * sizeof(float2) + 16 * kTwRow * sizeof(float2) +
            24 * sizeof(double);
 }
 
@@ -112,7 +112,7 @@ bool texture_unit_enabled();
 // when a list is given.  out: [n_img][n_shift][ring_num][kSlots] float2
 // (see polar_spectra.cu).  tex_objs: texture objects of st built by a
 // TexStack (samples through the texture unit), or null (the emulation).
-cudaError_t launch_polar_spectra(const StackDesc& st, const float2* tmpl, const float2* twiddle,
+cudaError_t launch_polar_spectra(const StackDesc& st, const float2* dirs, const float2* twiddle,
                                  unsigned ring_num, const int2* shift_int, unsigned n_shift,
                                  const float2* base, unsigned img0, unsigned n_img, int is_ref,
                                  float2* out, cudaStream_t stream, const unsigned* img_list = nullptr,
@@ -137,10 +137,11 @@ struct SpectraJob {
 // per block of kJobLutRows rows, the index of the job holding the block's
 // first row.  One CTA per row: `grid` must cover the rows (CTAs past them
 // return); the same launch serves any table the device buffers hold.
+// textures: whether every job has texture objects.
 constexpr unsigned kJobLutRows = 32;
 cudaError_t launch_polar_spectra_jobs(const SpectraJob* jobs, const unsigned* hdr, const unsigned* lut,
-                                      const float2* tmpl, const float2* twiddle, unsigned ring_num, unsigned grid,
-                                      cudaStream_t stream);
+                                      const float2* dirs, const float2* twiddle, unsigned ring_num, unsigned grid,
+                                      cudaStream_t stream, bool textures);
 
 // ---------------------------------------------------------------------------
 // Rings of 512 samples (ring512.cu): spectra rows [ring][kSlots512] float2 in
@@ -148,7 +149,7 @@ cudaError_t launch_polar_spectra_jobs(const SpectraJob* jobs, const unsigned* hd
 // inverse-FFT / peak search over them; tw512[e] = e^(-2 pi i e / 512).
 constexpr int kRingLen512 = 512;
 constexpr int kSlots512 = kRingLen512 / 2;
-cudaError_t launch_polar_spectra512(const StackDesc& st, const float2* tmpl, const float2* tw512, unsigned ring_num,
+cudaError_t launch_polar_spectra512(const StackDesc& st, const float2* dirs, const float2* tw512, unsigned ring_num,
                                     const int2* shift_int, unsigned n_shift, const float2* base, unsigned img0,
                                     unsigned n_img, int is_ref, float2* out, cudaStream_t stream,
                                     const unsigned long long* tex_objs);
@@ -188,7 +189,7 @@ struct OperandLayout {
 // set): subjects (is_ref = 0) as rows of particle tiles, references (is_ref)
 // as rows of reference tiles; the spectra values are those
 // launch_polar_spectra writes, bit for bit, before the split.
-cudaError_t launch_polar_operands(const StackDesc& st, const float2* tmpl, const float2* twiddle,
+cudaError_t launch_polar_operands(const StackDesc& st, const float2* dirs, const float2* twiddle,
                                   unsigned ring_num, const int2* shift_int, unsigned n_shift,
                                   const float2* base, unsigned img0, unsigned n_img, int is_ref,
                                   const OperandLayout& opnd, cudaStream_t stream,

@@ -137,7 +137,7 @@ struct Rec {
 
 struct GroupState {
     std::mutex mu;
-    Buf<float2> tw, tmpl, shifts_f, ref_sp, sbj_sp;
+    Buf<float2> tw, dirs, shifts_f, ref_sp, sbj_sp;
     Buf<int2> shifts_i, zero;
     Buf<unsigned char> tables;
     Buf<unsigned> err;
@@ -295,7 +295,7 @@ extern "C" int gpuisac_multi_ref_align_groups_device(const AlignConfig* cfg, con
     G_CK(S.sbj_sp.ensure(row_elems * Sn * max_rows));
     G_CK(S.ref_sp.ensure(row_elems * ref_rows));
     G_CK(S.tw.ensure(kRingLen));
-    G_CK(S.tmpl.ensure(geo.tmpl.size()));
+    G_CK(S.dirs.ensure(geo.dirs.size()));
     G_CK(S.shifts_f.ensure(Sn));
     G_CK(S.shifts_i.ensure(Sn));
     G_CK(S.zero.ensure(1));
@@ -429,7 +429,7 @@ extern "C" int gpuisac_multi_ref_align_groups_device(const AlignConfig* cfg, con
         h[6] = lut_first;
     }
     G_CK(cudaMemcpy(S.tw.p, geo.tw.data(), kRingLen * sizeof(float2), cudaMemcpyHostToDevice));
-    G_CK(cudaMemcpy(S.tmpl.p, geo.tmpl.data(), geo.tmpl.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    G_CK(cudaMemcpy(S.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice));
     G_CK(cudaMemcpy(S.shifts_f.p, geo.shifts_f.data(), Sn * sizeof(float2), cudaMemcpyHostToDevice));
     G_CK(cudaMemcpy(S.shifts_i.p, geo.shifts_i.data(), Sn * sizeof(int2), cudaMemcpyHostToDevice));
     const int2 zero = make_int2(0, 0);
@@ -442,7 +442,7 @@ extern "C" int gpuisac_multi_ref_align_groups_device(const AlignConfig* cfg, con
     const unsigned spec_grid = caps.rows;
     const unsigned fill_grid = (unsigned)std::max(1, sms) * 8;
     std::vector<unsigned char> key;
-    const void* ptrs[9] = {dt, S.tw.p, S.tmpl.p, S.shifts_f.p, S.shifts_i.p, S.zero.p, S.err.p, nullptr, nullptr};
+    const void* ptrs[9] = {dt, S.tw.p, S.dirs.p, S.shifts_f.p, S.shifts_i.p, S.zero.p, S.err.p, nullptr, nullptr};
     append(key, ptrs, sizeof(ptrs));
     const unsigned shape[8] = {(unsigned)dev, NR, Sn, W, caps.waves, spec_grid, hw ? 1u : 0u, ccf_tile_generation()};
     append(key, shape, sizeof(shape));
@@ -463,8 +463,8 @@ extern "C" int gpuisac_multi_ref_align_groups_device(const AlignConfig* cfg, con
                                      fill_grid, cap);
         for (unsigned w = 0; w < W && e == cudaSuccess; w++) {
             e = launch_polar_spectra_jobs(reinterpret_cast<const SpectraJob*>(dt + L.jobs), d_hdr + kHdrWave * w + 3,
-                                          reinterpret_cast<const unsigned*>(dt + L.luts), S.tmpl.p, S.tw.p, NR,
-                                          spec_grid, cap);
+                                          reinterpret_cast<const unsigned*>(dt + L.luts), S.dirs.p, S.tw.p, NR,
+                                          spec_grid, cap, hw);
             if (e != cudaSuccess)
                 break;
             CcfWork cw{};

@@ -29,7 +29,7 @@ struct HostGeometry {
     unsigned P = 0, R = 0, D = 0, NR = 0, S = 0;
     std::vector<float2> shifts_f; // the reference's float shift grid
     std::vector<int2> shifts_i;   // truncated to int, as the resample kernel receives them
-    std::vector<float2> tmpl;     // polar template [NR][256]
+    std::vector<float2> dirs;     // directions (cosf, sinf) of a ring's 256 sampling angles
     std::vector<float2> tw;       // e^(-2 pi i e / 256), e = 0..255
     unsigned sbj_batch = 1;       // the reference's subject batch size
 };

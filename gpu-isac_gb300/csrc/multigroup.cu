@@ -235,7 +235,7 @@ struct MgState {
     AlignParam* params = nullptr; // host memory the caller reads and writes
     std::vector<unsigned> cid_idx;
     DBuf<float> sbj, ref, d;
-    DBuf<float2> tw, tmpl, shifts_f, ref_sp, sbj_sp, base, ftw, fscratch;
+    DBuf<float2> tw, dirs, shifts_f, ref_sp, sbj_sp, base, ftw, fscratch;
     DBuf<int2> shifts_i, zero;
     DBuf<float4> peak;
     TexStack sbj_tex, ref_tex; // the particles (built at init) and the averages (each iteration)
@@ -254,7 +254,7 @@ void clear_mg(MgState& s)
     s.ref.release();
     s.d.release();
     s.tw.release();
-    s.tmpl.release();
+    s.dirs.release();
     s.shifts_f.release();
     s.ref_sp.release();
     s.sbj_sp.release();
@@ -334,7 +334,7 @@ int run_iteration(MgState& s)
     const unsigned long long* sbj_tx = nullptr;
     if (hw)
         sbj_tx = s.sbj_tex.objects() ? s.sbj_tex.objects() : s.sbj_tex.try_build(sbjs, st);
-    MG_CK(launch_polar_spectra(refs, s.tmpl.p, s.tw.p, NR, s.zero.p, 1, nullptr, 0, R, 1, s.ref_sp.p, st, nullptr,
+    MG_CK(launch_polar_spectra(refs, s.dirs.p, s.tw.p, NR, s.zero.p, 1, nullptr, 0, R, 1, s.ref_sp.p, st, nullptr,
                                ref_tx));
 
     // base shifts: the particles' accumulated shifts
@@ -395,7 +395,7 @@ int run_iteration(MgState& s)
                           cudaMemcpyHostToDevice, st));
 
     for (const ChunkWork& cw : work) {
-        MG_CK(launch_polar_spectra(sbjs, s.tmpl.p, s.tw.p, NR, s.shifts_i.p, S, s.base.p, cw.c0, cw.c, 0, s.sbj_sp.p,
+        MG_CK(launch_polar_spectra(sbjs, s.dirs.p, s.tw.p, NR, s.shifts_i.p, S, s.base.p, cw.c0, cw.c, 0, s.sbj_sp.p,
                                    st, nullptr, sbj_tx));
         CcfWork w{};
         w.groups = s.table.p + cw.first;
@@ -591,12 +591,12 @@ AlignParam* ref_free_alignment_2D_init(const AlignConfig* aln_cfg, const float**
     const int2 zero = make_int2(0, 0);
     bool ok = s.sbj.ensure((size_t)s.P * img) == cudaSuccess && s.ref.ensure((size_t)s.R * img) == cudaSuccess &&
               s.d.ensure(s.P) == cudaSuccess && s.tw.ensure(kRingLen) == cudaSuccess &&
-              s.tmpl.ensure(geo.tmpl.size()) == cudaSuccess && s.ref_sp.ensure((size_t)s.R * row) == cudaSuccess &&
+              s.dirs.ensure(geo.dirs.size()) == cudaSuccess && s.ref_sp.ensure((size_t)s.R * row) == cudaSuccess &&
               s.base.ensure(s.P) == cudaSuccess && s.zero.ensure(1) == cudaSuccess &&
               s.peak.ensure(s.P) == cudaSuccess && s.err.ensure(2) == cudaSuccess &&
               s.cid.ensure(s.R + 1) == cudaSuccess && s.xf.ensure(s.P) == cudaSuccess;
     ok = ok && cudaMemcpy(s.tw.p, geo.tw.data(), kRingLen * sizeof(float2), cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemcpy(s.tmpl.p, geo.tmpl.data(), geo.tmpl.size() * sizeof(float2), cudaMemcpyHostToDevice) ==
+         cudaMemcpy(s.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice) ==
              cudaSuccess &&
          cudaMemcpy(s.zero.p, &zero, sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemcpy(s.cid.p, cid_idx.data(), (s.R + 1) * sizeof(unsigned), cudaMemcpyHostToDevice) == cudaSuccess;

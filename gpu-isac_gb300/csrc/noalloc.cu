@@ -62,7 +62,7 @@ namespace {
 // the array carved for one call: tables, reference spectra, then as many
 // particles' spectra as fit
 struct Carve {
-    size_t off_err, off_tw, off_zero, off_tmpl, off_sf, off_si, off_ref, off_sbj, per_particle, need;
+    size_t off_err, off_tw, off_zero, off_dirs, off_sf, off_si, off_ref, off_sbj, per_particle, need;
     unsigned chunk;
 };
 
@@ -73,8 +73,8 @@ Carve carve(const HostGeometry& g)
     c.off_err = 0;
     c.off_tw = c.off_err + 256;
     c.off_zero = c.off_tw + up256(kRingLen * sizeof(float2));
-    c.off_tmpl = c.off_zero + up256(sizeof(int2));
-    c.off_sf = c.off_tmpl + up256(g.tmpl.size() * sizeof(float2));
+    c.off_dirs = c.off_zero + up256(sizeof(int2));
+    c.off_sf = c.off_dirs + up256((size_t)g.NR * kRingLen * sizeof(float2));
     c.off_si = c.off_sf + up256((size_t)g.S * sizeof(float2));
     c.off_ref = c.off_si + up256((size_t)g.S * sizeof(int2));
     c.off_sbj = c.off_ref + up256((size_t)g.R * row_bytes);
@@ -150,7 +150,7 @@ int enqueue_and_wait(const HostGeometry& g, const Carve& c, unsigned char* base,
     unsigned* err = reinterpret_cast<unsigned*>(base + c.off_err);
     float2* tw = reinterpret_cast<float2*>(base + c.off_tw);
     int2* zero = reinterpret_cast<int2*>(base + c.off_zero);
-    float2* tmpl = reinterpret_cast<float2*>(base + c.off_tmpl);
+    float2* dirs = reinterpret_cast<float2*>(base + c.off_dirs);
     float2* sf = reinterpret_cast<float2*>(base + c.off_sf);
     int2* si = reinterpret_cast<int2*>(base + c.off_si);
     float2* ref_sp = reinterpret_cast<float2*>(base + c.off_ref);
@@ -160,7 +160,7 @@ int enqueue_and_wait(const HostGeometry& g, const Carve& c, unsigned char* base,
     NA_CK(cudaMemsetAsync(err, 0, sizeof(unsigned), st));
     NA_CK(cudaMemcpyAsync(tw, g.tw.data(), kRingLen * sizeof(float2), cudaMemcpyHostToDevice, st));
     NA_CK(cudaMemcpyAsync(zero, &zero_h, sizeof(int2), cudaMemcpyHostToDevice, st));
-    NA_CK(cudaMemcpyAsync(tmpl, g.tmpl.data(), g.tmpl.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
+    NA_CK(cudaMemcpyAsync(dirs, g.dirs.data(), g.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice, st));
     NA_CK(cudaMemcpyAsync(sf, g.shifts_f.data(), g.S * sizeof(float2), cudaMemcpyHostToDevice, st));
     NA_CK(cudaMemcpyAsync(si, g.shifts_i.data(), g.S * sizeof(int2), cudaMemcpyHostToDevice, st));
 
@@ -171,10 +171,10 @@ int enqueue_and_wait(const HostGeometry& g, const Carve& c, unsigned char* base,
     StackDesc refs{ref, g.R, g.D, ref_batch, tex};
     StackDesc sbjs{sbj, g.P, g.D, g.sbj_batch, tex};
     const float2* bs = reinterpret_cast<const float2*>(base_shift);
-    NA_CK(launch_polar_spectra(refs, tmpl, tw, g.NR, zero, 1, nullptr, 0, g.R, 1, ref_sp, st));
+    NA_CK(launch_polar_spectra(refs, dirs, tw, g.NR, zero, 1, nullptr, 0, g.R, 1, ref_sp, st));
     for (unsigned p0 = 0; p0 < g.P; p0 += chunk) {
         const unsigned n = std::min(chunk, g.P - p0);
-        NA_CK(launch_polar_spectra(sbjs, tmpl, tw, g.NR, si, g.S, bs, p0, n, 0, sbj_sp, st));
+        NA_CK(launch_polar_spectra(sbjs, dirs, tw, g.NR, si, g.S, bs, p0, n, 0, sbj_sp, st));
         NA_CK(launch_ccf_peak(sbj_sp, ref_sp, tw, g.NR, g.S, g.R, n, p0, g.P, sf, bs, d_out,
                               reinterpret_cast<float4*>(peak_out), err, st));
     }

@@ -75,7 +75,7 @@ struct PreState {
     HostGeometry geo;
     AlignParam* params = nullptr; // host memory the caller reads and writes
     DBuf<float> sbj, ref;
-    DBuf<float2> tw, tmpl, shifts_f, ref_sp, sbj_sp, base;
+    DBuf<float2> tw, dirs, shifts_f, ref_sp, sbj_sp, base;
     DBuf<int2> shifts_i, zero;
     DBuf<float> d;
     DBuf<float4> peak;
@@ -90,7 +90,7 @@ void clear_pre(PreState& s)
     s.sbj.release();
     s.ref.release();
     s.tw.release();
-    s.tmpl.release();
+    s.dirs.release();
     s.shifts_f.release();
     s.ref_sp.release();
     s.sbj_sp.release();
@@ -238,14 +238,14 @@ AlignParam* pre_align_init(unsigned int num_particles, const AlignConfig* aln_cf
     const size_t img = (size_t)geo.D * geo.D;
     const int2 zero = make_int2(0, 0);
     bool ok = s.sbj.ensure((size_t)s.capacity * img) == cudaSuccess && s.ref.ensure(img) == cudaSuccess &&
-              s.tw.ensure(kRingLen) == cudaSuccess && s.tmpl.ensure(geo.tmpl.size()) == cudaSuccess &&
+              s.tw.ensure(kRingLen) == cudaSuccess && s.dirs.ensure(geo.dirs.size()) == cudaSuccess &&
               s.zero.ensure(1) == cudaSuccess && s.err.ensure(2) == cudaSuccess &&
               s.ref_sp.ensure((size_t)geo.NR * kSlots) == cudaSuccess;
     // slots never fetched read as zero (the reference leaves them undefined)
     ok = ok && cudaMemset(s.sbj.p, 0, (size_t)s.capacity * img * sizeof(float)) == cudaSuccess &&
          cudaMemset(s.ref.p, 0, img * sizeof(float)) == cudaSuccess &&
          cudaMemcpy(s.tw.p, geo.tw.data(), kRingLen * sizeof(float2), cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemcpy(s.tmpl.p, geo.tmpl.data(), geo.tmpl.size() * sizeof(float2), cudaMemcpyHostToDevice) ==
+         cudaMemcpy(s.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice) ==
              cudaSuccess &&
          cudaMemcpy(s.zero.p, &zero, sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess;
     if (!ok || upload_shift_tables(s)) {
@@ -314,7 +314,7 @@ void pre_align_run(int start_idx, int stop_idx)
         PRE_CK(cudaMemsetAsync(s.err.p, 0, sizeof(unsigned), st));
         // the reference at zero shift (reference basis, ring weights folded in)
         StackDesc refs{s.ref.p, 1, g.D, 1, tex};
-        PRE_CK(launch_polar_spectra(refs, s.tmpl.p, s.tw.p, g.NR, s.zero.p, 1, nullptr, 0, 1, 1, s.ref_sp.p, st));
+        PRE_CK(launch_polar_spectra(refs, s.dirs.p, s.tw.p, g.NR, s.zero.p, 1, nullptr, 0, 1, 1, s.ref_sp.p, st));
         // base shifts: the particles' accumulated shifts, by stack slot
         s.h_base.resize(n);
         for (unsigned i = 0; i < n; i++)
@@ -335,7 +335,7 @@ void pre_align_run(int start_idx, int stop_idx)
             sbj_tx = s.sbj_tex.try_build(sbjs, st);
         for (unsigned c0 = 0; c0 < n; c0 += chunk) {
             const unsigned c = std::min(chunk, n - c0);
-            PRE_CK(launch_polar_spectra(sbjs, s.tmpl.p, s.tw.p, g.NR, s.shifts_i.p, g.S, s.base.p, c0, c, 0,
+            PRE_CK(launch_polar_spectra(sbjs, s.dirs.p, s.tw.p, g.NR, s.shifts_i.p, g.S, s.base.p, c0, c, 0,
                                         s.sbj_sp.p, st, nullptr, sbj_tx));
             PRE_CK(launch_ccf_peak(s.sbj_sp.p, s.ref_sp.p, s.tw.p, g.NR, g.S, 1, c, c0, n, s.shifts_f.p, s.base.p,
                                    s.d.p, s.peak.p, s.err.p, st, kPeakPreAlign, s.err.p + 1));

@@ -61,7 +61,7 @@ struct Buf {
 
 struct PropState {
     std::mutex mu;
-    Buf<float2> tw, tmpl, shifts_f, ref_sp, sbj_sp;
+    Buf<float2> tw, dirs, shifts_f, ref_sp, sbj_sp;
     Buf<int2> shifts_i, zero;
     Buf<CcfGroup> table;
     Buf<unsigned> err, sel;
@@ -99,7 +99,7 @@ extern "C" int gpuisac_align_proposals_device(const AlignConfig* cfg, const floa
     const unsigned qt = ccf_refs_per_item(NR, variant);
 
     P_CK(S.tw.ensure(kRingLen));
-    P_CK(S.tmpl.ensure(geo.tmpl.size()));
+    P_CK(S.dirs.ensure(geo.dirs.size()));
     P_CK(S.shifts_f.ensure(Sn));
     P_CK(S.shifts_i.ensure(Sn));
     P_CK(S.zero.ensure(1));
@@ -108,7 +108,7 @@ extern "C" int gpuisac_align_proposals_device(const AlignConfig* cfg, const floa
     P_CK(S.table.ensure(n_sel));
     const int2 zero = make_int2(0, 0);
     P_CK(cudaMemcpy(S.tw.p, geo.tw.data(), kRingLen * sizeof(float2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.tmpl.p, geo.tmpl.data(), geo.tmpl.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    P_CK(cudaMemcpy(S.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice));
     P_CK(cudaMemcpy(S.shifts_f.p, geo.shifts_f.data(), Sn * sizeof(float2), cudaMemcpyHostToDevice));
     P_CK(cudaMemcpy(S.shifts_i.p, geo.shifts_i.data(), Sn * sizeof(int2), cudaMemcpyHostToDevice));
     P_CK(cudaMemcpy(S.zero.p, &zero, sizeof(int2), cudaMemcpyHostToDevice));
@@ -140,7 +140,7 @@ extern "C" int gpuisac_align_proposals_device(const AlignConfig* cfg, const floa
     const unsigned long long *ref_tx = nullptr, *sbj_tx = nullptr;
     if (texture_unit_enabled())
         ref_tx = S.ref_tex.try_build(refs, st);
-    P_CK(launch_polar_spectra(refs, S.tmpl.p, S.tw.p, NR, S.zero.p, 1, nullptr, 0, geo.R, 1, S.ref_sp.p, st, nullptr,
+    P_CK(launch_polar_spectra(refs, S.dirs.p, S.tw.p, NR, S.zero.p, 1, nullptr, 0, geo.R, 1, S.ref_sp.p, st, nullptr,
                               ref_tx));
 
     // one group per selected particle: 1 particle x its k references
@@ -177,7 +177,7 @@ extern "C" int gpuisac_align_proposals_device(const AlignConfig* cfg, const floa
             table[c0 + i] = g;
         }
         P_CK(cudaMemcpyAsync(S.table.p + c0, table.data() + c0, n * sizeof(CcfGroup), cudaMemcpyHostToDevice, st));
-        P_CK(launch_polar_spectra(sbjs, S.tmpl.p, S.tw.p, NR, S.shifts_i.p, Sn, bs, c0, n, 0, S.sbj_sp.p, st,
+        P_CK(launch_polar_spectra(sbjs, S.dirs.p, S.tw.p, NR, S.shifts_i.p, Sn, bs, c0, n, 0, S.sbj_sp.p, st,
                                   sel_dev ? sel_dev + c0 : nullptr, sbj_tx));
         CcfWork w{};
         w.groups = S.table.p + c0;
@@ -264,7 +264,7 @@ __global__ void best_of_kernel(const float* __restrict__ d, const float4* __rest
 
 struct LearnState {
     std::mutex mu;
-    Buf<float2> tw, tmpl, shifts_f, ref_sp, sbj_sp;
+    Buf<float2> tw, dirs, shifts_f, ref_sp, sbj_sp;
     Buf<int2> shifts_i, zero;
     Buf<CcfGroup> table;
     Buf<unsigned> err, prop, fb_list, fb_flag;
@@ -309,7 +309,7 @@ extern "C" int gpuisac_learned_align_device(const AlignConfig* cfg, const float*
     const unsigned qt = ccf_refs_per_item(NR, variant);
 
     P_CK(S.tw.ensure(kRingLen));
-    P_CK(S.tmpl.ensure(geo.tmpl.size()));
+    P_CK(S.dirs.ensure(geo.dirs.size()));
     P_CK(S.shifts_f.ensure(Sn));
     P_CK(S.shifts_i.ensure(Sn));
     P_CK(S.zero.ensure(1));
@@ -317,7 +317,7 @@ extern "C" int gpuisac_learned_align_device(const AlignConfig* cfg, const float*
     P_CK(S.ref_sp.ensure(row_elems * R));
     const int2 zero = make_int2(0, 0);
     P_CK(cudaMemcpy(S.tw.p, geo.tw.data(), kRingLen * sizeof(float2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.tmpl.p, geo.tmpl.data(), geo.tmpl.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    P_CK(cudaMemcpy(S.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice));
     P_CK(cudaMemcpy(S.shifts_f.p, geo.shifts_f.data(), Sn * sizeof(float2), cudaMemcpyHostToDevice));
     P_CK(cudaMemcpy(S.shifts_i.p, geo.shifts_i.data(), Sn * sizeof(int2), cudaMemcpyHostToDevice));
     P_CK(cudaMemcpy(S.zero.p, &zero, sizeof(int2), cudaMemcpyHostToDevice));
@@ -328,7 +328,7 @@ extern "C" int gpuisac_learned_align_device(const AlignConfig* cfg, const float*
     const unsigned long long *ref_tx = nullptr, *sbj_tx = nullptr;
     if (texture_unit_enabled())
         ref_tx = S.ref_tex.try_build(refs, st);
-    P_CK(launch_polar_spectra(refs, S.tmpl.p, S.tw.p, NR, S.zero.p, 1, nullptr, 0, R, 1, S.ref_sp.p, st, nullptr,
+    P_CK(launch_polar_spectra(refs, S.dirs.p, S.tw.p, NR, S.zero.p, 1, nullptr, 0, R, 1, S.ref_sp.p, st, nullptr,
                               ref_tx));
 
     // chunk of particles: spectra at every shift, network activations over
@@ -396,7 +396,7 @@ extern "C" int gpuisac_learned_align_device(const AlignConfig* cfg, const float*
         const unsigned n = std::min(chunk, P - c0);
         const long rows = (long)n * Sn;
         // 1. subject spectra at every shift
-        P_CK(launch_polar_spectra(sbjs, S.tmpl.p, S.tw.p, NR, S.shifts_i.p, Sn, bs, c0, n, 0, S.sbj_sp.p, st, nullptr,
+        P_CK(launch_polar_spectra(sbjs, S.dirs.p, S.tw.p, NR, S.shifts_i.p, Sn, bs, c0, n, 0, S.sbj_sp.p, st, nullptr,
                                   sbj_tx));
         // 2. standardised ring features of every (particle, shift) row
         NN_CK(gpuisac_nn_features(reinterpret_cast<const float*>(S.sbj_sp.p), (unsigned)rows, NR, net->nk, net->mu,

@@ -36,7 +36,7 @@ constexpr int kShiftBlock = 8;   // shifts per CCF block
 __device__ __forceinline__ unsigned ring_off(unsigned r) { return (r >> 1) * 2 * kPair + (r & 1) * kL; }
 
 __global__ void __launch_bounds__(256)
-polar_spectra512_kernel(StackDesc st, const float2* __restrict__ tmpl, const float2* __restrict__ tw512,
+polar_spectra512_kernel(StackDesc st, const float2* __restrict__ dirs, const float2* __restrict__ tw512,
                         unsigned ring_num, const int2* __restrict__ shift_int, unsigned n_shift,
                         const float2* __restrict__ base, unsigned img0, unsigned n_img, int is_ref,
                         float2* __restrict__ out, const unsigned long long* __restrict__ tex_objs)
@@ -69,13 +69,15 @@ polar_spectra512_kernel(StackDesc st, const float2* __restrict__ tmpl, const flo
     const float yoff = (float)(place.local * st.dim);
     const cudaTextureObject_t tobj = tex_objs ? (cudaTextureObject_t)__ldg(tex_objs + place.tex_id) : 0;
 
+    const float2 dir[2] = {__ldg(&dirs[tid]), __ldg(&dirs[tid + 256])};
+    const RingScale scale(ring_num);
     float s1 = 0.f, s2 = 0.f;
     for (unsigned r = 0; r < ring_num; r++) {
         const float w = (float)(r + 1);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const unsigned j = tid + 256 * h;
-            const float2 o = __ldg(&tmpl[r * kL + j]);
+            const float2 o = scale.offset(dir[h], w);
             const float x = cnt_x + o.x;
             const float y = (yoff + cnt_y) + o.y;
             const float v = tex_objs ? tex2D<float>(tobj, x, y) : tex_sample(st, place, x, y);
@@ -349,7 +351,7 @@ size_t ccf512_smem(unsigned ring_num)
 
 GPUISAC_CHECKED_READER(checked_read_ring512)
 
-cudaError_t launch_polar_spectra512(const StackDesc& st, const float2* tmpl, const float2* tw512, unsigned ring_num,
+cudaError_t launch_polar_spectra512(const StackDesc& st, const float2* dirs, const float2* tw512, unsigned ring_num,
                                     const int2* shift_int, unsigned n_shift, const float2* base, unsigned img0,
                                     unsigned n_img, int is_ref, float2* out, cudaStream_t stream,
                                     const unsigned long long* tex_objs)
@@ -365,7 +367,7 @@ cudaError_t launch_polar_spectra512(const StackDesc& st, const float2* tmpl, con
     if (rows > 0x7FFFFFFFull)
         return cudaErrorInvalidValue;
     polar_spectra512_kernel<<<(unsigned)rows, 256, spectra512_smem(ring_num), stream>>>(
-        st, tmpl, tw512, ring_num, shift_int, n_shift, base, img0, n_img, is_ref, out, tex_objs);
+        st, dirs, tw512, ring_num, shift_int, n_shift, base, img0, n_img, is_ref, out, tex_objs);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaGetLastError();
 }
