@@ -574,8 +574,15 @@ int run_alignment_l512(const Geometry& g, Workspace& ws, const StackDesc& refs, 
     const double frac = (mem_request > 0.f && mem_request <= 1.f) ? mem_request : 0.9;
     const size_t budget = (size_t)((double)free_b * frac) / 2;
     const size_t per_part = row_elems * g.S * sizeof(float2);
-    const size_t chunk = std::min<size_t>(std::max<size_t>(1, std::min<size_t>(budget / per_part, 2048)), g.P);
-    if (ws.sbj_sp.ensure(per_part / sizeof(float2) * chunk))
+    // the ring sums of a chunk (4 KB per particle, reference and shift) take
+    // at most 8 GB: references in blocks where one particle against all of
+    // them would need more, then particles
+    const size_t z_cap = std::min<size_t>(budget, (size_t)8 << 30);
+    const size_t z_ref = ccf512_z_bytes(1, 1, g.S);
+    const unsigned rb = (unsigned)std::min<size_t>(g.R, std::max<size_t>(1, z_cap / z_ref));
+    size_t chunk = std::min<size_t>({budget / per_part, z_cap / (z_ref * rb), (size_t)2048});
+    chunk = std::min<size_t>(std::max<size_t>(1, chunk), g.P);
+    if (ws.sbj_sp.ensure(per_part / sizeof(float2) * chunk) || ws.zsp.ensure(z_ref * rb * chunk / sizeof(float2)))
         return E_NOMEM;
     for (unsigned p0 = 0; p0 < g.P; p0 += (unsigned)chunk) {
         const unsigned n = (unsigned)std::min<size_t>(chunk, g.P - p0);
@@ -584,8 +591,10 @@ int run_alignment_l512(const Geometry& g, Workspace& ws, const StackDesc& refs, 
                                    ws.sbj_sp.p, st, sbj_tx));
         g_timer.end(K_SPECTRA, ev, st);
         ev = g_timer.begin(st);
-        CK(launch_ccf_peak512(ws.sbj_sp.p, ws.ref_sp.p, ws.tw512.p, g.NR, g.S, g.R, n, p0, g.P, ws.shifts_f.p, d_base,
-                              d_out, d_peak, st));
+        for (unsigned q0 = 0; q0 < g.R; q0 += rb)
+            CK(launch_ccf_peak512(ws.sbj_sp.p, ws.ref_sp.p + q0 * row_elems, ws.tw512.p, g.NR, g.S,
+                                  std::min(rb, g.R - q0), n, p0, g.P, q0, g.R, ws.shifts_f.p, d_base,
+                                  reinterpret_cast<float4*>(ws.zsp.p), d_out, d_peak, st));
         g_timer.end(K_CCF, ev, st);
     }
     if (host) {

@@ -69,6 +69,32 @@ __device__ __forceinline__ float2 cmul_fixed(float2 a, float2 b)
 {
     return make_float2(__fmaf_rn(a.x, b.x, -__fmul_rn(a.y, b.y)), __fmaf_rn(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
+// Packed pairs as 64-bit registers for the contractions: an FFMA2 whose
+// operands are register pairs runs two FMAs a lane in the issue slot of one and
+// reads its operands at full rate (126 of 128 FMAs per cycle and SM measured on
+// an outer product, 97 for scalar FMAs with three distinct registers).  Through
+// float2 the compiler packs a broadcast operand again at every use.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ void fma_f32x2(f32x2& acc, f32x2 a, f32x2 b)
+{
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+// p = (x, y) -> (x, x) and (y, y)
+__device__ __forceinline__ void splat_both(f32x2 p, f32x2& xx, f32x2& yy)
+{
+    asm("{\n\t.reg .f32 x, y;\n\t"
+        "mov.b64 {x, y}, %2;\n\t"
+        "mov.b64 %0, {x, x};\n\t"
+        "mov.b64 %1, {y, y};\n\t}"
+        : "=l"(xx), "=l"(yy)
+        : "l"(p));
+}
+__device__ __forceinline__ float2 unpack_f32x2(f32x2 p)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
 // multiply by +i (SIGN>0) or -i (SIGN<0)
 template <int SIGN>
 __device__ __forceinline__ float2 cmul_i(float2 a)

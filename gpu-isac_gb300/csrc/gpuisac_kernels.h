@@ -153,12 +153,19 @@ cudaError_t launch_polar_spectra512(const StackDesc& st, const float2* dirs, con
                                     const int2* shift_int, unsigned n_shift, const float2* base, unsigned img0,
                                     unsigned n_img, int is_ref, float2* out, cudaStream_t stream,
                                     const unsigned long long* tex_objs);
-// results for particle i of sbj_sp to column p_first + i of d_out / peak_out
-// [n_ref][p_total]; base: base shifts by global particle index, or null
+// CCF of n_part particles against n_ref references (ref_sp's rows): the ring
+// sums to z (ccf512_z_bytes bytes), then inverse FFT and peak search; results
+// for particle i and reference q to row q_first + q, column p_first + i of
+// d_out / peak_out [q_total][p_total]; base: base shifts by global particle
+// index, or null
+inline size_t ccf512_z_bytes(size_t n_part, size_t n_ref, size_t n_shift)
+{
+    return n_part * n_ref * n_shift * kSlots512 * sizeof(float4);
+}
 cudaError_t launch_ccf_peak512(const float2* sbj_sp, const float2* ref_sp, const float2* tw512, unsigned ring_num,
                                unsigned n_shift, unsigned n_ref, unsigned n_part, unsigned p_first, unsigned p_total,
-                               const float2* shifts_f, const float2* base, float* d_out, float4* peak_out,
-                               cudaStream_t stream);
+                               unsigned q_first, unsigned q_total, const float2* shifts_f, const float2* base,
+                               float4* z, float* d_out, float4* peak_out, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------
 // Operands of the tensor-core contraction (ccf_split.cu).  For every spectrum
