@@ -101,6 +101,20 @@ __device__ __forceinline__ void write_z(float2* zp, int k, float a1, float a2, f
     }
 }
 
+// the same for two references: entries (re A, re B, im A, im B)
+__device__ __forceinline__ void write_z_two(float4* zp, int k, const float (&a)[4], const float (&b)[4])
+{
+    if (k == 0) {
+        const float pa1 = 0.25f * (a[0] + a[1] + a[2] + a[3]), pa2 = 0.25f * (a[0] - a[1] + a[2] - a[3]);
+        const float pb1 = 0.25f * (b[0] + b[1] + b[2] + b[3]), pb2 = 0.25f * (b[0] - b[1] + b[2] - b[3]);
+        zp[0] = make_float4(pa1, pb1, pa1, pb1);
+        zp[kSlots] = make_float4(pa2, pb2, pa2, pb2);
+    } else {
+        zp[k] = make_float4(a[0], b[0], a[1], b[1]);
+        zp[kRingLen - k] = make_float4(a[2], b[2], a[3], b[3]);
+    }
+}
+
 // inverse FFT of the pair spectrum this thread holds (x[m] = Z[l + 16 m]) and
 // the peak search of both mirrors; gz is the group's workspace of
 // kPairStride float2 (kTwl: tw is this thread's row of precomputed twiddles,
@@ -188,6 +202,101 @@ __device__ __forceinline__ void fft_peak(float2* gz, const float2* tw, int l, un
     for (int m = 0; m < 16; m++)
         x[m] = gz[l + 16 * m];
     fft_peak_regs<kTwl>(x, gz, tw, l, gmask, s, n_shift, st, rule);
+}
+
+__device__ __forceinline__ float fmax3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// the two halves of a pair of transforms (x from ifft256_two)
+template <int H>
+__device__ __forceinline__ float half_of(f32x2 p)
+{
+    const float2 v = unpack_f32x2(p);
+    return H == 0 ? v.x : v.y;
+}
+
+// fft_peak_regs' search on half H of a pair of transforms: x[perm16(k2)] holds
+// the correlations at angle l + 16 k2 (re normal, im mirrored); wf: 256 floats
+// of the group's workspace
+template <int H>
+__device__ __forceinline__ void peak_two(const Cx2 (&x)[16], float* wf, int l, unsigned gmask, unsigned s,
+                                         unsigned n_shift, PeakState& st, unsigned rule)
+{
+    if (rule == kPeakPreAlign && s == 0 && st.bv == 0.f && st.bh == 0 && st.bt == 0) {
+        // the starting index (normal, shift 0, angle 0) stays the answer when
+        // no value beats 0: keep its 7 neighbours
+        __syncwarp(gmask);
+#pragma unroll
+        for (int k2 = 0; k2 < 16; k2++)
+            wf[l + 16 * k2] = half_of<H>(x[perm16(k2)].re);
+        __syncwarp(gmask);
+        if (l < 7)
+            st.nb = wf[((unsigned)l - 3u) & (kRingLen - 1)];
+        __syncwarp(gmask);
+    }
+    // this thread's maximum of each mirror, then the group's over both; the
+    // normal mirror wins if any thread holds the maximum there (its scan index
+    // is lower).  Maxima ignore NaN: v is NaN only when every value is, on
+    // every thread alike, so the branches below stay group-uniform.
+    float vn = half_of<H>(x[0].re), vm = half_of<H>(x[0].im);
+#pragma unroll
+    for (int i = 1; i < 15; i += 2) {
+        vn = fmax3(vn, half_of<H>(x[i].re), half_of<H>(x[i + 1].re));
+        vm = fmax3(vm, half_of<H>(x[i].im), half_of<H>(x[i + 1].im));
+    }
+    vn = fmaxf(vn, half_of<H>(x[15].re));
+    float v = fmax3(vn, vm, half_of<H>(x[15].im));
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1)
+        v = fmaxf(v, __shfl_xor_sync(gmask, v, off));
+    if (!(v >= st.bv))
+        return;
+    const bool mir = !__any_sync(gmask, vn == v);
+    unsigned t = 0xffffffffu;
+#pragma unroll
+    for (int k2 = 15; k2 >= 0; k2--)
+        if (half_of<H>(mir ? x[perm16(k2)].im : x[perm16(k2)].re) == v)
+            t = l + 16 * k2;
+#pragma unroll
+    for (int off = 8; off > 0; off >>= 1)
+        t = min(t, __shfl_xor_sync(gmask, t, off));
+    const unsigned hc = mir ? n_shift + s : s;
+    if (t < (unsigned)kRingLen && better(v, hc, t, st.bv, st.bh, st.bt)) {
+        st.bv = v;
+        st.bh = hc;
+        st.bt = t;
+        __syncwarp(gmask);
+#pragma unroll
+        for (int k2 = 0; k2 < 16; k2++)
+            wf[l + 16 * k2] = half_of<H>(mir ? x[perm16(k2)].im : x[perm16(k2)].re);
+        __syncwarp(gmask);
+        if (l < 7)
+            st.nb = wf[(t + (unsigned)l - 3u) & (kRingLen - 1)];
+        __syncwarp(gmask);
+    }
+}
+
+// inverse FFTs and peak searches of the pair spectra of two references in gz
+// (256 entries (re A, re B, im A, im B), natural order; then the workspace);
+// two: whether B is a reference
+__device__ __forceinline__ void fft_peak_two(ulonglong2* gz, const float2* twl, int l, unsigned gmask, unsigned s,
+                                             unsigned n_shift, PeakState& sa, PeakState& sb, bool two, unsigned rule)
+{
+    Cx2 x[16];
+#pragma unroll
+    for (int m = 0; m < 16; m++) {
+        const ulonglong2 v = gz[l + 16 * m];
+        x[m] = Cx2{v.x, v.y};
+    }
+    ifft256_two(x, gz, twl, l, gmask);
+    float* const wf = reinterpret_cast<float*>(gz);
+    peak_two<0>(x, wf, l, gmask, s, n_shift, sa, rule);
+    if (two)
+        peak_two<1>(x, wf, l, gmask, s, n_shift, sb, rule);
 }
 
 // named barrier `id` over n threads (id 0 with n = blockDim is __syncthreads)

@@ -303,13 +303,25 @@ ccf_peak_tmem_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned rin
 // warp-specialised tensor-memory kernel: 512 threads.  Threads 0..255 stage
 // the subject spectra and run the contraction (references in tensor memory,
 // as above); threads 256..511 run the inverse FFTs and the peak search of the
-// previous shift group at the same time.  The two sides hand over the 16
+// previous shift groups at the same time.  The two sides hand over the 16
 // pair spectra through two shared-memory buffers guarded by named barriers
 // (FULL: contraction -> FFT, EMPTY: FFT -> contraction).
-constexpr int kWsBarC = 1;     // contraction side only (256 threads)
-constexpr int kWsBarFull = 2;  // + buffer: 2, 3
-constexpr int kWsBarEmpty = 4; // + buffer: 4, 5
-constexpr int kWsBarF = 6;     // FFT side only (256 threads)
+//
+// What bounds it: issue and FMA throughput of the CUDA cores (issue 62 %, FMA
+// pipe 52 %; scalar FMAs on three distinct registers reach 97 of 128 per cycle
+// and SM at best), 3,000 x 200 at 35 rings and 49 shifts: contraction alone
+// 25.5 ms, FFT side alone 19.8, without the copies 32.7, all of it 33.8 (37.4
+// with one team transforming one reference per group and the contraction side
+// meeting at every shift group; 150 x 300 at 61 rings 9.05 -> 8.40, 2,000 x 16
+// at 29 rings 1.18 -> 1.07).  On the way: two references per group in one team
+// 40.5 (four FFT warps wait on their own latency), two teams 36.4, halves 33.9.
+// Not kept: packed FMAs in the contraction (bit-identical; 35.7 against 33.9),
+// the staging area refilled in parts of a row as they are summed (47).
+constexpr int kWsBarC = 1;      // contraction side, item changes
+constexpr int kWsBarCH = 2;     // + half: 2, 3 (one half of the contraction side)
+constexpr int kWsBarFull = 4;   // + 2 buffer + half: 4 .. 7
+constexpr int kWsBarEmpty = 8;  // + 2 buffer + half: 8 .. 11
+constexpr int kWsBarF = 12;     // + team: 12, 13 (one FFT team only); 14: both teams
 
 // CW contraction warps (slot k x NSI*128/(32 CW) shifts per thread) + one
 // 16-thread FFT group per pair of the shift group (NSI shifts x 4 references).
@@ -317,7 +329,23 @@ constexpr int kWsBarF = 6;     // FFT side only (256 threads)
 // to kWsMaxRings rings (the references' tensor-memory columns bound both).
 // QR: reference slots the contraction sums (4; 1 when every group of the
 // launch has one reference -- the other slots' pairs stay idle).
-template <int CW, int NSI, int QR>
+// More than one reference: the FFT side is two teams, each 16-thread group
+// transforming two references at once (packed halves), and the item's
+// particles run as two streams (even and odd ones), team t on stream t and
+// buffer t, their shift groups taken in turn by the contraction -- so that two
+// shift groups are in the FFT side at a time.  One reference: one team, one
+// stream, the buffers in turn.
+// With 8 contraction warps each half of them (4 warps: every slot) has half of
+// the shift group's shifts, its own part of the staging area with its own
+// barrier, and its own hand-over to the FFT groups of its shifts: while one
+// half waits for its copies the other sums.  The halves only meet when the
+// references change.
+// kSplit (launches whose items hold one particle each, a proposal list's): the
+// two streams are the two halves of the particle's shifts instead, the teams'
+// bests merged at its end (a learned search of 4,000 particles with 16
+// proposals: 14.9 ms, 15.7 with one stream empty).  As a branch of the general
+// form it cost that form 12 %.
+template <int CW, int NSI, int QR, bool kSplit>
 __global__ void __launch_bounds__(32 * CW + NSI * 64, 1)
 ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_num, unsigned n_shift,
                    const float2* __restrict__ shifts_f, unsigned* __restrict__ err)
@@ -325,7 +353,13 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
     constexpr int QT = 4;
     constexpr int NP = NSI * QT;        // pairs per shift group
     constexpr int NC = 32 * CW;         // contraction threads
-    constexpr int NF = 16 * NP;         // FFT / peak threads
+    constexpr bool kTwo = QR > 1;       // two references per FFT group (packed halves)
+    constexpr int kTeams = kTwo ? 2 : 1;
+    constexpr int NF = 64 * NSI;        // FFT / peak threads
+    constexpr int NFT = NF / kTeams;    // of one team
+    constexpr int kHalves = CW / 4;     // of the contraction side
+    constexpr int NCH = NC / kHalves;   // threads of a half (128)
+    constexpr int NH = NCH + NFT / kHalves; // threads of a half's hand-over
     constexpr int NT = NC + NF;         // all threads
     constexpr int SPT = NSI * 128 / NC; // shifts per contraction thread
     static_assert((CW == 4 || CW == 8) && (NSI == 2 || NSI == 4) && SPT >= 1, "tile shape");
@@ -334,14 +368,13 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
     float2* sbuf = reinterpret_cast<float2*>(smem_raw);                // [NSI][nrp][kSlots]
     float2* zbuf = sbuf + (size_t)NSI * nrp * kSlots;                  // [2][NP][kPairStride]
     float2* tw = zbuf + 2 * NP * kPairStride;                          // [16][kTwRow] per FFT lane
-    PeakSlot* slots = reinterpret_cast<PeakSlot*>(tw + 16 * kTwRow);   // [16]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(slots + 16);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    // the item after the current one, by item parity: taken from the work
-    // counter (w.item_counter) by the contraction side's thread 0, read by
-    // both sides
-    volatile unsigned* next_item = reinterpret_cast<volatile unsigned*>(abort_flag + 1);
+    PeakSlot* slots = reinterpret_cast<PeakSlot*>(tw + 16 * kTwRow);   // [team][16]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(slots + 32); // [half]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
+    // the items after the current one, a ring of 4 (the contraction side can be
+    // two items ahead of an FFT team): taken from the work counter
+    // (w.item_counter) by the contraction side's thread 0, read by both sides
+    volatile unsigned* next_item = reinterpret_cast<volatile unsigned*>(tmem_slot + 1);
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
@@ -350,8 +383,21 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
     // stream, particle-major: with n_shift >= NSI a group may hold the end of
     // one particle and the start of the next, so no group is left part empty
     // at a particle's end.  Below NSI shifts every particle is padded to whole
-    // groups.  Row v of the item is particle v / vstride, shift v % vstride.
+    // groups.  Row v of stream t is the item's particle kTeams (v / vstride) +
+    // t, shift v % vstride.
     const unsigned vstride = n_shift >= (unsigned)NSI ? n_shift : (n_shift + NSI - 1) / NSI * NSI;
+    // v / vstride as a high product: exact while rows x vstride < 2^32
+    // (vstride <= 4,096, work items of at most 256 particles)
+    const unsigned vrecip = 0xFFFFFFFFu / vstride + 1;
+
+    // rows of stream t of np particles, and its shift groups (at least one:
+    // every team takes part in every item)
+    static_assert(!kSplit || kTeams == 2, "two streams");
+    const unsigned half_s = (n_shift + 1) / 2;
+    auto stream_rows = [&](unsigned np, unsigned t) {
+        return kSplit ? (t ? n_shift - half_s : half_s) : (np + kTeams - 1 - t) / kTeams * vstride;
+    };
+    auto stream_groups = [&](unsigned np, unsigned t) { return max(1u, (stream_rows(np, t) + NSI - 1) / NSI); };
 
     unsigned item = blockIdx.x;
     CcfGroup grp;
@@ -359,8 +405,8 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
     if (!decode_item(w, item, QT, grp, q0, pb, pe))
         return;
 
-    if (tid < kRingLen) { // lane l's inverse-FFT twiddles, row l
-        const int tl = tid >> 4, tj = tid & 15;
+    for (int i = tid; i < kRingLen; i += NT) { // lane l's inverse-FFT twiddles, row l
+        const int tl = i >> 4, tj = i & 15;
         const float2 t = twiddle[(tl * tj) & (kRingLen - 1)];
         tw[tl * kTwRow + tj] = make_float2(t.x, t.y * -1.f);
     }
@@ -369,55 +415,68 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
     if (warp == 0)
         tmem_alloc(tmem_slot, kTmemCols);
     if (tid == 0) {
-        mbar_init(bar, 1);
+        mbar_init(bars, 1);
+        mbar_init(bars + 1, 1);
         mbar_fence_init();
-        *abort_flag = 0;
     }
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
 
-    bool failed = false;
-    uint32_t phase = 0;
     if (contraction_side) {
         // ================= contraction side =================
         const int k = tid & (kSlots - 1);
         const int half = tid >> 7; // which SPT shifts of the group (0 when CW = 4)
+        const bool lead = (tid & (NCH - 1)) == 0; // issues the half's copies
+        uint64_t* const bar = bars + half;
+        uint32_t phase = 0;
+        // a half whose copies did not arrive in time stops copying and waiting
+        // and runs through its items (in-bounds, results void: the host reports
+        // the call as failed), so that every hand-over still takes place
+        bool failed = false;
         // lane k of the tensor memory holds slot k; columns: [ring][ref][u, v]
         const uint32_t tmem = *tmem_slot + ((uint32_t)(32 * (warp & 3)) << 16);
         const uint32_t row_bytes = ring_num * kSlots * sizeof(float2);
-        // the shift group of rows v0..v0+NSI-1 (item-local) of the item whose
-        // particles start at p0 and number np
+        // this half's part of the shift group of rows v0..v0+NSI-1 of stream t of
+        // the item whose particles start at p0 and number np
         const uint32_t wlim = wait_tries(w.wait_iters);
         // returns whether copies were issued
-        auto issue = [&](const CcfGroup& gg, unsigned p0, unsigned np, unsigned v0) -> bool {
+        auto issue = [&](const CcfGroup& gg, unsigned p0, unsigned np, unsigned t, unsigned v0) -> bool {
             const float2* sp = gg.sbj_sp;
             if (w.test_stall)
                 return false;
+            size_t at[SPT];
+            bool in[SPT];
             unsigned nv = 0;
-            for (unsigned i = 0; i < (unsigned)NSI; i++) {
-                const unsigned v = v0 + i, pl = v / vstride;
-                nv += (pl < np && v - pl * vstride < n_shift) ? 1u : 0u;
+#pragma unroll
+            for (int i = 0; i < SPT; i++) {
+                const unsigned v = v0 + SPT * half + i;
+                unsigned pl = 0, sv = t * half_s + v; // the row's particle of the item and shift
+                if (!kSplit) {
+                    pl = __umulhi(v, vrecip);
+                    sv = v - pl * vstride;
+                    pl = kTeams * pl + t;
+                }
+                at[i] = ((size_t)(p0 + pl) * n_shift + sv) * ring_num * kSlots;
+                in[i] = kSplit ? v < stream_rows(np, t) : pl < np && sv < n_shift;
+                nv += in[i] ? 1u : 0u;
             }
             fence_proxy_async();
             mbar_expect_tx(bar, nv * row_bytes);
-            for (unsigned i = 0; i < (unsigned)NSI; i++) {
-                const unsigned v = v0 + i, pl = v / vstride, sv = v - pl * vstride;
-                const size_t at = ((size_t)(p0 + pl) * n_shift + sv) * ring_num * kSlots;
-                if (pl < np && sv < n_shift &&
-                    GPUISAC_IN_BOUNDS(kChkCcfRow, at + (size_t)ring_num * kSlots - 1,
-                                      (size_t)gg.n_part * n_shift * ring_num * kSlots))
-                    bulk_g2s(sbuf + (size_t)i * nrp * kSlots, sp + at, row_bytes, bar);
-            }
+#pragma unroll
+            for (int i = 0; i < SPT; i++)
+                if (in[i] && GPUISAC_IN_BOUNDS(kChkCcfRow, at[i] + (size_t)ring_num * kSlots - 1,
+                                               (size_t)gg.n_part * n_shift * ring_num * kSlots))
+                    bulk_g2s(sbuf + (size_t)(SPT * half + i) * nrp * kSlots, sp + at[i], row_bytes, bar);
             return true;
         };
-        bool pending = false; // thread 0: copies in flight
-        if (tid == 0)
-            pending = issue(grp, pb, pe - pb, 0);
+        bool pending = false; // lead thread: copies in flight
+        if (lead)
+            pending = issue(grp, pb, pe - pb, 0, 0);
         unsigned it = 0, ii = 0;
-        while (!failed) {
+        while (true) {
             if (tid == 0)
-                next_item[ii & 1u] = w.item_counter ? gridDim.x + atomicAdd(w.item_counter, 1u) : item + gridDim.x;
+                next_item[ii & 3u] = w.item_counter ? gridDim.x + atomicAdd(w.item_counter, 1u) : item + gridDim.x;
             // this item's references -> tensor memory (both halves read every ring)
             for (unsigned j = 2 * half; j < nrp; j += 2 * (NC / 128)) {
 #pragma unroll
@@ -440,26 +499,23 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
             tmem_fence_after();
             CcfGroup ngrp;
             unsigned nq0 = 0, npb = 0, npe = 0;
-            const unsigned nxt = next_item[ii & 1u];
+            const unsigned nxt = next_item[ii & 3u];
             const bool has_next = decode_item(w, nxt, QT, ngrp, nq0, npb, npe);
 
-            const unsigned nrows = (pe - pb) * vstride;
-            for (unsigned v0 = 0; v0 < nrows && !failed; v0 += NSI, it++) {
+            const unsigned np = pe - pb;
+            const unsigned ng0 = stream_groups(np, 0), ng1 = kTeams == 2 ? stream_groups(np, 1) : 0;
+            // shift group j of stream t, then (j, 1) or (j + 1, 0)
+            for (unsigned j = 0, t = 0; j < ng0; it++) {
                 {
-                    const unsigned b = it & 1u;
-                    // ---- wait for this group's spectra (bounded) ----
-                    const bool ok = mbar_wait(bar, phase, wlim);
-                    if (ok && tid == 0)
-                        pending = false;
-                    if (!nbar_and(kWsBarC, NC, ok)) {
-                        // hand the FFT side an empty buffer marked abort
-                        failed = true;
-                        nbar_sync(kWsBarEmpty + b, NT);
-                        if (tid == 0)
-                            *abort_flag = 1;
-                        __threadfence_block();
-                        nbar_arrive(kWsBarFull + b, NT);
-                        break;
+                    const unsigned b = kTeams == 2 ? t : it & 1u;
+                    const bool to_other = kTeams == 2 && t == 0 && j < ng1;
+                    const unsigned nj = to_other ? j : j + 1, nt = to_other ? 1u : 0u;
+                    // ---- wait for this half's spectra (bounded) ----
+                    if (!failed) {
+                        const bool ok = mbar_wait(bar, phase, wlim);
+                        if (ok && lead)
+                            pending = false;
+                        failed = !nbar_and(kWsBarCH + half, NCH, ok);
                     }
                     phase ^= 1u;
                     float acc[QR][SPT][4];
@@ -523,28 +579,36 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
                             ring_pair(ra, nrp - 2);
                     }
                     tmem_fence_before();
-                    nbar_sync(kWsBarC, NC); // the staging area is consumed
+                    nbar_sync(kWsBarCH + half, NCH); // this half's staging area is consumed
                     tmem_fence_after();
-                    if (tid == 0) {
-                        if (v0 + NSI < nrows)
-                            pending = issue(grp, pb, pe - pb, v0 + NSI);
+                    if (lead && !failed) {
+                        if (nj < ng0)
+                            pending = issue(grp, pb, np, nt, nj * NSI);
                         else if (has_next)
-                            pending = issue(ngrp, npb, npe - npb, 0);
+                            pending = issue(ngrp, npb, npe - npb, 0, 0);
                     }
                     // ---- hand the pair spectra to the FFT side ----
                     float2* zb = zbuf + (size_t)b * NP * kPairStride;
-                    nbar_sync(kWsBarEmpty + b, NT);
+                    nbar_sync(kWsBarEmpty + 2 * b + half, NH);
 #pragma unroll
                     for (int ii = 0; ii < SPT; ii++)
+                        if constexpr (kTwo) {
+#pragma unroll
+                            for (int q = 0; q < QR; q += 2)
+                                write_z_two(reinterpret_cast<float4*>(zb + ((SPT * half + ii) * QT + q) * kPairStride),
+                                            k, acc[q][ii], acc[q + 1][ii]);
+                        } else
 #pragma unroll
                         for (int q = 0; q < QR; q++)
                             write_z(zb + ((SPT * half + ii) * QT + q) * kPairStride, k, acc[q][ii][0], acc[q][ii][1],
                                     acc[q][ii][2], acc[q][ii][3]);
                     __threadfence_block();
-                    nbar_arrive(kWsBarFull + b, NT);
+                    nbar_arrive(kWsBarFull + 2 * b + half, NH);
+                    j = nj;
+                    t = nt;
                 }
             }
-            if (failed || !has_next)
+            if (!has_next)
                 break;
             item = nxt;
             ii++;
@@ -558,67 +622,94 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
             nbar_sync(kWsBarC, NC);
             tmem_fence_after();
         }
-        if (failed && tid == 0) {
+        if (failed && lead) {
             atomicExch(err, 1u);
             if (pending)
                 mbar_wait(bar, phase, wlim); // let copies in flight land before leaving (bounded)
         }
     } else {
         // ================= FFT / peak side =================
-        const int ftid = tid - NC;
+        const int team = kTeams == 2 ? (tid - NC) / NFT : 0;
+        const int ftid = tid - NC - team * NFT;
         const int g = ftid >> 4, l = ftid & 15;
         const unsigned gmask = 0xffffu << (ftid & 16);
-        const int g_shift = g / QT;
-        // both buffers start empty
-        nbar_arrive(kWsBarEmpty + 0, NT);
-        nbar_arrive(kWsBarEmpty + 1, NT);
+        PeakSlot* const tslots = slots + NP * team;
+        // the group's shift of the shift group and its (first) reference slot
+        const int g_shift = kTwo ? g / (QT / 2) : g / QT;
+        const int g_ref = kTwo ? 2 * (g % (QT / 2)) : g % QT;
+        const int slot = g_shift * QT + g_ref;
+        const int half = g_shift / SPT; // the contraction half that fills this group's pairs
+        // the buffers start empty (a team of two has one)
+        nbar_arrive(kWsBarEmpty + 2 * team + half, NH);
+        if (kTeams == 1)
+            nbar_arrive(kWsBarEmpty + 2 + half, NH);
         unsigned it = 0, ii = 0;
-        while (!failed) {
+        while (true) {
             // st: the slot's running best of particle pb + pc, the particle of
             // the shift group's first row.  In the group that holds pc's last
             // row, a slot whose row already belongs to pc + 1 parks its best
             // of pc before starting afresh, the others after their row; then
             // the slots are merged for pc.
-            const unsigned nrows = (pe - pb) * vstride;
+            const unsigned nrows = stream_rows(pe - pb, team), ng = stream_groups(pe - pb, team);
             unsigned pc = 0;
-            PeakState st;
+            PeakState st, st2; // (st2: the group's second reference)
             st.reset(grp.rule);
-            for (unsigned v0 = 0; v0 < nrows; v0 += NSI, it++) {
-                const unsigned b = it & 1u;
-                nbar_sync(kWsBarFull + b, NT);
-                if (*abort_flag) {
-                    failed = true;
-                    break;
+            st2.reset(grp.rule);
+            auto park = [&]() {
+                park_slot(tslots, st, slot, l);
+                st.reset(grp.rule);
+                if (kTwo) {
+                    park_slot(tslots, st2, slot + 1, l);
+                    st2.reset(grp.rule);
                 }
-                float2* gz = zbuf + (size_t)b * NP * kPairStride + g * kPairStride;
-                const unsigned v = v0 + g_shift, pl = v / vstride, s = v - pl * vstride;
-                const bool last = (pc + 1) * vstride <= v0 + NSI; // pc's last row is in this group
-                const bool next = pl != pc;                        // the same on both groups of a warp
-                if (last && next) {
-                    park_slot(slots, st, g, l);
-                    st.reset(grp.rule);
-                }
+            };
+            for (unsigned j = 0; j < ng; j++, it++) {
+                const unsigned b = kTeams == 2 ? (unsigned)team : it & 1u, v0 = j * NSI;
+                nbar_sync(kWsBarFull + 2 * b + half, NH);
+                float2* gz = zbuf + (size_t)b * NP * kPairStride + slot * kPairStride;
+                const unsigned v = v0 + g_shift, pl = kSplit ? 0 : __umulhi(v, vrecip);
+                const unsigned s = kSplit ? team * half_s + v : v - pl * vstride;
+                // pc's last row is in this group
+                const bool last = !kSplit && nrows > 0 && (pc + 1) * vstride <= v0 + NSI;
+                const bool next = pl != pc; // the same on both groups of a warp
+                if (last && next)
+                    park();
                 // pairs of reference slots the group does not fill stay idle
-                if (v < nrows && s < n_shift && q0 + (unsigned)(g % QT) < grp.n_ref)
-                    fft_peak<true>(gz, tw + l * kTwRow, l, gmask, s, n_shift, st, grp.rule);
+                if (v < nrows && s < n_shift && q0 + (unsigned)g_ref < grp.n_ref) {
+                    if constexpr (kTwo)
+                        fft_peak_two(reinterpret_cast<ulonglong2*>(gz), tw + l * kTwRow, l, gmask, s, n_shift, st,
+                                     st2, q0 + (unsigned)g_ref + 1 < grp.n_ref, grp.rule);
+                    else
+                        fft_peak<true>(gz, tw + l * kTwRow, l, gmask, s, n_shift, st, grp.rule);
+                }
                 __threadfence_block();
-                nbar_arrive(kWsBarEmpty + b, NT);
+                nbar_arrive(kWsBarEmpty + 2 * b + half, NH);
                 if (last) {
-                    if (!next) {
-                        park_slot(slots, st, g, l);
-                        st.reset(grp.rule);
-                    }
-                    merge_slots<kWsBarF, NF>(slots, ftid, QT, NSI, q0, grp.n_ref, n_shift, grp.p_first + pb + pc,
-                                             grp.p_total, shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule);
+                    if (!next)
+                        park();
+                    const unsigned pg = grp.p_first + pb + kTeams * pc + team;
+                    if (team == 0)
+                        merge_slots<kWsBarF, NFT>(tslots, ftid, QT, NSI, q0, grp.n_ref, n_shift, pg, grp.p_total,
+                                                  shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule);
+                    else
+                        merge_slots<kWsBarF + 1, NFT>(tslots, ftid, QT, NSI, q0, grp.n_ref, n_shift, pg, grp.p_total,
+                                                      shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule);
                     pc++;
                 }
             }
-            if (failed)
-                break;
+            if constexpr (kSplit) {
+                // both teams' bests of the particle, merged by team 0
+                park();
+                nbar_sync(kWsBarF + 2, NF);
+                if (team == 0)
+                    merge_slots<kWsBarF, NFT>(slots, ftid, QT, 2 * NSI, q0, grp.n_ref, n_shift, grp.p_first + pb,
+                                              grp.p_total, shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule);
+                nbar_sync(kWsBarF + 2, NF); // team 1's slots are free again
+            }
             // (written by the contraction side before this item's first full buffer)
             CcfGroup ngrp;
             unsigned nq0 = 0, npb = 0, npe = 0;
-            const unsigned nxt = next_item[ii & 1u];
+            const unsigned nxt = next_item[ii & 3u];
             if (!decode_item(w, nxt, QT, ngrp, nq0, npb, npe))
                 break;
             item = nxt;
@@ -789,17 +880,17 @@ static size_t ws_smem_bytes(unsigned ring_num)
 {
     const unsigned nrp = 2 * ((ring_num + 1) / 2), nsi = ws_shifts_per_group(ring_num);
     return (size_t)nsi * nrp * kSlots * sizeof(float2) + 2 * nsi * 4 * kPairStride * sizeof(float2) +
-           16 * kTwRow * sizeof(float2) + 16 * sizeof(PeakSlot) + 16 + 16; // barrier, tensor-memory slot, abort, next items
+           16 * kTwRow * sizeof(float2) + 32 * sizeof(PeakSlot) + 16 + 32; // barriers, tensor-memory slot, next items
 }
 
-template <int CW, int NSI, int QR>
+template <int CW, int NSI, int QR, bool kSplit = false>
 static cudaError_t launch_ws(const CcfWork& w, unsigned grid, const float2* twiddle, unsigned ring_num,
                              unsigned n_shift, const float2* shifts_f, unsigned* err, cudaStream_t stream)
 {
-    cudaError_t e = set_max_smem(ccf_peak_ws_kernel<CW, NSI, QR>);
+    cudaError_t e = set_max_smem(ccf_peak_ws_kernel<CW, NSI, QR, kSplit>);
     if (e != cudaSuccess)
         return e;
-    ccf_peak_ws_kernel<CW, NSI, QR><<<grid, 32 * CW + NSI * 64, ws_smem_bytes(ring_num), stream>>>(
+    ccf_peak_ws_kernel<CW, NSI, QR, kSplit><<<grid, 32 * CW + NSI * 64, ws_smem_bytes(ring_num), stream>>>(
         w, twiddle, ring_num, n_shift, shifts_f, err);
     return cudaSuccess;
 }
@@ -932,12 +1023,16 @@ cudaError_t launch_ccf_peak_work(const CcfWork& w_in, int variant, const float2*
         if (ring_num <= kTmaMaxRings) {
             if (one_ref)
                 e = launch_ws<8, 4, 1>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
+            else if (w.ppc == 1 || w.max_part == 1)
+                e = launch_ws<8, 4, 4, true>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
             else
                 e = four ? launch_ws<4, 4, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
                          : launch_ws<8, 4, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
         } else {
             if (one_ref)
                 e = launch_ws<8, 2, 1>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
+            else if (w.ppc == 1 || w.max_part == 1)
+                e = launch_ws<8, 2, 4, true>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
             else
                 e = four ? launch_ws<4, 2, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
                          : launch_ws<8, 2, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
@@ -998,6 +1093,7 @@ cudaError_t launch_ccf_peak(const float2* sbj_sp, const float2* ref_sp, const fl
     g.rule = rule;
     w.n_items = g.ref_tiles * ((n_part + w.ppc - 1) / w.ppc);
     w.max_ref = n_ref;
+    w.max_part = n_part;
     w.item_counter = item_counter;
     return launch_ccf_peak_work(w, variant, twiddle, ring_num, n_shift, shifts_f, err, stream);
 }

@@ -230,6 +230,117 @@ __device__ __forceinline__ void fft256_group_twl(float2 (&x)[16], float2* ws, co
 }
 
 // ---------------------------------------------------------------------------
+// Two 256-point inverse FFTs per group of 16 threads, one in each half of the
+// packed registers: with real parts (A, B) and imaginary parts (A, B) as
+// pairs every add, subtract and multiply is one packed instruction for both
+// transforms, and the rotations by i only exchange registers (a single
+// complex number as a pair leaves them scalar: 10 instead of 8 instructions
+// per 4-point step and transform, twiddles 4 instead of 2).  Each half rounds
+// as the compiler rounds fft256_group_twl<+1>: its products by the constants
+// fuse the first, its twiddle products' imaginary parts the second summand.
+struct Cx2 {
+    f32x2 re, im;
+};
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 pack_f32x2(float x, float y)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+// a times (c + i s), c and s in both halves (ns = -s): re = c a.re - s a.im,
+// the imaginary part's fused product the one with s (kImS) or with c
+template <bool kImS>
+__device__ __forceinline__ Cx2 cmul2(const Cx2& a, f32x2 c, f32x2 s, f32x2 ns)
+{
+    return Cx2{fma2(a.re, c, mul2(a.im, ns)),
+               kImS ? fma2(a.re, s, mul2(a.im, c)) : fma2(a.im, c, mul2(a.re, s))};
+}
+__device__ __forceinline__ void dft4_two(Cx2& x0, Cx2& x1, Cx2& x2, Cx2& x3)
+{
+    const Cx2 a{add2(x0.re, x2.re), add2(x0.im, x2.im)}, b{sub2(x0.re, x2.re), sub2(x0.im, x2.im)};
+    const Cx2 c{add2(x1.re, x3.re), add2(x1.im, x3.im)}, e{sub2(x1.re, x3.re), sub2(x1.im, x3.im)};
+    x0 = Cx2{add2(a.re, c.re), add2(a.im, c.im)};
+    x2 = Cx2{sub2(a.re, c.re), sub2(a.im, c.im)};
+    x1 = Cx2{sub2(b.re, e.im), add2(b.im, e.re)}; // b + i e
+    x3 = Cx2{add2(b.re, e.im), sub2(b.im, e.re)}; // b - i e
+}
+// dft16<+1> of both halves
+__device__ __forceinline__ void dft16_two(Cx2 (&x)[16])
+{
+    const float c1 = 0.923879532511286756f, s1 = 0.382683432365089772f, c2 = 0.707106781186547524f;
+    const f32x2 pc1 = pack_f32x2(c1, c1), ps1 = pack_f32x2(s1, s1), pc2 = pack_f32x2(c2, c2);
+    const f32x2 nc1 = pack_f32x2(-c1, -c1), ns1 = pack_f32x2(-s1, -s1), nc2 = pack_f32x2(-c2, -c2);
+#pragma unroll
+    for (int n1 = 0; n1 < 4; n1++)
+        dft4_two(x[n1], x[n1 + 4], x[n1 + 8], x[n1 + 12]);
+    // x[n1 + 4 k1] times e^(2 pi i n1 k1 / 16)
+    x[5] = cmul2<true>(x[5], pc1, ps1, ns1);    // 1
+    x[9] = cmul2<true>(x[9], pc2, pc2, nc2);    // 2
+    x[13] = cmul2<true>(x[13], ps1, pc1, nc1);  // 3
+    x[6] = cmul2<true>(x[6], pc2, pc2, nc2);    // 2
+    {                                         // 4: i
+        const f32x2 t = x[10].re;
+        x[10].re = x[10].im ^ 0x8000000080000000ull;
+        x[10].im = t;
+    }
+    x[14] = cmul2<true>(x[14], nc2, pc2, nc2);  // 6
+    x[7] = cmul2<true>(x[7], ps1, pc1, nc1);    // 3
+    x[11] = cmul2<true>(x[11], nc2, pc2, nc2);  // 6
+    x[15] = cmul2<true>(x[15], nc1, ns1, ps1);  // 9
+#pragma unroll
+    for (int k1 = 0; k1 < 4; k1++)
+        dft4_two(x[4 * k1], x[4 * k1 + 1], x[4 * k1 + 2], x[4 * k1 + 3]);
+}
+// In: x[m] = (z_A, z_B)[l + 16 m]; out: x[perm16(k2)] = (Z_A, Z_B)[l + 16 k2].
+// ws: 16 x 17 ulonglong2 (re pair, im pair); twl: thread l's row of kTwRow
+// float2 e^(+2 pi i l j / 256).
+__device__ __forceinline__ void ifft256_two(Cx2 (&x)[16], ulonglong2* ws, const float2* twl, int l, unsigned mask)
+{
+    dft16_two(x);
+#pragma unroll
+    for (int j = 1; j < 16; j++) {
+        const float2 w = twl[j];
+        x[perm16(j)] = cmul2<false>(x[perm16(j)], pack_f32x2(w.x, w.x), pack_f32x2(w.y, w.y), pack_f32x2(-w.y, -w.y));
+    }
+    __syncwarp(mask);
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+        ws[l * 17 + j] = make_ulonglong2(x[perm16(j)].re, x[perm16(j)].im);
+    __syncwarp(mask);
+#pragma unroll
+    for (int n = 0; n < 16; n++) {
+        const ulonglong2 v = ws[n * 17 + l];
+        x[n] = Cx2{v.x, v.y};
+    }
+    __syncwarp(mask);
+    dft16_two(x);
+}
+
+// ---------------------------------------------------------------------------
 // Polar sampling offsets.  The reference's template
 // (generate_polar_sampling_points, cuda/gpu_aln_common.cu:39-62) holds, for
 // ring radius R and direction (c, s) = (cosf, sinf) of the sample's angle,

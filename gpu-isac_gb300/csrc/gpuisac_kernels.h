@@ -249,6 +249,7 @@ struct CcfWork {
     unsigned* item_counter;
     unsigned ppc;     // particles per work item
     unsigned max_ref; // most references of any group (0: not known); 1 selects the one-reference contraction
+    unsigned max_part; // most particles of any group (0: not known); 1 (or ppc = 1) selects the split-shift streams
     // failure-path tests only (gpuisac_test_stall_ccf): the kernels that stage
     // with bulk copies issue none, and their bounded waits give up after
     // wait_iters tries (0: the default, about a second)
