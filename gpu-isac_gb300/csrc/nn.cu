@@ -130,58 +130,229 @@ __global__ void group_max_kernel(const float* __restrict__ G, long n, int group,
 // ---------------------------------------------------------------- GEMM
 // C[m][n] = alpha * sum_k A(m,k) B(k,n) + beta * C[m][n], with A(m,k) at
 // A[m*sam + k*sak] and B(k,n) at B[k*sbk + n*sbn] (strides give transposes).
-// 64x64 tile per CTA of 256 threads, 4x4 outputs per thread, K in steps of 16.
-constexpr int TM = 64, TN = 64, TK = 16;
+// A launch runs up to kMaxProblems of them (tiles numbered through), each with
+// an optional second product added to it (a weight's gradient from particles
+// and references), bias + ReLU or a ReLU mask.  Every output is summed by one
+// thread in the order of k.
+//
+// What bounds it: the network's products are small (500 x 256 x 560 at most in
+// a training step of 500 particles and 200 references), so the time is the
+// latency of one tile's K loop.  64 x 64 tiles over 8 to 32 CTAs, loading each
+// K step of 16 between two barriers, took 44 us a product, 573 of a step's 640
+// us on the device; 32 x 32 tiles with the next 64 of K in flight, and
+// independent products sharing a launch, take 91 of 102 us (15 us a launch; 27
+// with 128 threads a tile and the operand's layout told apart at every load).
+// Products with at least one 64 x 64 tile per SM keep that tile (half the
+// loads per FMA).
+constexpr int kMaxProblems = 4;
+struct GemmPart {
+    const float *A, *B;
+    long sam, sak, sbk, sbn;
+    int K;
+};
+struct GemmProblem {
+    int M, N;
+    float alpha, beta;
+    GemmPart part[2]; // (part[1].K = 0: none)
+    float* C;
+    long ldc;
+    const float* bias; // added per column, then ReLU if relu; or null
+    int relu;
+    const float* mask; // zero C where mask[m * ldc + n] is not positive; or null
+    int tiles_n, tile_begin;
+};
+// sums of columns: db[j] = sum_i dY[i][j] (+ the same of dY2), by the last CTAs
+struct ColSum {
+    const float *dY, *dY2;
+    long rows, rows2;
+    int cols;
+    float* db;
+};
+struct GemmGroup {
+    GemmProblem p[kMaxProblems];
+    int n, tiles;
+    ColSum cs[2];
+};
 
-__global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, float alpha, const float* __restrict__ A,
-                                                   long sam, long sak, const float* __restrict__ B, long sbk,
-                                                   long sbn, float beta, float* __restrict__ C, long ldc)
+// sum of a column in row order (16 loads in flight)
+__device__ __forceinline__ float col_sum(const float* __restrict__ dY, long rows, int cols, int j)
 {
-    __shared__ float As[TK][TM + 4];
-    __shared__ float Bs[TK][TN + 4];
+    float s = 0.f;
+#pragma unroll 16
+    for (long i = 0; i < rows; i++)
+        s += dY[i * cols + j];
+    return s;
+}
+
+// One operand's loads of a K step: T outer indices (rows of A, columns of B) x
+// TK of k by 256 threads, kN each, along the operand's unit-stride dimension:
+// k fastest (kK: a warp reads 8 k of 4 outer indices, whole sectors) or the
+// outer index fastest (32 in a row).  No two lanes of a warp store to one bank
+// of s[k][outer] (row length T + 4).
+template <int T, int TK, bool kK>
+struct GemmLoad {
+    static constexpr int kN = T * TK / 256;
+    static constexpr int kOuter = kK ? T / 32 : 1, kPer = kN / kOuter;
+    const float* p[kOuter];
+    bool in[kOuter];
+    long step_k; // between the thread's successive k
+    int o0, kk0, K;
+    __device__ __forceinline__ GemmLoad(const float* base, long so, long sk, int first, int n, int k_count)
+    {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        if (kK) {
+            o0 = (lane >> 3) + 4 * warp;
+            kk0 = lane & 7;
+        } else {
+            constexpr int kStrips = T / 32; // warps side by side
+            o0 = lane + 32 * (warp % kStrips);
+            kk0 = warp / kStrips;
+        }
+        K = k_count;
+        step_k = sk;
+#pragma unroll
+        for (int j = 0; j < kOuter; j++) {
+            in[j] = first + o0 + 32 * j < n;
+            p[j] = base + (in[j] ? (long)(first + o0 + 32 * j) * so + (long)kk0 * sk : 0);
+        }
+    }
+    static constexpr int kStep = kK ? 8 : 8 / (T / 32); // k between a thread's loads
+    __device__ __forceinline__ void fetch(float (&r)[kN], int k0) const
+    {
+#pragma unroll
+        for (int j = 0; j < kOuter; j++)
+#pragma unroll
+            for (int i = 0; i < kPer; i++)
+                r[j * kPer + i] =
+                    in[j] && k0 + kk0 + kStep * i < K ? __ldg(p[j] + (long)(k0 + kStep * i) * (kK ? 1 : step_k)) : 0.f;
+    }
+    __device__ __forceinline__ void store(const float (&r)[kN], float (*s)[T + 4]) const
+    {
+#pragma unroll
+        for (int j = 0; j < kOuter; j++)
+#pragma unroll
+            for (int i = 0; i < kPer; i++)
+                s[kk0 + kStep * i][o0 + 32 * j] = r[j * kPer + i];
+    }
+};
+
+// one product of a tile, added to acc
+template <int T, int TK, bool kA, bool kB>
+__device__ __forceinline__ void gemm_part(const GemmPart& q, int m0, int M, int n0, int N, float (*As)[TK][T + 4],
+                                          float (*Bs)[TK][T + 4], float (&acc)[T / 16][T / 16])
+{
+    constexpr int U = T / 16; // outputs per thread and dimension
+    const GemmLoad<T, TK, kA> la(q.A, q.sam, q.sak, m0, M, q.K);
+    const GemmLoad<T, TK, kB> lb(q.B, q.sbn, q.sbk, n0, N, q.K);
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        for (int e = threadIdx.x; e < TK * TM; e += 256) {
-            const int kk = e / TM, mm = e - kk * TM;
-            const int gm = m0 + mm, gk = k0 + kk;
-            As[kk][mm] = (gm < M && gk < K) ? A[(long)gm * sam + (long)gk * sak] : 0.f;
+    float ra[la.kN], rb[lb.kN];
+    la.fetch(ra, 0);
+    lb.fetch(rb, 0);
+    int buf = 0;
+    __syncthreads(); // (a previous product's last readers)
+    for (int k0 = 0; k0 < q.K; k0 += TK, buf ^= 1) {
+        la.store(ra, As[buf]);
+        lb.store(rb, Bs[buf]);
+        __syncthreads(); // (the other buffer's readers passed the barrier before)
+        if (k0 + TK < q.K) {
+            la.fetch(ra, k0 + TK);
+            lb.fetch(rb, k0 + TK);
         }
-        for (int e = threadIdx.x; e < TK * TN; e += 256) {
-            const int kk = e / TN, nn = e - kk * TN;
-            const int gn = n0 + nn, gk = k0 + kk;
-            Bs[kk][nn] = (gn < N && gk < K) ? B[(long)gk * sbk + (long)gn * sbn] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
+#pragma unroll 8
         for (int kk = 0; kk < TK; kk++) {
-            float a[4], b[4];
+            float a[U], b[U];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                a[i] = As[kk][ty * 4 + i];
-                b[i] = Bs[kk][tx * 4 + i];
+            for (int i = 0; i < U; i++) {
+                a[i] = As[buf][kk][ty * U + i];
+                b[i] = Bs[buf][kk][tx * U + i];
             }
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < U; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++)
+                for (int j = 0; j < U; j++)
                     acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
-        __syncthreads();
+    }
+}
+
+// tiles of T x T, 256 threads
+template <int T, int TK>
+__global__ void __launch_bounds__(256) gemm_kernel(const __grid_constant__ GemmGroup g)
+{
+    constexpr int U = T / 16;
+    __shared__ __align__(16) float As[2][TK][T + 4];
+    __shared__ __align__(16) float Bs[2][TK][T + 4];
+    const int tid = threadIdx.x;
+    const int tile = blockIdx.x;
+    if (tile >= g.tiles) { // column sums, 32 columns per CTA (its first warp)
+        int j = (tile - g.tiles) * 32 + tid;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const ColSum& cs = g.cs[c];
+            if (tid < 32 && j >= 0 && j < cs.cols) {
+                const float s1 = col_sum(cs.dY, cs.rows, cs.cols, j);
+                cs.db[j] = cs.dY2 ? s1 + col_sum(cs.dY2, cs.rows2, cs.cols, j) : s1;
+            }
+            j -= (cs.cols + 31) / 32 * 32;
+        }
+        return;
+    }
+    int pi = 0;
+    while (pi + 1 < g.n && g.p[pi + 1].tile_begin <= tile)
+        pi++;
+    const GemmProblem& p = g.p[pi];
+    const int lt = tile - p.tile_begin;
+    const int m0 = lt / p.tiles_n * T, n0 = lt % p.tiles_n * T;
+    const int tx = tid & 15, ty = tid >> 4;
+    float acc[U][U], prev[U][U];
+#pragma unroll
+    for (int i = 0; i < U; i++)
+#pragma unroll
+        for (int j = 0; j < U; j++)
+            acc[i][j] = prev[i][j] = 0.f;
+    const int n_parts = p.part[1].K > 0 ? 2 : 1;
+    for (int h = 0; h < n_parts; h++) {
+        const GemmPart& q = p.part[h];
+        if (h == 1) { // the first product is complete
+#pragma unroll
+            for (int i = 0; i < U; i++)
+#pragma unroll
+                for (int j = 0; j < U; j++) {
+                    prev[i][j] = p.alpha * acc[i][j];
+                    acc[i][j] = 0.f;
+                }
+        }
+        if (q.sak == 1) {
+            if (q.sbk == 1)
+                gemm_part<T, TK, true, true>(q, m0, p.M, n0, p.N, As, Bs, acc);
+            else
+                gemm_part<T, TK, true, false>(q, m0, p.M, n0, p.N, As, Bs, acc);
+        } else {
+            if (q.sbk == 1)
+                gemm_part<T, TK, false, true>(q, m0, p.M, n0, p.N, As, Bs, acc);
+            else
+                gemm_part<T, TK, false, false>(q, m0, p.M, n0, p.N, As, Bs, acc);
+        }
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int gm = m0 + ty * 4 + i;
-        if (gm >= M)
+    for (int i = 0; i < U; i++) {
+        const int gm = m0 + ty * U + i;
+        if (gm >= p.M)
             continue;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int gn = n0 + tx * 4 + j;
-            if (gn >= N)
+        for (int j = 0; j < U; j++) {
+            const int gn = n0 + tx * U + j;
+            if (gn >= p.N)
                 continue;
-            float* c = C + (long)gm * ldc + gn;
-            *c = alpha * acc[i][j] + (beta != 0.f ? beta * *c : 0.f);
+            float* c = p.C + (long)gm * p.ldc + gn;
+            float v = p.alpha * acc[i][j] + (n_parts == 2 ? prev[i][j] : p.beta != 0.f ? p.beta * *c : 0.f);
+            if (p.bias) {
+                v = v + p.bias[gn];
+                v = p.relu ? fmaxf(v, 0.f) : v;
+            }
+            if (p.mask && !(p.mask[(long)gm * p.ldc + gn] > 0.f))
+                v = 0.f;
+            *c = v;
         }
     }
 }
@@ -212,9 +383,7 @@ __global__ void colsum_kernel(const float* __restrict__ dY, long rows, int cols,
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= cols)
         return;
-    float s = 0.f;
-    for (long i = 0; i < rows; i++)
-        s += dY[i * cols + j];
+    const float s = col_sum(dY, rows, cols, j);
     db[j] = accumulate ? db[j] + s : s;
 }
 
@@ -348,6 +517,59 @@ __global__ void topk_kernel(const float* __restrict__ S, long rows, int cols, in
 
 inline unsigned blocks(long n, int per) { return (unsigned)((n + per - 1) / per); }
 
+int device_sms()
+{
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
+}
+
+// numbers the tiles of g's problems and launches them with its column sums
+cudaError_t launch_gemms(GemmGroup& g, cudaStream_t st)
+{
+    auto count = [&](int t) {
+        long tiles = 0;
+        for (int i = 0; i < g.n; i++) {
+            GemmProblem& p = g.p[i];
+            p.tiles_n = (p.N + t - 1) / t;
+            p.tile_begin = (int)tiles;
+            tiles += (long)p.tiles_n * ((p.M + t - 1) / t);
+        }
+        return tiles;
+    };
+    int t = 64;
+    long tiles = count(t);
+    if (tiles < device_sms())
+        tiles = count(t = 32);
+    long grid = tiles;
+    for (const ColSum& c : g.cs)
+        grid += (c.cols + 31) / 32;
+    if (grid > 0x7FFFFFFFl)
+        return cudaErrorInvalidValue;
+    g.tiles = (int)tiles;
+    if (t == 64)
+        gemm_kernel<64, 32><<<(unsigned)grid, 256, 0, st>>>(g);
+    else
+        gemm_kernel<32, 64><<<(unsigned)grid, 256, 0, st>>>(g);
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    return cudaGetLastError();
+}
+
+GemmProblem gemm_problem(int M, int N, int K, float alpha, const float* A, long sam, long sak, const float* B, long sbk,
+                         long sbn, float beta, float* C, long ldc)
+{
+    GemmProblem p{};
+    p.M = M;
+    p.N = N;
+    p.alpha = alpha;
+    p.beta = beta;
+    p.part[0] = GemmPart{A, B, sam, sak, sbk, sbn, K};
+    p.C = C;
+    p.ldc = ldc;
+    return p;
+}
+
 } // namespace
 } // namespace gpuisac
 
@@ -376,15 +598,87 @@ int gpuisac_nn_gemm(int M, int N, int K, float alpha, const float* A, long sam, 
         return 2;
     if (M == 0 || N == 0)
         return 0;
-    // grid.y is limited to 65535 tiles: long M runs in slabs
-    const int slab = 65535 * TM;
-    for (int m0 = 0; m0 < M; m0 += slab) {
-        const int mm = M - m0 < slab ? M - m0 : slab;
-        dim3 grid((N + TN - 1) / TN, (mm + TM - 1) / TM);
-        gemm_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(mm, N, K, alpha, A + (long)m0 * sam, sam, sak, B, sbk,
-                                                            sbn, beta, C + (long)m0 * ldc, ldc);
-        g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-    }
+    GemmGroup g{};
+    g.n = 1;
+    g.p[0] = gemm_problem(M, N, K, alpha, A, sam, sak, B, sbk, sbn, beta, C, ldc);
+    return launch_gemms(g, (cudaStream_t)stream) == cudaSuccess ? 0 : 1;
+}
+
+// One training batch: the forward pass of particles and references, the
+// cross-entropy of their scores and its gradient.  Independent products of
+// particles and references share launches: nine kernels.
+int gpuisac_nn_loss_grad(const GpuisacNnTrain* t, void* stream)
+{
+    if (!t || !t->Xp || !t->Xr || !t->labels || !t->params || !t->grad || !t->loss || !t->work || t->n_in <= 0 ||
+        t->hidden <= 0 || t->emb <= 0 || t->n_part <= 0 || t->n_ref <= 0)
+        return 2;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int P = t->n_part, R = t->n_ref, I = t->n_in, H = t->hidden, E = t->emb;
+    const float *W1 = t->params, *b1 = W1 + (size_t)H * I, *W2 = b1 + H, *b2 = W2 + (size_t)E * H;
+    float *gW1 = t->grad, *gb1 = gW1 + (size_t)H * I, *gW2 = gb1 + H, *gb2 = gW2 + (size_t)E * H;
+    // rows of particles, then of references (one normalisation launch for both)
+    const size_t n = (size_t)P + R;
+    float* w = t->work;
+    auto take = [&](size_t k) {
+        float* r = w;
+        w += k;
+        return r;
+    };
+    float *Hb = take(n * H), *Z = take(n * E), *Eb = take(n * E), *nrm = take(n), *S = take((size_t)P * R),
+          *dS = take((size_t)P * R), *dE = take(n * E), *dZ = take(n * E), *dH = take(n * H);
+    const size_t rH = (size_t)P * H, rE = (size_t)P * E;
+    GemmGroup g{};
+    auto dense = [&](const float* X, int rows, int k, const float* W, int out, const float* b, int relu, float* Y) {
+        GemmProblem p = gemm_problem(rows, out, k, 1.f, X, k, 1, W, 1, k, 0.f, Y, out);
+        p.bias = b;
+        p.relu = relu;
+        return p;
+    };
+    // H = relu(X W1^T + b1), Z = H W2^T + b2, E = Z / |Z|
+    g.n = 2;
+    g.p[0] = dense(t->Xp, P, I, W1, H, b1, 1, Hb);
+    g.p[1] = dense(t->Xr, R, I, W1, H, b1, 1, Hb + rH);
+    if (launch_gemms(g, st) != cudaSuccess)
+        return 1;
+    g = GemmGroup{};
+    g.n = 1;
+    g.p[0] = dense(Hb, (int)n, H, W2, E, b2, 0, Z);
+    if (launch_gemms(g, st) != cudaSuccess)
+        return 1;
+    l2norm_kernel<<<blocks((long)n, 8), 256, 0, st>>>(Z, (long)n, E, Eb, nrm);
+    // S = scale Ep Er^T, its cross-entropy and dS
+    g = GemmGroup{};
+    g.n = 1;
+    g.p[0] = gemm_problem(P, R, E, t->scale, Eb, E, 1, Eb + rE, 1, E, 0.f, S, R);
+    if (launch_gemms(g, st) != cudaSuccess)
+        return 1;
+    softmax_xent_kernel<<<blocks(P, 8), 256, 0, st>>>(S, t->labels, P, R, t->loss, dS);
+    // dEp = scale dS Er, dEr = scale dS^T Ep
+    g = GemmGroup{};
+    g.n = 2;
+    g.p[0] = gemm_problem(P, E, R, t->scale, dS, R, 1, Eb + rE, E, 1, 0.f, dE, E);
+    g.p[1] = gemm_problem(R, E, P, t->scale, dS, 1, R, Eb, E, 1, 0.f, dE + rE, E);
+    if (launch_gemms(g, st) != cudaSuccess)
+        return 1;
+    l2norm_bwd_kernel<<<blocks((long)n, 8), 256, 0, st>>>(Eb, dE, nrm, (long)n, E, dZ);
+    // dH = dZ W2 where H > 0; gW2 = dZ^T H, particles then references
+    g = GemmGroup{};
+    g.n = 2;
+    g.p[0] = gemm_problem((int)n, H, E, 1.f, dZ, E, 1, W2, H, 1, 0.f, dH, H);
+    g.p[0].mask = Hb;
+    g.p[1] = gemm_problem(E, H, P, 1.f, dZ, 1, E, Hb, H, 1, 0.f, gW2, H);
+    g.p[1].part[1] = GemmPart{dZ + rE, Hb + rH, 1, E, H, 1, R};
+    g.cs[0] = ColSum{dZ, dZ + rE, P, R, E, gb2};
+    if (launch_gemms(g, st) != cudaSuccess)
+        return 1;
+    g = GemmGroup{};
+    g.n = 1;
+    g.p[0] = gemm_problem(H, I, P, 1.f, dH, 1, H, t->Xp, I, 1, 0.f, gW1, I);
+    g.p[0].part[1] = GemmPart{dH + rH, t->Xr, 1, H, I, 1, R};
+    g.cs[0] = ColSum{dH, dH + rH, P, R, H, gb1};
+    if (launch_gemms(g, st) != cudaSuccess)
+        return 1;
+    g_kernel_launches.fetch_add(3, std::memory_order_relaxed);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
@@ -414,7 +708,7 @@ int gpuisac_nn_colsum(const float* dY, long rows, int cols, float* db, int accum
 {
     if (!dY || !db || rows < 0 || cols <= 0)
         return 2;
-    colsum_kernel<<<blocks(cols, 128), 128, 0, (cudaStream_t)stream>>>(dY, rows, cols, db, accumulate);
+    colsum_kernel<<<blocks(cols, 32), 32, 0, (cudaStream_t)stream>>>(dY, rows, cols, db, accumulate);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }

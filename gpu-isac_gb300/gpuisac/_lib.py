@@ -46,7 +46,7 @@ EXPORTS = (
     "gpuisac_kernel_time", "gpuisac_multi_ref_align_device_noalloc", "gpuisac_multi_ref_align_groups_device",
     "gpuisac_align_proposals_device", "gpuisac_nn_features", "gpuisac_nn_gemm", "gpuisac_nn_bias_act",
     "gpuisac_nn_relu_backward", "gpuisac_nn_colsum", "gpuisac_nn_l2norm", "gpuisac_nn_l2norm_backward",
-    "gpuisac_nn_softmax_xent", "gpuisac_nn_adam", "gpuisac_nn_topk", "gpuisac_nn_col_stats",
+    "gpuisac_nn_softmax_xent", "gpuisac_nn_adam", "gpuisac_nn_topk", "gpuisac_nn_col_stats", "gpuisac_nn_loss_grad",
     "gpuisac_nn_affine_cols", "gpuisac_nn_group_max", "gpuisac_learned_align_device", "gpuisac_autotune_ccf",
     "gpuisac_ccf_tile_name", "gpuisac_nn_gemm_bf16", "gpuisac_assign_groups_device", "gpuisac_assign_groups",
     "gpuisac_ref_free_averages", "gpuisac_set_contraction", "gpuisac_get_contraction", "gpuisac_test_stall_ccf", "gpuisac_normalize_mask",
@@ -72,6 +72,14 @@ class GpuisacProposalNet(ctypes.Structure):
     _fields_ = [("nk", ctypes.c_uint), ("hidden", ctypes.c_uint), ("emb", ctypes.c_uint),
                 ("mu", ctypes.c_void_p), ("inv_sd", ctypes.c_void_p), ("W1", ctypes.c_void_p),
                 ("b1", ctypes.c_void_p), ("W2", ctypes.c_void_p), ("b2", ctypes.c_void_p)]
+
+
+class GpuisacNnTrain(ctypes.Structure):
+    """Mirror of GpuisacNnTrain (include/gpu_aln_pack.h): device pointers."""
+    _fields_ = [("n_in", ctypes.c_int), ("hidden", ctypes.c_int), ("emb", ctypes.c_int), ("n_part", ctypes.c_int),
+                ("n_ref", ctypes.c_int), ("scale", ctypes.c_float), ("Xp", ctypes.c_void_p),
+                ("labels", ctypes.c_void_p), ("Xr", ctypes.c_void_p), ("params", ctypes.c_void_p),
+                ("grad", ctypes.c_void_p), ("loss", ctypes.c_void_p), ("work", ctypes.c_void_p)]
 
 
 class GpuIsacError(RuntimeError):
@@ -167,6 +175,8 @@ def load(path: str | None = None) -> ctypes.CDLL:
     L.gpuisac_nn_l2norm.argtypes = [vp, cl, ci, vp, vp, vp]
     L.gpuisac_nn_l2norm_backward.argtypes = [vp, vp, vp, cl, ci, vp, vp]
     L.gpuisac_nn_softmax_xent.argtypes = [vp, vp, cl, ci, vp, vp, vp]
+    L.gpuisac_nn_loss_grad.argtypes = [ctypes.POINTER(GpuisacNnTrain), vp]
+    L.gpuisac_nn_loss_grad.restype = ci
     L.gpuisac_nn_adam.argtypes = [vp, vp, vp, vp, cl, cf, cf, cf, cf, cf, ci, vp]
     L.gpuisac_nn_topk.argtypes = [vp, cl, ci, ci, vp, vp]
     for name in ("gpuisac_align_proposals_device", "gpuisac_nn_features", "gpuisac_nn_gemm", "gpuisac_nn_bias_act",

@@ -264,56 +264,18 @@ class ProposalNet:
         return out
 
     # ---------------------------------------------------------------- training
-    def _backward_batch(self, X, H, E, nrm, dE, tag, accumulate):
-        """gradients of one batch's embeddings dE into self.grad"""
-        L = _lib.load()
-        st = _stream(self.device)
-        n = X.shape[0]
-        acc = 1.0 if accumulate else 0.0
-        W2 = self.view(self.flat, "W2")
-        gW1, gb1 = self.view(self.grad, "W1"), self.view(self.grad, "b1")
-        gW2, gb2 = self.view(self.grad, "W2"), self.view(self.grad, "b2")
-        dZ = self._buf(tag + "dZ", (n, self.emb))
-        dH = self._buf(tag + "dH", (n, self.hidden))
-        _call(L, "gpuisac_nn_l2norm_backward", E.data_ptr(), dE.data_ptr(), nrm.data_ptr(), n, self.emb,
-              dZ.data_ptr(), st)
-        # gW2 (+)= dZ^T H: A(m, k) = dZ[k][m], B(k, j) = H[k][j]
-        _call(L, "gpuisac_nn_gemm", self.emb, self.hidden, n, 1.0, dZ.data_ptr(), 1, self.emb, H.data_ptr(),
-              self.hidden, 1, acc, gW2.data_ptr(), self.hidden, st)
-        _call(L, "gpuisac_nn_colsum", dZ.data_ptr(), n, self.emb, gb2.data_ptr(), int(accumulate), st)
-        # dH = dZ W2: B(k, j) = W2[k][j]
-        _call(L, "gpuisac_nn_gemm", n, self.hidden, self.emb, 1.0, dZ.data_ptr(), self.emb, 1, W2.data_ptr(),
-              self.hidden, 1, 0.0, dH.data_ptr(), self.hidden, st)
-        _call(L, "gpuisac_nn_relu_backward", dH.data_ptr(), H.data_ptr(), n * self.hidden, st)
-        # gW1 (+)= dH^T X
-        _call(L, "gpuisac_nn_gemm", self.hidden, self.n_in, n, 1.0, dH.data_ptr(), 1, self.hidden, X.data_ptr(),
-              self.n_in, 1, acc, gW1.data_ptr(), self.n_in, st)
-        _call(L, "gpuisac_nn_colsum", dH.data_ptr(), n, self.hidden, gb1.data_ptr(), int(accumulate), st)
-
     def loss_and_grad(self, Xp, labels, Xr):
         """mean cross-entropy of one particle batch against every reference;
         leaves the gradient in self.grad and returns the per-particle loss
         (device tensor)."""
-        L = _lib.load()
-        st = _stream(self.device)
+        from ._lib import GpuisacNnTrain
         B, R = Xp.shape[0], Xr.shape[0]
-        Hp, _, Ep, np_ = self._forward(Xp, "p")
-        Hr, _, Er, nr_ = self._forward(Xr, "r")
-        S = self._buf("S", (B, R))
-        dS = self._buf("dS", (B, R))
         loss = self._buf("loss", (B,))
-        dEp = self._buf("dEp", (B, self.emb))
-        dEr = self._buf("dEr", (R, self.emb))
-        self.scores(Ep, Er, out=S)
-        _call(L, "gpuisac_nn_softmax_xent", S.data_ptr(), labels.data_ptr(), B, R, loss.data_ptr(), dS.data_ptr(),
-              st)
-        # dEp = scale dS Er;  dEr = scale dS^T Ep
-        _call(L, "gpuisac_nn_gemm", B, self.emb, R, self.scale, dS.data_ptr(), R, 1, Er.data_ptr(), self.emb, 1,
-              0.0, dEp.data_ptr(), self.emb, st)
-        _call(L, "gpuisac_nn_gemm", R, self.emb, B, self.scale, dS.data_ptr(), 1, R, Ep.data_ptr(), self.emb, 1,
-              0.0, dEr.data_ptr(), self.emb, st)
-        self._backward_batch(Xp, Hp, Ep, np_, dEp, "p", False)
-        self._backward_batch(Xr, Hr, Er, nr_, dEr, "r", True)
+        work = self._buf("train", ((B + R) * (2 * self.hidden + 4 * self.emb + 1) + 2 * B * R,))
+        t = GpuisacNnTrain(self.n_in, self.hidden, self.emb, B, R, self.scale, Xp.data_ptr(), labels.data_ptr(),
+                           Xr.data_ptr(), self.flat.data_ptr(), self.grad.data_ptr(), loss.data_ptr(),
+                           work.data_ptr())
+        _call(_lib.load(), "gpuisac_nn_loss_grad", ctypes.byref(t), _stream(self.device))
         return loss
 
     def adam(self, lr: float, b1: float = 0.9, b2: float = 0.999, eps: float = 1e-8, wd: float = 0.0):

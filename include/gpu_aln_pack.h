@@ -411,6 +411,22 @@ int gpuisac_nn_softmax_xent(const float *S, const int *labels, long rows, int co
 /* AdamW step (bias-corrected, step >= 1) on n parameters. */
 int gpuisac_nn_adam(float *p, const float *g, float *m, float *v, long n, float lr, float b1, float b2, float eps,
                     float wd, int step, void *stream);
+/* One training batch of the proposal network (all device pointers, row-major
+ * FP32): params and grad hold W1 [hidden][n_in], b1, W2 [emb][hidden], b2 one
+ * after another; loss [n_part]; work: (n_part + n_ref) * (2 * hidden +
+ * 4 * emb + 1) + 2 * n_part * n_ref floats. */
+typedef struct GpuisacNnTrain {
+    int n_in, hidden, emb, n_part, n_ref;
+    float scale;
+    const float *Xp;    /* [n_part][n_in] standardised particle features */
+    const int *labels;  /* [n_part] */
+    const float *Xr;    /* [n_ref][n_in] */
+    const float *params;
+    float *grad, *loss, *work;
+} GpuisacNnTrain;
+/* loss[i] = cross-entropy of particle i's scores (scale * e_p . e_r) against
+ * its label, and the gradient of their mean in grad (overwritten). */
+int gpuisac_nn_loss_grad(const GpuisacNnTrain *t, void *stream);
 /* idx[i][0..k-1] = columns of the k largest S[i][.], best first (cols <= 1024, k <= 64). */
 int gpuisac_nn_topk(const float *S, long rows, int cols, int k, unsigned int *idx, void *stream);
 
