@@ -1077,7 +1077,12 @@ cudaError_t launch_ccf_peak(const float2* sbj_sp, const float2* ref_sp, const fl
     CcfWork w{};
     w.groups = nullptr;
     w.n_groups = 1;
-    w.ppc = tile.ppc;
+    // Particles per work item: the tile's, or fewer where that leaves items for
+    // less than four rounds of the SMs (an 8 x 4 alignment is one item of 8
+    // particles on one SM otherwise: 145 us, 40 as 8 items)
+    const unsigned tiles = (n_ref + qt - 1) / qt;
+    const size_t share = (size_t)n_part * tiles / (4 * (size_t)persistent_grid(~0u, 1));
+    w.ppc = (unsigned)std::min<size_t>(tile.ppc, std::max<size_t>(1, share));
     CcfGroup& g = w.one;
     g.sbj_sp = sbj_sp;
     g.ref_sp = ref_sp;
@@ -1089,7 +1094,7 @@ cudaError_t launch_ccf_peak(const float2* sbj_sp, const float2* ref_sp, const fl
     g.n_ref = n_ref;
     g.p_total = p_total;
     g.item_begin = 0;
-    g.ref_tiles = (n_ref + qt - 1) / qt;
+    g.ref_tiles = tiles;
     g.rule = rule;
     w.n_items = g.ref_tiles * ((n_part + w.ppc - 1) / w.ppc);
     w.max_ref = n_ref;

@@ -1,5 +1,6 @@
 """The warp-specialised CCF kernel at the edges of its particle streams,
-reference pairs and shift groups (odd particle counts, reference tiles with
+reference pairs and shift groups (odd particle counts, work items of one and
+of several particles, reference tiles with
 one, two or three references, fewer shifts than a group, one shift group per
 work item, both group sizes) against the general kernel, bit for bit: both run
 the same sums in the same order."""
@@ -13,7 +14,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("P,R,NR,rng", [(1, 1, 5, 0.0), (1, 5, 29, 2.0), (2, 3, 7, 1.0), (3, 2, 29, 1.0), (9, 6, 12, 1.0),
                                         (17, 9, 30, 2.0), (8, 4, 1, 0.0), (7, 7, 37, 1.0), (10, 11, 45, 2.0),
-                                        (1, 1300, 3, 0.0), (5, 700, 40, 0.0)])
+                                        (1, 1300, 3, 0.0), (5, 700, 40, 0.0),
+                                        # work items of 2, 8 (the last of one particle) and 4 particles
+                                        (1301, 3, 5, 1.0), (1217, 14, 3, 1.0), (701, 13, 37, 0.0)])
 def test_streams_equal_general_kernel(gpulib, cuda, monkeypatch, P, R, NR, rng):
     import torch
     from gpuisac.align import multi_ref_align_device
