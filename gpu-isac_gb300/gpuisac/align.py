@@ -61,12 +61,22 @@ def ptr_array(stack: np.ndarray):
     reference's get_c_ptr_array, bin/sp_isac2_gpu.py:166-174)."""
     assert stack.flags["C_CONTIGUOUS"] and stack.dtype == np.float32
     n = stack.shape[0]
-    step = stack.strides[0]
-    base = stack.ctypes.data
-    arr = (float_ptr * max(n, 1))()
-    for i in range(n):
-        arr[i] = ctypes.cast(base + i * step, float_ptr)
-    return arr
+    ptrs = np.zeros(max(n, 1), np.uintp)
+    ptrs[:n] = stack.ctypes.data + np.arange(n, dtype=np.uintp) * np.uintp(stack.strides[0])
+    return (float_ptr * max(n, 1)).from_buffer(ptrs)
+
+
+# AlignParam (include/gpu_aln_pack.h) as a numpy record
+PARAM_DTYPE = np.dtype({"names": ["sbj_id", "ref_id", "shift_x", "shift_y", "angle", "mirror"],
+                        "formats": ["i4", "i4", "f4", "f4", "f4", "?"], "offsets": [0, 4, 8, 12, 16, 20],
+                        "itemsize": ctypes.sizeof(_lib.AlignParam)})
+
+
+def param_view(params, n: int) -> np.ndarray:
+    """The library's AlignParam array at params (a pointer) as a writable numpy
+    record array; valid until gpu_clear."""
+    addr = ctypes.cast(params, ctypes.c_void_p).value
+    return np.frombuffer((ctypes.c_char * (n * PARAM_DTYPE.itemsize)).from_address(addr), PARAM_DTYPE, count=n)
 
 
 def multi_ref_align(particles: np.ndarray, refs: np.ndarray, ring_num: int, shift_rng_x: float,
@@ -105,9 +115,8 @@ def _multi_ref_align(particles, refs, ring_num, shift_rng_x, shift_rng_y, shift_
     try:
         if base_shifts is not None:
             bs = np.asarray(base_shifts, np.float32).reshape(P, 2)
-            for i in range(P):
-                params[i].shift_x = float(bs[i, 0])
-                params[i].shift_y = float(bs[i, 1])
+            view = param_view(params, P)
+            view["shift_x"], view["shift_y"] = bs[:, 0], bs[:, 1]
         sp, rp = ptr_array(particles), ptr_array(refs)
         L.multi_ref_align(sp, rp, peak_list.ctypes.data_as(float_ptr), d.ctypes.data_as(float_ptr), pitch,
                           mem_request)

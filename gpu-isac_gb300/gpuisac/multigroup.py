@@ -16,8 +16,8 @@ import math
 import numpy as np
 
 from . import _lib
-from ._lib import AlignParam, GpuIsacError
-from .align import make_config, ptr_array
+from ._lib import GpuIsacError
+from .align import make_config, param_view, ptr_array
 
 
 def multigroup_refinement(particles: np.ndarray, cid_list, ring_num: int, shift_rng_x: float, shift_rng_y: float,
@@ -38,17 +38,16 @@ def multigroup_refinement(particles: np.ndarray, cid_list, ring_num: int, shift_
         init_averages = np.stack([particles[cid == k].mean(0) for k in range(R)]).astype(np.float32)
     avgs = np.ascontiguousarray(init_averages, np.float32).reshape(R, D, D)
     cfg = make_config(P, R, D, ring_num, 256, 1.0, shift_rng_x, shift_rng_y, b"multigroup_aln")
-    cids = (ctypes.c_int * P)(*[int(c) for c in cid])
+    cids = (ctypes.c_int * P).from_buffer(cid.astype(np.int32))
     addr = L.ref_free_alignment_2D_init(ctypes.byref(cfg), ptr_array(particles), ptr_array(avgs), cids, device)
     if not addr:
         _lib.check(L)
         raise GpuIsacError("ref_free_alignment_2D_init returned NULL")
-    prm = ctypes.cast(addr, ctypes.POINTER(AlignParam))
+    prm = param_view(addr, P)
     try:
         if init_shifts is not None:
             sh = np.asarray(init_shifts, np.float32).reshape(P, 2)
-            for i in range(P):
-                prm[i].shift_x, prm[i].shift_y = float(sh[i, 0]), float(sh[i, 1])
+            prm["shift_x"], prm["shift_y"] = sh[:, 0], sh[:, 1]
         for i in range(num_iter):
             if cutoff_freq > 0.0:
                 freq = 0.1 + (cutoff_freq - 0.1) * i / float(num_iter - 1)
@@ -56,8 +55,7 @@ def multigroup_refinement(particles: np.ndarray, cid_list, ring_num: int, shift_
                 _lib.check(L)
             L.ref_free_alignment_2D()
             _lib.check(L)
-        out = np.array([(prm[i].angle, prm[i].shift_x, prm[i].shift_y, float(prm[i].mirror)) for i in range(P)],
-                       np.float32)
+        out = np.stack([prm["angle"], prm["shift_x"], prm["shift_y"], prm["mirror"]], 1).astype(np.float32)
         final = None
         if return_averages:
             final = np.zeros((R, D, D), np.float32)

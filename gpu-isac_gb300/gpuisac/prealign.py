@@ -9,8 +9,8 @@ import ctypes
 import numpy as np
 
 from . import _lib
-from ._lib import AlignParam, GpuIsacError
-from .align import make_config, ptr_array
+from ._lib import GpuIsacError
+from .align import make_config, param_view, ptr_array
 
 
 def pre_align(particles: np.ndarray, ref: np.ndarray, ring_num: int, shift_range: float, shift_step: float = 1.0,
@@ -31,12 +31,11 @@ def pre_align(particles: np.ndarray, ref: np.ndarray, ring_num: int, shift_range
     if not addr:
         _lib.check(L)
         raise GpuIsacError("pre_align_init returned NULL")
-    prm = ctypes.cast(addr, ctypes.POINTER(AlignParam))
+    prm = param_view(addr, P)
     try:
         if base_shifts is not None:
             bs = np.asarray(base_shifts, np.float32).reshape(P, 2)
-            for i in range(P):
-                prm[i].shift_x, prm[i].shift_y = float(bs[i, 0]), float(bs[i, 1])
+            prm["shift_x"], prm["shift_y"] = bs[:, 0], bs[:, 1]
         rp = ptr_array(ref)
         L.pre_align_fetch(rp, 1, b"ref_batch")
         _lib.check(L)
@@ -52,8 +51,7 @@ def pre_align(particles: np.ndarray, ref: np.ndarray, ring_num: int, shift_range
                     _lib.check(L)
                 L.pre_align_run(s0, s1)
                 _lib.check(L)
-        out = np.array([[prm[i].shift_x, prm[i].shift_y, prm[i].angle, float(prm[i].mirror)] for i in range(P)],
-                       np.float32)
+        out = np.stack([prm["shift_x"], prm["shift_y"], prm["angle"], prm["mirror"]], 1).astype(np.float32)
     finally:
         if not keep_session:
             L.gpu_clear()
