@@ -1062,6 +1062,15 @@ cudaError_t launch_ccf_peak_work(const CcfWork& w_in, int variant, const float2*
     return cudaGetLastError();
 }
 
+// The tile's particles per work item, or fewer where that leaves items for less
+// than four rounds of the SMs (an 8 x 4 alignment is one item of 8 particles on
+// one SM otherwise: 145 us, 40 as 8 items).
+unsigned ccf_particles_per_item(const CcfTile& tile, size_t particle_tiles)
+{
+    const size_t share = particle_tiles / (4 * (size_t)persistent_grid(~0u, 1));
+    return (unsigned)std::min<size_t>(tile.ppc, std::max<size_t>(1, share));
+}
+
 cudaError_t launch_ccf_peak(const float2* sbj_sp, const float2* ref_sp, const float2* twiddle, unsigned ring_num,
                             unsigned n_shift, unsigned n_ref, unsigned n_part, unsigned p_global0, unsigned p_total,
                             const float2* shifts_f, const float2* base, float* d_out, float4* peak_out,
@@ -1077,12 +1086,8 @@ cudaError_t launch_ccf_peak(const float2* sbj_sp, const float2* ref_sp, const fl
     CcfWork w{};
     w.groups = nullptr;
     w.n_groups = 1;
-    // Particles per work item: the tile's, or fewer where that leaves items for
-    // less than four rounds of the SMs (an 8 x 4 alignment is one item of 8
-    // particles on one SM otherwise: 145 us, 40 as 8 items)
     const unsigned tiles = (n_ref + qt - 1) / qt;
-    const size_t share = (size_t)n_part * tiles / (4 * (size_t)persistent_grid(~0u, 1));
-    w.ppc = (unsigned)std::min<size_t>(tile.ppc, std::max<size_t>(1, share));
+    w.ppc = ccf_particles_per_item(tile, (size_t)n_part * tiles);
     CcfGroup& g = w.one;
     g.sbj_sp = sbj_sp;
     g.ref_sp = ref_sp;

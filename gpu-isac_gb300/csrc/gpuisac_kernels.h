@@ -291,6 +291,9 @@ int ccf_variant(unsigned ring_num, bool aligned, unsigned n_shift = 0);
 // references per work item of that variant
 unsigned ccf_refs_per_item(unsigned ring_num, int variant);
 
+// particles per work item for a launch of that many (particle, reference tile) pairs
+unsigned ccf_particles_per_item(const CcfTile& tile, size_t particle_tiles);
+
 // persistent launch over the work items of w
 cudaError_t launch_ccf_peak_work(const CcfWork& w, int variant, const float2* twiddle, unsigned ring_num,
                                  unsigned n_shift, const float2* shifts_f, unsigned* err, cudaStream_t stream);

@@ -21,6 +21,10 @@ struct NvtxRange {
     NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Spectra held at a time by the sessions that run init / clear cycles
+// (pre-alignment, multigroup).
+constexpr size_t kSpectraBytes = (size_t)1 << 30;
+
 // failure-path tests (gpuisac_test_fail_alloc): true while injected failures
 // of workspace allocations are pending; each call consumes one
 bool take_injected_alloc_failure();

@@ -348,12 +348,12 @@ int run_iteration(MgState& s)
     const size_t per_part = row * S * sizeof(float2);
     const unsigned chunk = (unsigned)std::max<size_t>(
         1, std::min<size_t>({(size_t)P, (size_t)(0.4 * (double)(free_b + s.sbj_sp.n * sizeof(float2))) / per_part,
-                             (size_t)16384}));
+                             std::max<size_t>(1, kSpectraBytes / per_part)}));
     MG_CK(s.sbj_sp.ensure(row * S * chunk));
 
     // group table: one entry per (class, chunk) segment, one reference each
     const CcfTile tile = ccf_tile(NR, S, true);
-    const unsigned ppc = tile.ppc;
+    const unsigned ppc = ccf_particles_per_item(tile, chunk);
     struct ChunkWork {
         unsigned c0, c, first, n_groups, n_items;
     };

@@ -327,7 +327,8 @@ void pre_align_run(int start_idx, int stop_idx)
         PRE_CK(cudaMemGetInfo(&free_b, &total_b));
         const size_t per_part = row * g.S * sizeof(float2);
         const unsigned chunk = (unsigned)std::max<size_t>(
-            1, std::min<size_t>({(size_t)n, (size_t)(0.4 * (double)free_b) / per_part, (size_t)16384}));
+            1, std::min<size_t>({(size_t)n, (size_t)(0.4 * (double)free_b) / per_part,
+                                 std::max<size_t>(1, kSpectraBytes / per_part)}));
         PRE_CK(s.sbj_sp.ensure(row * g.S * chunk));
         StackDesc sbjs{s.sbj.p, s.capacity, g.D, s.capacity, tex};
         const unsigned long long* sbj_tx = nullptr;
