@@ -221,10 +221,14 @@ __device__ __forceinline__ float half_of(f32x2 p)
 
 // fft_peak_regs' search on half H of a pair of transforms: x[perm16(k2)] holds
 // the correlations at angle l + 16 k2 (re normal, im mirrored); wf: 256 floats
-// of the group's workspace
+// of the group's workspace.  best (or null): the largest value any group has
+// found for the same pair so far; a transform below it cannot be the pair's
+// answer and skips the index search.  Groups write it without order: a lost
+// update only makes the bound weaker.
 template <int H>
 __device__ __forceinline__ void peak_two(const Cx2 (&x)[16], float* wf, int l, unsigned gmask, unsigned s,
-                                         unsigned n_shift, PeakState& st, unsigned rule)
+                                         unsigned n_shift, PeakState& st, unsigned rule,
+                                         volatile float* best = nullptr)
 {
     if (rule == kPeakPreAlign && s == 0 && st.bv == 0.f && st.bh == 0 && st.bt == 0) {
         // the starting index (normal, shift 0, angle 0) stays the answer when
@@ -255,6 +259,14 @@ __device__ __forceinline__ void peak_two(const Cx2 (&x)[16], float* wf, int l, u
         v = fmaxf(v, __shfl_xor_sync(gmask, v, off));
     if (!(v >= st.bv))
         return;
+    if (best) {
+        // (one lane's reading for the whole group: the branch stays group-uniform)
+        const float bound = __shfl_sync(gmask, l == 0 ? *best : 0.f, 0, 16);
+        if (v < bound)
+            return;
+        if (l == 0 && v > bound)
+            *best = v;
+    }
     const bool mir = !__any_sync(gmask, vn == v);
     unsigned t = 0xffffffffu;
 #pragma unroll
@@ -292,7 +304,7 @@ __device__ __forceinline__ void fft_peak_two(ulonglong2* gz, const float2* twl, 
         const ulonglong2 v = gz[l + 16 * m];
         x[m] = Cx2{v.x, v.y};
     }
-    ifft256_two(x, gz, twl, l, gmask);
+    ifft256_two<false>(x, gz, twl, l, gmask);
     float* const wf = reinterpret_cast<float*>(gz);
     peak_two<0>(x, wf, l, gmask, s, n_shift, sa, rule);
     if (two)

@@ -338,43 +338,53 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ccf_mma_kernel(SplitMmaWork w,
 
 // ============================================================================
 // inverse FFT + peak search of the pair spectra Z, one (particle, reference)
-// per work item, one 16-thread group per shift of a block (w.block groups, up
-// to kSplitMaxBlock = 49, in whole warps), plus one control warp.  The units
-// (item, shift block) stream through one shared buffer of ring sums in
-// kZfftParts parts (of 128 / kZfftParts slots each): the control warp copies a
-// part of unit u + 1 in as soon as every group has taken its values of that
-// part of unit u into registers (mbarriers `empty`), so several copies can be
-// in flight and they overlap the FFTs; each group then transforms in its own
-// workspace and runs on without waiting for the others.
+// per work item, one 16-thread group per two shifts of a block (up to
+// kSplitMaxBlock = 49 shifts, 25 groups; the two transforms in the halves of
+// packed registers, ifft256_two), plus one control warp.  The units (item,
+// shift block) stream through a ring of kZfftBufs shared buffers, each half a
+// unit of ring sums (64 slots): the control warp refills a buffer as soon as
+// every group has taken its values into registers (mbarriers `empty`); three
+// buffers keep a copy in flight while the groups read and hand over a unit.
+// Each group then transforms in its own workspace and runs on without waiting
+// for the others.
 // A finished item's group bests are parked in one of kZfftRing slot sets
 // (mbarrier `parked`); the control warp merges them, writes the outputs and
 // hands the set back (mbarrier `freed`).
+//
+// What bounds it: the delivery of the ring sums (2 KB a pair and shift, read
+// once: 60 GB on 3,000 x 200 pairs at 49 shifts, 4.7 TB/s, 0.70 of the measured
+// copy bandwidth).  One shift per group took 362 instructions a transform and
+// 15.64 ms there; two shifts per group, and the index search only for
+// transforms that reach the pair's best so far, 14.24; the exchange through a
+// workspace of half the size, which makes room for the third buffer, 12.66
+// (12.93 with two).  150 x 300 at 61 rings, 81 shifts: 2.04 -> 1.63.
 constexpr int kZfftCtlThreads = 32;
 constexpr unsigned kZfftRing = 4;
-constexpr int kZfftParts = 2; // divides 8: a lane's 8 slots l + 16 m split evenly (4 parts: FFT kernel 261 -> 289 ms)
-__host__ __device__ constexpr unsigned zfft_group_threads(unsigned groups) { return (16 * groups + 31) / 32 * 32; }
-__host__ __device__ constexpr size_t zfft_zbuf_bytes(unsigned zw)
-{
-    return ((size_t)kRingLen * zw * sizeof(float2) + 15) / 16 * 16;
-}
+constexpr int kZfftParts = 2; // of a unit; divides 8: a lane's 8 slots l + 16 m split evenly
+constexpr unsigned kZfftBufs = 3;
+__host__ __device__ constexpr unsigned zfft_groups(unsigned block) { return (block + 1) / 2; }
+__host__ __device__ constexpr unsigned zfft_group_threads(unsigned block) { return (16 * zfft_groups(block) + 31) / 32 * 32; }
+// one part of a unit: [128 / kZfftParts slots][zw shifts][a, b] float2
+__host__ __device__ constexpr size_t zfft_part_bytes(unsigned zw) { return (size_t)kRingLen / kZfftParts * zw * sizeof(float2); }
 
 __global__ void __launch_bounds__(zfft_group_threads(kSplitMaxBlock) + kZfftCtlThreads, 1)
 zfft_peak_kernel(SplitFftWork w, const float2* __restrict__ twiddle, unsigned* __restrict__ err)
 {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    const unsigned groups = w.block;
+    const unsigned groups = zfft_groups(w.block);
     const unsigned gthreads = 16 * groups;
-    const bool ctl = threadIdx.x >= zfft_group_threads(groups);
+    const bool ctl = threadIdx.x >= zfft_group_threads(w.block);
     const size_t unit_elems = (size_t)kRingLen * w.zw;
-    float2* const zb = reinterpret_cast<float2*>(smem_raw);                                // [128][zw][a, b]
-    float2* const wsp = reinterpret_cast<float2*>(smem_raw + zfft_zbuf_bytes(w.zw));       // [groups][kPairStride]
-    float2* const tw = wsp + (size_t)groups * kPairStride;                                 // [16][kTwRow]
+    const uint32_t part_bytes = (uint32_t)zfft_part_bytes(w.zw); // (a multiple of 1 KiB)
+    f32x2* const wsp = reinterpret_cast<f32x2*>(smem_raw + kZfftBufs * part_bytes);        // [groups][kPairStride]
+    float2* const tw = reinterpret_cast<float2*>(wsp + (size_t)groups * kPairStride);      // [16][kTwRow]
     PeakSlot* const slots = reinterpret_cast<PeakSlot*>(tw + 16 * kTwRow);                 // [kZfftRing][64]
-    uint64_t* const full = reinterpret_cast<uint64_t*>(slots + kZfftRing * 64); // [kZfftParts]
-    uint64_t* const empty = full + kZfftParts;     // [kZfftParts]
-    uint64_t* const parked = empty + kZfftParts;   // [kZfftRing]
+    uint64_t* const full = reinterpret_cast<uint64_t*>(slots + kZfftRing * 64); // [kZfftBufs]
+    uint64_t* const empty = full + kZfftBufs;      // [kZfftBufs]
+    uint64_t* const parked = empty + kZfftBufs;    // [kZfftRing]
     uint64_t* const freed = parked + kZfftRing;    // [kZfftRing]
     volatile int* const abort_flag = reinterpret_cast<volatile int*>(freed + kZfftRing);
+    volatile float* const bests = reinterpret_cast<volatile float*>(abort_flag + 1); // [kZfftRing] of each set's pair
 
     const int tid = threadIdx.x;
     const unsigned n_items = w.n_part * w.n_ref;
@@ -386,13 +396,14 @@ zfft_peak_kernel(SplitFftWork w, const float2* __restrict__ twiddle, unsigned* _
         tw[tl * kTwRow + tj] = make_float2(t.x, t.y * -1.f);
     }
     if (tid == 0) {
-        for (int h = 0; h < kZfftParts; h++) {
-            mbar_init(full + h, 1);
-            mbar_init(empty + h, gthreads);
+        for (unsigned i = 0; i < kZfftBufs; i++) {
+            mbar_init(full + i, 1);
+            mbar_init(empty + i, gthreads);
         }
         for (unsigned i = 0; i < kZfftRing; i++) {
             mbar_init(parked + i, gthreads);
             mbar_init(freed + i, 1);
+            bests[i] = -3.40282e+038f;
         }
         *abort_flag = 0;
         mbar_fence_init();
@@ -408,18 +419,19 @@ zfft_peak_kernel(SplitFftWork w, const float2* __restrict__ twiddle, unsigned* _
     if (ctl) {
         // ---------------- control warp: copies, merges, outputs ----------------
         const int lane = tid & 31;
-        const size_t half = unit_elems / kZfftParts; // one part: [128 / kZfftParts][zw][a, b]
-        auto issue = [&](unsigned u, int h) {
+        // part q % kZfftParts of unit q / kZfftParts into buffer q % kZfftBufs
+        const unsigned n_q = n_units * kZfftParts;
+        auto issue = [&](unsigned q) {
             if (w.test_stall)
                 return; // failure-path test: no copies
-            const unsigned item = unit_item(u), b = u % w.n_blocks;
-            const uint32_t bytes = (uint32_t)(half * sizeof(float2));
-            const size_t at = ((size_t)item * w.n_blocks + b) * unit_elems + h * half;
-            if (!GPUISAC_IN_BOUNDS(kChkZfftZ, at + half - 1, (size_t)n_items * w.n_blocks * unit_elems))
+            const unsigned u = q / kZfftParts, h = q % kZfftParts, buf = q % kZfftBufs;
+            const size_t at = ((size_t)unit_item(u) * w.n_blocks + u % w.n_blocks) * unit_elems +
+                              h * (unit_elems / kZfftParts);
+            if (!GPUISAC_IN_BOUNDS(kChkZfftZ, at + unit_elems / kZfftParts - 1, (size_t)n_items * w.n_blocks * unit_elems))
                 return; // (checked build) the groups' bounded wait reports the failure
             fence_proxy_async();
-            mbar_expect_tx(full + h, bytes);
-            bulk_g2s(zb + h * half, w.z + at, bytes, full + h);
+            mbar_expect_tx(full + buf, part_bytes);
+            bulk_g2s(smem_raw + buf * part_bytes, w.z + at, part_bytes, full + buf);
         };
         // the groups' parked bests of a finished item, reduced in the
         // reference's order (better(); equal entries: the lower group, which
@@ -467,53 +479,54 @@ zfft_peak_kernel(SplitFftWork w, const float2* __restrict__ twiddle, unsigned* _
             }
         };
         bool failed = false;
-        unsigned issued[kZfftParts] = {}, n_done = 0; // units issued per part
-        if (lane == 0 && n_units > 0)
-            for (int h = 0; h < kZfftParts; h++)
-                issue(0, h);
-        if (n_units > 0)
-            for (int h = 0; h < kZfftParts; h++)
-                issued[h] = 1;
-        for (unsigned u = 0; u < n_units; u++) {
-            // every group holds its unit-u values of a part: the part takes unit u + 1
-            bool ok = true;
-#pragma unroll
+        unsigned issued = min(kZfftBufs, n_q), n_done = 0;
+        if (lane == 0)
+            for (unsigned q = 0; q < issued; q++)
+                issue(q);
+        // item n_done's groups have parked their bests: outputs, set handed back
+        auto finish = [&]() -> bool {
+            const unsigned set = n_done % kZfftRing;
+            const bool ok = mbar_wait_abort(parked + set, (n_done / kZfftRing) & 1u, abort_flag, wlim);
+            if (!__all_sync(0xffffffffu, ok))
+                return false;
+            merge(blockIdx.x + n_done * gridDim.x, slots + 64 * set);
+            __syncwarp();
+            if (lane == 0) {
+                bests[set] = -3.40282e+038f;
+                mbar_arrive(freed + set);
+            }
+            n_done++;
+            return true;
+        };
+        for (unsigned u = 0; u < n_units && !failed; u++) {
             for (int h = 0; h < kZfftParts; h++) {
+                // every group holds its values of the part: its buffer is free
+                const unsigned q = u * kZfftParts + h;
+                bool ok = true;
                 if (lane == 0) {
-                    ok = ok && mbar_wait_abort(empty + h, u & 1u, abort_flag, wlim);
-                    if (ok && u + 1 < n_units)
-                        issue(u + 1, h);
+                    ok = mbar_wait_abort(empty + q % kZfftBufs, (q / kZfftBufs) & 1u, abort_flag, wlim);
+                    if (ok && q + kZfftBufs < n_q)
+                        issue(q + kZfftBufs);
                 }
-                if (!__shfl_sync(0xffffffffu, ok, 0))
-                    break;
-                if (u + 1 < n_units)
-                    issued[h] = u + 2;
-            }
-            if (!__shfl_sync(0xffffffffu, ok, 0)) {
-                failed = true;
-                break;
-            }
-            if (u % w.n_blocks == w.n_blocks - 1) {
-                const unsigned set = n_done % kZfftRing;
-                ok = mbar_wait_abort(parked + set, (n_done / kZfftRing) & 1u, abort_flag, wlim);
-                if (!__all_sync(0xffffffffu, ok)) {
+                if (!__shfl_sync(0xffffffffu, ok, 0)) {
                     failed = true;
                     break;
                 }
-                merge(unit_item(u), slots + 64 * set);
-                __syncwarp();
-                if (lane == 0)
-                    mbar_arrive(freed + set);
-                n_done++;
+                issued = min(q + kZfftBufs + 1, n_q);
             }
+            // the item before this unit's (its bests are parked by now: the
+            // copies come first)
+            if (!failed && u && u % w.n_blocks == 0)
+                failed = !finish();
         }
+        if (!failed && n_units)
+            failed = !finish();
         if (failed && lane == 0) {
             *abort_flag = 1;
             atomicExch(err, 1u);
             // the last copies issued land before the CTA ends (bounded)
-            for (int h = 0; h < kZfftParts; h++)
-                if (issued[h] && !w.test_stall)
-                    mbar_wait(full + h, (issued[h] - 1) & 1u, wlim);
+            for (unsigned q = issued > kZfftBufs ? issued - kZfftBufs : 0; q < issued && !w.test_stall; q++)
+                mbar_wait(full + q % kZfftBufs, (q / kZfftBufs) & 1u, wlim);
         }
         return;
     }
@@ -523,27 +536,35 @@ zfft_peak_kernel(SplitFftWork w, const float2* __restrict__ twiddle, unsigned* _
     if ((unsigned)g >= groups)
         return; // the unused half of the last warp
     const unsigned gmask = 0xffffu << (tid & 16);
-    float2* const gz = wsp + (size_t)g * kPairStride;
+    f32x2* const gz = wsp + (size_t)g * kPairStride;
     PeakState st;
     st.reset(w.rule);
     unsigned n_done = 0;
     for (unsigned u = 0; u < n_units; u++) {
-        const unsigned b = u % w.n_blocks;
+        const unsigned b = u % w.n_blocks, set = n_done % kZfftRing;
         const unsigned s0 = b * w.block, nsb = min(w.block, w.n_shift - s0);
-        const bool has = (unsigned)g < nsb; // group-uniform
+        const bool has = 2 * (unsigned)g < nsb, two = 2 * (unsigned)g + 1 < nsb; // group-uniform
+        // the item's slot set is free, its best cleared
+        if (b == 0 && !mbar_wait_abort(freed + set, ((n_done / kZfftRing) & 1u) ^ 1u, abort_flag, wlim)) {
+            *abort_flag = 1;
+            atomicExch(err, 1u);
+            return;
+        }
         // the ring sums e = (ua, va, ub, vb) of slot l + 16 m (m < 8) give
         // Z[k] = (ua, ub) for k = l + 16 m (input m) and Z[256 - k] =
         // (vb, va), input 15 - m of lane (16 - l) mod 16; lane 0 keeps its
         // own: Z[256 - 16 m] is its input 16 - m, and slot 0 (the real
         // (F[0], F[128]) products) gives Z[0] and Z[128].  Slots l + 16 m
-        // are in part m / (8 / kZfftParts) of the buffer.
-        float2 x[16];
-        float p2 = 0.f;
-        const float4* z4 = reinterpret_cast<const float4*>(zb);
+        // are in part m / (8 / kZfftParts) of the buffer.  Two shifts side by
+        // side (the second zero past the block's last).
+        Cx2 x[16];
+        f32x2 p2 = 0;
         const int partner = (16 - l) & 15;
 #pragma unroll
         for (int h = 0; h < kZfftParts; h++) {
-            if (!mbar_wait_abort(full + h, u & 1u, abort_flag, wlim)) {
+            const unsigned q = u * kZfftParts + h, buf = q % kZfftBufs;
+            const float4* const z4 = reinterpret_cast<const float4*>(smem_raw + buf * part_bytes);
+            if (!mbar_wait_abort(full + buf, (q / kZfftBufs) & 1u, abort_flag, wlim)) {
                 *abort_flag = 1;
                 atomicExch(err, 1u);
                 return;
@@ -551,35 +572,36 @@ zfft_peak_kernel(SplitFftWork w, const float2* __restrict__ twiddle, unsigned* _
             if (has) {
 #pragma unroll
                 for (int m = h * (8 / kZfftParts); m < (h + 1) * (8 / kZfftParts); m++) {
-                    const float4 e = z4[(l + 16 * m) * w.zw + g];
-                    x[m] = make_float2(e.x, e.z);
-                    x[15 - m] =
-                        make_float2(__shfl_sync(gmask, e.w, partner, 16), __shfl_sync(gmask, e.y, partner, 16));
+                    const float4* const zp = z4 + (l + 16 * (m - h * (8 / kZfftParts))) * w.zw + 2 * g;
+                    const float4 e = zp[0], f = two ? zp[1] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    x[m] = Cx2{pack_f32x2(e.x, f.x), pack_f32x2(e.z, f.z)};
+                    x[15 - m] = Cx2{pack_f32x2(__shfl_sync(gmask, e.w, partner, 16), __shfl_sync(gmask, f.w, partner, 16)),
+                                    pack_f32x2(__shfl_sync(gmask, e.y, partner, 16), __shfl_sync(gmask, f.y, partner, 16))};
                     if (l == 0) {
                         if (m == 0) {
-                            const float p1 = 0.25f * (e.x + e.z + e.w + e.y);
-                            p2 = 0.25f * (e.x - e.z + e.w - e.y);
-                            x[0] = make_float2(p1, p1);
+                            const f32x2 p1 = pack_f32x2(0.25f * (e.x + e.z + e.w + e.y), 0.25f * (f.x + f.z + f.w + f.y));
+                            p2 = pack_f32x2(0.25f * (e.x - e.z + e.w - e.y), 0.25f * (f.x - f.z + f.w - f.y));
+                            x[0] = Cx2{p1, p1};
                         } else {
-                            x[16 - m] = make_float2(e.w, e.y);
+                            x[16 - m] = Cx2{pack_f32x2(e.w, f.w), pack_f32x2(e.y, f.y)};
                         }
                     }
                 }
             }
-            mbar_arrive(empty + h);
+            mbar_arrive(empty + buf);
         }
-        if (has && l == 0)
-            x[8] = make_float2(p2, p2);
-        if (has)
-            fft_peak_regs<true>(x, gz, tw + l * kTwRow, l, gmask, s0 + g, w.n_shift, st, w.rule);
+        if (has) {
+            if (l == 0)
+                x[8] = Cx2{p2, p2};
+            ifft256_two<true>(x, gz, tw + l * kTwRow, l, gmask);
+            float* const wf = reinterpret_cast<float*>(gz);
+            const unsigned s = s0 + 2 * g;
+            peak_two<0>(x, wf, l, gmask, s, w.n_shift, st, w.rule, bests + set);
+            if (two)
+                peak_two<1>(x, wf, l, gmask, s + 1, w.n_shift, st, w.rule, bests + set);
+        }
         if (b == w.n_blocks - 1) {
             // every shift of the pair has been searched: park the group's best
-            const unsigned set = n_done % kZfftRing;
-            if (!mbar_wait_abort(freed + set, ((n_done / kZfftRing) & 1u) ^ 1u, abort_flag, wlim)) {
-                *abort_flag = 1;
-                atomicExch(err, 1u);
-                return;
-            }
             park_slot(slots + 64 * set, st, g, l);
             mbar_arrive(parked + set);
             st.reset(w.rule);
@@ -611,8 +633,9 @@ static size_t mma_smem(const SplitPlan& p) { return (size_t)p.n_stages * mma_sta
 
 static size_t fft_smem(const SplitPlan& p)
 {
-    return zfft_zbuf_bytes(p.zw) + (size_t)p.fft_groups * kPairStride * sizeof(float2) + 16 * kTwRow * sizeof(float2) +
-           kZfftRing * 64 * sizeof(PeakSlot) + (2 * kZfftParts + 2 * kZfftRing) * sizeof(uint64_t) + 16;
+    return kZfftBufs * zfft_part_bytes(p.zw) + (size_t)p.fft_groups * kPairStride * sizeof(f32x2) +
+           16 * kTwRow * sizeof(float2) + kZfftRing * 64 * sizeof(PeakSlot) +
+           (2 * kZfftBufs + 2 * kZfftRing) * sizeof(uint64_t) + 16 + kZfftRing * sizeof(float);
 }
 
 bool split_plan(unsigned ring_num, unsigned n_shift, unsigned n_ref, SplitPlan& p)
@@ -625,7 +648,7 @@ bool split_plan(unsigned ring_num, unsigned n_shift, unsigned n_ref, SplitPlan& 
     p.kg = (ring_num + 7) / 8;
     p.rga = (2 * p.block + 7) / 8;
     p.rounds = 1;
-    p.fft_groups = p.block;
+    p.fft_groups = zfft_groups(p.block);
     const size_t cap = std::min<size_t>((size_t)smem_optin_max(), 227 * 1024);
     // references per tile: as many as N = 2 x refs <= 256 allows with at
     // least two operand stages, tiles balanced
@@ -742,7 +765,7 @@ cudaError_t launch_zfft_peak(const SplitPlan& p, const float2* z, unsigned n_par
     cudaError_t e;
     if ((e = opt_in_smem_k(zfft_peak_kernel, fs)) != cudaSuccess)
         return e;
-    zfft_peak_kernel<<<grid, zfft_group_threads(p.fft_groups) + kZfftCtlThreads, fs, stream>>>(fw, twiddle, err);
+    zfft_peak_kernel<<<grid, zfft_group_threads(p.block) + kZfftCtlThreads, fs, stream>>>(fw, twiddle, err);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaGetLastError();
 }

@@ -316,9 +316,11 @@ __device__ __forceinline__ void dft16_two(Cx2 (&x)[16])
         dft4_two(x[4 * k1], x[4 * k1 + 1], x[4 * k1 + 2], x[4 * k1 + 3]);
 }
 // In: x[m] = (z_A, z_B)[l + 16 m]; out: x[perm16(k2)] = (Z_A, Z_B)[l + 16 k2].
-// ws: 16 x 17 ulonglong2 (re pair, im pair); twl: thread l's row of kTwRow
-// float2 e^(+2 pi i l j / 256).
-__device__ __forceinline__ void ifft256_two(Cx2 (&x)[16], ulonglong2* ws, const float2* twl, int l, unsigned mask)
+// twl: thread l's row of kTwRow float2 e^(+2 pi i l j / 256).  ws: 16 x 17
+// entries of (re pair, im pair); kTwoPass: of one pair, the real parts and then
+// the imaginary parts exchanged through it (half the workspace).
+template <bool kTwoPass>
+__device__ __forceinline__ void ifft256_two(Cx2 (&x)[16], void* ws, const float2* twl, int l, unsigned mask)
 {
     dft16_two(x);
 #pragma unroll
@@ -327,14 +329,35 @@ __device__ __forceinline__ void ifft256_two(Cx2 (&x)[16], ulonglong2* ws, const 
         x[perm16(j)] = cmul2<false>(x[perm16(j)], pack_f32x2(w.x, w.x), pack_f32x2(w.y, w.y), pack_f32x2(-w.y, -w.y));
     }
     __syncwarp(mask);
+    if (kTwoPass) {
+        f32x2* const w1 = static_cast<f32x2*>(ws);
+        f32x2 re[16];
 #pragma unroll
-    for (int j = 0; j < 16; j++)
-        ws[l * 17 + j] = make_ulonglong2(x[perm16(j)].re, x[perm16(j)].im);
-    __syncwarp(mask);
+        for (int j = 0; j < 16; j++)
+            w1[l * 17 + j] = x[perm16(j)].re;
+        __syncwarp(mask);
 #pragma unroll
-    for (int n = 0; n < 16; n++) {
-        const ulonglong2 v = ws[n * 17 + l];
-        x[n] = Cx2{v.x, v.y};
+        for (int n = 0; n < 16; n++)
+            re[n] = w1[n * 17 + l];
+        __syncwarp(mask);
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+            w1[l * 17 + j] = x[perm16(j)].im;
+        __syncwarp(mask);
+#pragma unroll
+        for (int n = 0; n < 16; n++)
+            x[n] = Cx2{re[n], w1[n * 17 + l]};
+    } else {
+        ulonglong2* const w2 = static_cast<ulonglong2*>(ws);
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+            w2[l * 17 + j] = make_ulonglong2(x[perm16(j)].re, x[perm16(j)].im);
+        __syncwarp(mask);
+#pragma unroll
+        for (int n = 0; n < 16; n++) {
+            const ulonglong2 v = w2[n * 17 + l];
+            x[n] = Cx2{v.x, v.y};
+        }
     }
     __syncwarp(mask);
     dft16_two(x);
