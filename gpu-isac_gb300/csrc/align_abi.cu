@@ -459,6 +459,8 @@ int prepare_split_streams(Workspace& ws)
     return 0;
 }
 
+constexpr unsigned kSplitWaves = 8;
+
 int run_alignment_split(const Geometry& g, Workspace& ws, const StackDesc& refs, const StackDesc& sbjs,
                         const unsigned long long* ref_tx, const unsigned long long* sbj_tx, const float2* d_base,
                         float* d_out, float4* d_peak, float mem_request, cudaStream_t st, const HostOut* host)
@@ -489,13 +491,21 @@ int run_alignment_split(const Geometry& g, Workspace& ws, const StackDesc& refs,
     g_timer.end(K_SPECTRA, ev, hi);
     // particle chunk: two operand buffers and the pair spectra of a particle
     // (4.2 + 19.6 MB at 76², 35 rings, 49 shifts, 200 references) within the
-    // requested share of free memory, at most 2,048 particles
+    // requested share of free memory, and kSplitWaves rounds of the contraction's
+    // persistent CTAs (whole rounds: no part-filled last one): the operands of
+    // the first chunk are the ones nothing hides.  5,000 x 200 at 76² / 400 x 500
+    // at 128²: 47.2 / 16.9 ms with 8 rounds, 47.9 / 17.1 with 2, 47.5 / 17.3 with
+    // 16, 48.0 / 17.7 with chunks of 2,048 particles
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
+    int sms = 0, dev = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const double frac = (mem_request > 0.f && mem_request <= 1.f) ? mem_request : 0.9;
     const size_t budget = (size_t)((double)free_b * frac) / 2;
     const size_t per_part = 2 * split_sop_bytes(pl, 1) + split_z_bytes(pl, 1, g.R);
-    size_t chunk = std::max<size_t>(1, std::min<size_t>(budget / per_part, 2048));
+    const size_t rounds = std::max<size_t>(1, (size_t)kSplitWaves * std::max(sms, 1) / (pl.n_blocks * pl.n_rtiles));
+    size_t chunk = std::max<size_t>(1, std::min<size_t>({budget / per_part, rounds, (size_t)2048}));
     chunk = std::min<size_t>(chunk, g.P);
     const size_t sop_bytes = split_sop_bytes(pl, (unsigned)chunk);
     if (ws.sop.ensure(2 * sop_bytes) || ws.zsp.ensure(split_z_bytes(pl, (unsigned)chunk, g.R) / sizeof(float2)) ||
