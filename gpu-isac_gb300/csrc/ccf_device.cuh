@@ -294,9 +294,10 @@ __device__ __forceinline__ void peak_two(const Cx2 (&x)[16], float* wf, int l, u
 
 // inverse FFTs and peak searches of the pair spectra of two references in gz
 // (256 entries (re A, re B, im A, im B), natural order; then the workspace);
-// two: whether B is a reference
+// two: whether B is a reference; bests: peak_two's best of A's pair, then B's
 __device__ __forceinline__ void fft_peak_two(ulonglong2* gz, const float2* twl, int l, unsigned gmask, unsigned s,
-                                             unsigned n_shift, PeakState& sa, PeakState& sb, bool two, unsigned rule)
+                                             unsigned n_shift, PeakState& sa, PeakState& sb, bool two, unsigned rule,
+                                             volatile float* bests)
 {
     Cx2 x[16];
 #pragma unroll
@@ -306,9 +307,9 @@ __device__ __forceinline__ void fft_peak_two(ulonglong2* gz, const float2* twl, 
     }
     ifft256_two<false>(x, gz, twl, l, gmask);
     float* const wf = reinterpret_cast<float*>(gz);
-    peak_two<0>(x, wf, l, gmask, s, n_shift, sa, rule);
+    peak_two<0>(x, wf, l, gmask, s, n_shift, sa, rule, bests);
     if (two)
-        peak_two<1>(x, wf, l, gmask, s, n_shift, sb, rule);
+        peak_two<1>(x, wf, l, gmask, s, n_shift, sb, rule, bests + 1);
 }
 
 // named barrier `id` over n threads (id 0 with n = blockDim is __syncthreads)
@@ -360,9 +361,11 @@ template <int BAR = 0, int N = 256>
 __device__ __forceinline__ void merge_slots(PeakSlot* slots, int tid, int qt, int nsi, unsigned q0, unsigned n_ref,
                                             unsigned n_shift, unsigned pg, unsigned p_total, const float2* shifts_f,
                                             const float2* base, float* d_out, float4* peak_out,
-                                            unsigned rule = kPeakMref)
+                                            unsigned rule = kPeakMref, volatile float* bests = nullptr)
 {
     phase_sync<BAR, N>();
+    if (bests && tid < qt) // every slot of the pair is parked: its bound starts afresh
+        bests[tid] = -3.40282e+038f;
     if (tid < qt && q0 + tid < n_ref) {
         int best = tid;
         for (int i = 1; i < nsi; i++) {

@@ -315,6 +315,8 @@ ccf_peak_tmem_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned rin
 // meeting at every shift group; 150 x 300 at 61 rings 9.05 -> 8.40, 2,000 x 16
 // at 29 rings 1.18 -> 1.07).  On the way: two references per group in one team
 // 40.5 (four FFT warps wait on their own latency), two teams 36.4, halves 33.9.
+// The pair's best so far (`bests`) spares the transforms below it the index
+// search: 33.9 -> 33.2 ms (32 groups' search 35.4 -> 34.8).
 // Not kept: packed FMAs in the contraction (bit-identical; 35.7 against 33.9),
 // the staging area refilled in parts of a row as they are summed (47).
 constexpr int kWsBarC = 1;      // contraction side, item changes
@@ -369,7 +371,10 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
     float2* zbuf = sbuf + (size_t)NSI * nrp * kSlots;                  // [2][NP][kPairStride]
     float2* tw = zbuf + 2 * NP * kPairStride;                          // [16][kTwRow] per FFT lane
     PeakSlot* slots = reinterpret_cast<PeakSlot*>(tw + 16 * kTwRow);   // [team][16]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(slots + 32); // [half]
+    // the best of each reference slot's pair so far, by team and particle parity
+    // (a shift group reaches into two particles at most)
+    volatile float* const bests = reinterpret_cast<volatile float*>(slots + 32); // [team][parity][QT]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(slots + 32) + 8; // [half]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
     // the items after the current one, a ring of 4 (the contraction side can be
     // two items ahead of an FFT team): taken from the work counter
@@ -412,6 +417,8 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
     }
     for (unsigned i = tid; i < (unsigned)NSI * nrp * kSlots; i += NT)
         sbuf[i] = make_float2(0.f, 0.f); // the padding ring stays zero
+    if (tid < 16)
+        bests[tid] = -3.40282e+038f;
     if (warp == 0)
         tmem_alloc(tmem_slot, kTmemCols);
     if (tid == 0) {
@@ -678,7 +685,8 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
                 if (v < nrows && s < n_shift && q0 + (unsigned)g_ref < grp.n_ref) {
                     if constexpr (kTwo)
                         fft_peak_two(reinterpret_cast<ulonglong2*>(gz), tw + l * kTwRow, l, gmask, s, n_shift, st,
-                                     st2, q0 + (unsigned)g_ref + 1 < grp.n_ref, grp.rule);
+                                     st2, q0 + (unsigned)g_ref + 1 < grp.n_ref, grp.rule,
+                                     bests + (kSplit ? 0 : 8 * team + 4 * (pl & 1)) + g_ref);
                     else
                         fft_peak<true>(gz, tw + l * kTwRow, l, gmask, s, n_shift, st, grp.rule);
                 }
@@ -690,10 +698,12 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
                     const unsigned pg = grp.p_first + pb + kTeams * pc + team;
                     if (team == 0)
                         merge_slots<kWsBarF, NFT>(tslots, ftid, QT, NSI, q0, grp.n_ref, n_shift, pg, grp.p_total,
-                                                  shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule);
+                                                  shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule,
+                                                  bests + 4 * (pc & 1));
                     else
                         merge_slots<kWsBarF + 1, NFT>(tslots, ftid, QT, NSI, q0, grp.n_ref, n_shift, pg, grp.p_total,
-                                                      shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule);
+                                                      shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule,
+                                                      bests + 8 + 4 * (pc & 1));
                     pc++;
                 }
             }
@@ -703,7 +713,7 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
                 nbar_sync(kWsBarF + 2, NF);
                 if (team == 0)
                     merge_slots<kWsBarF, NFT>(slots, ftid, QT, 2 * NSI, q0, grp.n_ref, n_shift, grp.p_first + pb,
-                                              grp.p_total, shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule);
+                                              grp.p_total, shifts_f, grp.base, grp.d_out, grp.peak_out, grp.rule, bests);
                 nbar_sync(kWsBarF + 2, NF); // team 1's slots are free again
             }
             // (written by the contraction side before this item's first full buffer)
@@ -880,7 +890,7 @@ static size_t ws_smem_bytes(unsigned ring_num)
 {
     const unsigned nrp = 2 * ((ring_num + 1) / 2), nsi = ws_shifts_per_group(ring_num);
     return (size_t)nsi * nrp * kSlots * sizeof(float2) + 2 * nsi * 4 * kPairStride * sizeof(float2) +
-           16 * kTwRow * sizeof(float2) + 32 * sizeof(PeakSlot) + 16 + 32; // barriers, tensor-memory slot, next items
+           16 * kTwRow * sizeof(float2) + 32 * sizeof(PeakSlot) + 16 * sizeof(float) + 16 + 32; // bests, barriers, tensor-memory slot, next items
 }
 
 template <int CW, int NSI, int QR, bool kSplit = false>
