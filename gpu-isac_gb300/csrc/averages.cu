@@ -25,9 +25,11 @@
 //                            and every G-th row of the output, the quadratic
 //                            interpolation from shared memory, FP32 sums in
 //                            registers, one partial image per piece
-//  8. avg_finish_kernel      one CTA per group: its pieces summed in order,
-//                            times float(1/members); real 2D DFT, filter and
-//                            phase shift, inverse DFT
+//  8. avg_mean_kernel        each group's pieces summed in order, times
+//                            float(1/members)
+//  9. avg_rows_kernel, avg_cols_kernel, avg_inverse_kernel
+//                            with a filter or centring: real 2D DFT, filter
+//                            and phase shift, inverse DFT
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -48,8 +50,6 @@ constexpr unsigned kAvgChunk = 1024;      // particles per counting-sort chunk
 constexpr unsigned kSmemGroups = 16384;   // scatter: a chunk's group offsets in shared memory up to this
 constexpr unsigned kMaxDim = 256;         // image side limit
 constexpr unsigned kStagedMaxDim = 160;   // member images staged in shared memory (two buffers) up to this
-constexpr unsigned kFinishSmemDim = 160;  // finish kernel's spectra in shared memory up to this
-constexpr unsigned kFinishThreads = 512;
 constexpr double kPi = 3.141592653589793;
 
 // error words: [0] belongsto entries outside [0, n_class), [1] the first such
@@ -451,13 +451,15 @@ struct AvgFinishArgs {
     const unsigned* total;
     const double2* mean;
     const float2* tw; // e^(2 pi i j / D), j = 0..D-1
-    float2* scratch;  // [R][2][D][H] when the spectra do not fit in shared memory
+    float2* spec;     // [groups of the launch][D][H] half spectra
     float* avg;
     unsigned R, D;
+    unsigned r0, tiles; // first group of the launch, CTAs per group
     float fl, ff;
     int center;
 };
 
+// ---- averages from their pieces, filtered and moved ----
 // Per group: the sum of its pieces times float(1/members); then, when
 // filtering or centring, the real DFT over rows (x) then columns (y), the
 // spectrum times the filter 0.5 (tanh(k (r + fl)) - tanh(k (r - fl))),
@@ -465,177 +467,315 @@ struct AvgFinishArgs {
 // when ff = 0), and the phase exp(-2 pi i (kx dx + ky dy) / D) with (dx, dy) =
 // -mean shift, then the inverse DFT over columns and the real inverse over rows
 // (the imaginary parts of the kx = 0 and D/2 terms dropped), divided by D^2.
-// Memory (shared, or global scratch above side 160): the twiddles tw[D], then
-// two spectra F, G of D rows of Hs = H | 1 entries (an odd row length keeps a
-// warp's accesses down a column free of bank conflicts); the image and the
-// result sit in G's space with row stride D + 1.  In every pass a warp's lanes
-// run along the dimension its data is contiguous or oddly strided in, and all
-// lanes of a warp read the same twiddle (at most two distinct); each thread
-// computes two outputs that share their data loads.
-__global__ void __launch_bounds__(kFinishThreads)
-avg_finish_kernel(AvgFinishArgs a)
+//
+// Any side up to 256, so the transforms are plain sums, in three kernels: rows
+// (a CTA per group and 2 kFinTile rows), columns with filter and inverse columns
+// (per group and 2 kFinCols columns), inverse rows (as the first).  Each sum is
+// folded: terms j and D - j share a twiddle (their sum meets the cosine, their
+// difference the sine), and so do results k and D - k of a column or an inverse
+// row (they differ in the sine part's sign): half the products of the real passes,
+// a quarter of the complex ones.  A thread has one k (or pair of results) and
+// kFinTile rows or kFinCols columns, whose folded values it reads as float4 at one
+// address per warp (two where a tile ends).
+// What bounds it: latency; 200 groups of side 76 are 1,000 CTAs of three warps a
+// kernel.  Pieces, rows, columns, inverse rows 18 + 11 + 24 + 11 us there and 9 + 9 +
+// 17 + 9 for 20 groups of side 128, against 128 and 332 with one CTA per group and
+// unfolded sums; the error against FP64 went from 4.1e-7 to 2.5e-7.
+constexpr unsigned kFinTile = 8;  // rows per thread
+constexpr unsigned kFinCols = 4;  // columns per thread
+constexpr unsigned kFinRows = 2 * kFinTile;
+constexpr unsigned kFinColumns = 2 * kFinCols;
+constexpr unsigned kFinPitch = kFinRows + 4;       // of the folded rows: stores along x meet 4 banks deep, not 16
+constexpr unsigned kFinColPitch = kFinColumns + 1; // of the columns' spectra: stores along ky without conflicts
+constexpr size_t kFinSpecBytes = 64u << 20;        // half spectra held at once (in L2)
+constexpr unsigned kFinThreads = 288; // covers 2 (kMaxDim / 2 + 1) in whole warps
+
+// Each group's pieces summed in order, times float(1/members), into the averages
+// (0 without members): a thread per pixel, eight pieces' loads in flight.  (Inside
+// the row pass, a thread's pixels one after another, the two kernels' 18 us for 20
+// groups of side 128 with 19 pieces each were 63.)
+__global__ void __launch_bounds__(256)
+avg_mean_kernel(AvgFinishArgs a)
+{
+    const unsigned r = blockIdx.x / a.tiles, m = a.total[r];
+    const size_t npix = (size_t)a.D * a.D, q = (size_t)(blockIdx.x % a.tiles) * 256 + threadIdx.x;
+    if (q >= npix || !GPUISAC_IN_BOUNDS(kChkAvgOut, (size_t)r * npix + q, (size_t)a.R * npix))
+        return;
+    float s = 0.0f;
+    const unsigned p1 = a.pstart[r + 1];
+    for (unsigned p = a.pstart[r]; p < p1; p += 8) {
+        float v[8];
+#pragma unroll
+        for (unsigned i = 0; i < 8; i++)
+            v[i] = p + i < p1 ? a.partial[(size_t)(p + i) * npix + q] : 0.0f;
+#pragma unroll
+        for (unsigned i = 0; i < 8; i++)
+            s += v[i];
+    }
+    a.avg[(size_t)r * npix + q] = m ? s * __double2float_rn(1.0 / (double)m) : 0.0f;
+}
+
+// spec[y][kx] = sum_x img[y][x] e^(-2 pi i kx x / D): CTA r tiles + t is the launch's
+// group r, row tile t.  Shared memory: tw[D], then per x = 0..K the rows' folded sums
+// and differences (x = 0: the values at 0 and at D / 2).
+__global__ void __launch_bounds__(kFinThreads)
+avg_rows_kernel(AvgFinishArgs a)
 {
     extern __shared__ __align__(16) float2 fsm[];
-    const unsigned r = blockIdx.x, D = a.D, H = D / 2 + 1, Hs = H | 1u, S = D + 1, tid = threadIdx.x;
-    const size_t npix = (size_t)D * D, nspec = (size_t)D * Hs;
-    float* out = a.avg + (size_t)r * npix;
-    const unsigned m = a.total[r];
-    if (m == 0) {
-        for (size_t q = tid; q < npix; q += kFinishThreads)
-            out[q] = 0.0f;
+    const unsigned rl = blockIdx.x / a.tiles, tile0 = blockIdx.x % a.tiles, r = a.r0 + rl;
+    const unsigned D = a.D, H = D / 2 + 1, K = (D - 1) / 2, tid = threadIdx.x;
+    if (a.total[r] == 0)
         return;
-    }
-    const float inv = __double2float_rn(1.0 / (double)m);
-    const unsigned p0 = a.pstart[r], p1 = a.pstart[r + 1];
-    auto piece_sum = [&](size_t q) {
-        float s = 0.0f;
-        for (unsigned p = p0; p < p1; p++)
-            s += a.partial[(size_t)p * npix + q];
-        return s * inv;
-    };
-    if (!(a.fl > 0.0f || a.center)) {
-        for (size_t q = tid; q < npix; q += kFinishThreads)
-            out[q] = piece_sum(q);
-        return;
-    }
-    float2* tw = fsm;
-    float2* F = a.scratch ? a.scratch + (size_t)r * 2 * nspec : fsm + D;
-    float2* G = F + nspec;
-    float* img = reinterpret_cast<float*>(G); // [D][S]
-    for (size_t q = tid; q < npix; q += kFinishThreads)
-        img[(q / D) * S + q % D] = piece_sum(q);
-    for (unsigned j = tid; j < D; j += kFinishThreads)
+    const unsigned y0 = tile0 * kFinRows, rows = min(kFinRows, D - y0);
+    const size_t npix = (size_t)D * D;
+    float2* tw = fsm;                                             // [D | 1]
+    float* es = reinterpret_cast<float*>(fsm + ((D + 1) & ~1u));  // [K + 1][kFinPitch]
+    float* os = es + (K + 1) * kFinPitch;
+    const float* img = a.avg + (size_t)r * npix;
+    for (unsigned j = tid; j < D; j += blockDim.x)
         tw[j] = a.tw[j];
-    __syncthreads();
-
-    // rows: F[y][kx] = sum_x img[y][x] e^(-2 pi i kx x / D); lanes along y
-    const unsigned Hh = (H + 1) / 2;
-    for (unsigned e = tid; e < D * Hh; e += kFinishThreads) {
-        const unsigned k1 = e / D, y = e % D, k2 = k1 + Hh;
-        const bool two = k2 < H;
-        const unsigned k2s = two ? k2 : 0u;
-        const float* rowp = img + (size_t)y * S;
-        float r1 = 0.0f, i1 = 0.0f, r2 = 0.0f, i2 = 0.0f;
-        unsigned j1 = 0, j2 = 0;
-        for (unsigned x = 0; x < D; x++) {
-            const float v = rowp[x];
-            const float2 w1 = tw[j1], w2 = tw[j2];
-            r1 = fmaf(v, w1.x, r1);
-            i1 = fmaf(-v, w1.y, i1);
-            r2 = fmaf(v, w2.x, r2);
-            i2 = fmaf(-v, w2.y, i2);
-            j1 += k1;
-            j1 = j1 >= D ? j1 - D : j1;
-            j2 += k2s;
-            j2 = j2 >= D ? j2 - D : j2;
+    for (unsigned e = tid; e < kFinRows * (K + 1); e += blockDim.x) {
+        const unsigned yy = e / (K + 1), x = e % (K + 1);
+        float2 v = make_float2(0.0f, 0.0f);
+        if (yy < rows) {
+            const size_t row = (size_t)(y0 + yy) * D;
+            v = make_float2(img[row + x], img[row + (x > 0 ? D - x : D / 2)]);
+            if (x == 0 && D % 2 != 0)
+                v.y = 0.0f;
         }
-        F[(size_t)y * Hs + k1] = make_float2(r1, i1);
-        if (two)
-            F[(size_t)y * Hs + k2] = make_float2(r2, i2);
+        es[x * kFinPitch + yy] = x > 0 ? v.x + v.y : v.x;
+        os[x * kFinPitch + yy] = x > 0 ? v.x - v.y : v.y;
     }
     __syncthreads();
-
-    // columns, filter and phase: G[ky][kx] = h ph sum_y F[y][kx] e^(-2 pi i ky y / D);
-    // lanes along kx.  The phase exp(-2 pi i (kx dx + ky dy) / D) is
-    // sincospi(kx px + ky py), px = -2 dx / D rounded to float once per group.
-    const double2 mn = a.mean[r];
-    const float px = a.center ? (float)(2.0 * mn.x / (double)D) : 0.0f;
-    const float py = a.center ? (float)(2.0 * mn.y / (double)D) : 0.0f;
-    const float kf = a.ff > 0.0f ? (float)(kPi / (2.0 * (double)a.ff * (double)a.fl)) : 0.0f;
-    auto finish_term = [&](unsigned ky, unsigned kx, float re, float im) {
-        const int kys = 2 * ky > D ? (int)ky - (int)D : (int)ky;
-        float hf = 1.0f;
-        if (a.fl > 0.0f) {
-            const float fx = (float)kx / (float)D, fy = (float)kys / (float)D;
-            const float rr = sqrtf(fx * fx + fy * fy);
-            hf = a.ff > 0.0f ? 0.5f * (tanhf(kf * (rr + a.fl)) - tanhf(kf * (rr - a.fl)))
-                             : (rr < a.fl ? 1.0f : (rr == a.fl ? 0.5f : 0.0f));
+    const unsigned tile = tid / H, k = tid % H;
+    if (tile >= kFinRows / kFinTile)
+        return;
+    float re[kFinTile], im[kFinTile];
+    const float4* e4 = reinterpret_cast<const float4*>(es) + tile * (kFinTile / 4);
+    const float4* o4 = reinterpret_cast<const float4*>(os) + tile * (kFinTile / 4);
+#pragma unroll
+    for (unsigned i = 0; i < kFinTile; i++)
+        re[i] = im[i] = 0.0f;
+    unsigned j = k;
+    for (unsigned x = 1; x <= K; x++) {
+        const float2 w = tw[j];
+        e4 += kFinPitch / 4, o4 += kFinPitch / 4;
+#pragma unroll
+        for (unsigned q = 0; q < kFinTile / 4; q++) {
+            const float4 e = e4[q], o = o4[q];
+            re[4 * q] = fmaf(e.x, w.x, re[4 * q]), im[4 * q] = fmaf(-o.x, w.y, im[4 * q]);
+            re[4 * q + 1] = fmaf(e.y, w.x, re[4 * q + 1]), im[4 * q + 1] = fmaf(-o.y, w.y, im[4 * q + 1]);
+            re[4 * q + 2] = fmaf(e.z, w.x, re[4 * q + 2]), im[4 * q + 2] = fmaf(-o.z, w.y, im[4 * q + 2]);
+            re[4 * q + 3] = fmaf(e.w, w.x, re[4 * q + 3]), im[4 * q + 3] = fmaf(-o.w, w.y, im[4 * q + 3]);
         }
-        float ps = 0.0f, pc = 1.0f;
-        if (a.center)
-            sincospif(fmaf((float)kx, px, (float)kys * py), &ps, &pc);
-        G[(size_t)ky * Hs + kx] = make_float2((re * pc - im * ps) * hf, (re * ps + im * pc) * hf);
-    };
-    const unsigned Dh = (D + 1) / 2;
-    for (unsigned e = tid; e < Dh * H; e += kFinishThreads) {
-        const unsigned k1 = e / H, kx = e % H, k2 = k1 + Dh;
-        const bool two = k2 < D;
-        const unsigned k2s = two ? k2 : 0u;
-        float r1 = 0.0f, i1 = 0.0f, r2 = 0.0f, i2 = 0.0f;
-        unsigned j1 = 0, j2 = 0;
-        for (unsigned y = 0; y < D; y++) {
-            const float2 v = F[(size_t)y * Hs + kx];
-            const float2 w1 = tw[j1], w2 = tw[j2]; // (v.x + i v.y)(w.x - i w.y)
-            r1 = fmaf(v.x, w1.x, fmaf(v.y, w1.y, r1));
-            i1 = fmaf(v.y, w1.x, fmaf(-v.x, w1.y, i1));
-            r2 = fmaf(v.x, w2.x, fmaf(v.y, w2.y, r2));
-            i2 = fmaf(v.y, w2.x, fmaf(-v.x, w2.y, i2));
-            j1 += k1;
-            j1 = j1 >= D ? j1 - D : j1;
-            j2 += k2s;
-            j2 = j2 >= D ? j2 - D : j2;
-        }
-        finish_term(k1, kx, r1, i1);
-        if (two)
-            finish_term(k2, kx, r2, i2);
+        j += k;
+        j = j >= D ? j - D : j;
     }
-    __syncthreads();
-
-    // inverse columns: F[y][kx] = sum_ky G[ky][kx] e^(+2 pi i ky y / D); lanes along kx
-    for (unsigned e = tid; e < Dh * H; e += kFinishThreads) {
-        const unsigned y1 = e / H, kx = e % H, y2 = y1 + Dh;
-        const bool two = y2 < D;
-        const unsigned y2s = two ? y2 : 0u;
-        float r1 = 0.0f, i1 = 0.0f, r2 = 0.0f, i2 = 0.0f;
-        unsigned j1 = 0, j2 = 0;
-        for (unsigned ky = 0; ky < D; ky++) {
-            const float2 v = G[(size_t)ky * Hs + kx];
-            const float2 w1 = tw[j1], w2 = tw[j2];
-            r1 = fmaf(v.x, w1.x, fmaf(-v.y, w1.y, r1));
-            i1 = fmaf(v.y, w1.x, fmaf(v.x, w1.y, i1));
-            r2 = fmaf(v.x, w2.x, fmaf(-v.y, w2.y, r2));
-            i2 = fmaf(v.y, w2.x, fmaf(v.x, w2.y, i2));
-            j1 += y1;
-            j1 = j1 >= D ? j1 - D : j1;
-            j2 += y2s;
-            j2 = j2 >= D ? j2 - D : j2;
+    float2* out = a.spec + (size_t)rl * D * H;
+#pragma unroll
+    for (unsigned i = 0; i < kFinTile; i++) {
+        const unsigned yy = tile * kFinTile + i;
+        if (yy < rows) {
+            const float nyq = os[yy]; // 0 on an odd side
+            out[(size_t)(y0 + yy) * H + k] = make_float2(re[i] + es[yy] + ((k & 1u) ? -nyq : nyq), im[i]);
         }
-        F[(size_t)y1 * Hs + kx] = make_float2(r1, i1);
-        if (two)
-            F[(size_t)y2 * Hs + kx] = make_float2(r2, i2);
     }
-    __syncthreads();
+}
 
-    // inverse rows, half spectrum to real, into G's space; lanes along y
-    float* res = img;
-    const float scale = 1.0f / (float)npix;
+// A thread's results k and D - k of kFinCols columns of complex values, folded
+// in smem as fold[j][column] = (sum.re, sum.im, difference.re, difference.im) for
+// j = 1..K and (v[0], v[D / 2]) at j = 0: lo[c] = sum_j v[j] e^(-2 pi i k j / D),
+// hi[c] the same at D - k
+__device__ __forceinline__ void dft_columns(const float4* __restrict__ fold, const float2* __restrict__ tw, unsigned k,
+                                            unsigned D, float2 (&lo)[kFinCols], float2 (&hi)[kFinCols])
+{
     const unsigned K = (D - 1) / 2;
-    for (unsigned e = tid; e < D * Dh; e += kFinishThreads) {
-        const unsigned x1 = e / D, y = e % D, x2 = x1 + Dh;
-        const bool two = x2 < D;
-        const unsigned x2s = two ? x2 : 0u;
-        const float2* fr = F + (size_t)y * Hs;
-        float s1 = 0.0f, s2 = 0.0f;
-        unsigned j1 = x1, j2 = x2s;
-        for (unsigned kx = 1; kx <= K; kx++) {
-            const float2 v = fr[kx];
-            const float2 w1 = tw[j1], w2 = tw[j2];
-            s1 = fmaf(v.x, w1.x, fmaf(-v.y, w1.y, s1));
-            s2 = fmaf(v.x, w2.x, fmaf(-v.y, w2.y, s2));
-            j1 += x1;
-            j1 = j1 >= D ? j1 - D : j1;
-            j2 += x2s;
-            j2 = j2 >= D ? j2 - D : j2;
+    float ar[kFinCols], ai[kFinCols], br[kFinCols], bi[kFinCols]; // cosine and sine parts
+#pragma unroll
+    for (unsigned c = 0; c < kFinCols; c++)
+        ar[c] = ai[c] = br[c] = bi[c] = 0.0f;
+    unsigned j = k;
+    const float4* f = fold;
+    for (unsigned y = 1; y <= K; y++) {
+        const float2 w = tw[j];
+        f += kFinColumns;
+#pragma unroll
+        for (unsigned c = 0; c < kFinCols; c++) {
+            const float4 v = f[c];
+            ar[c] = fmaf(v.x, w.x, ar[c]);
+            ai[c] = fmaf(v.y, w.x, ai[c]);
+            br[c] = fmaf(v.w, w.y, br[c]);
+            bi[c] = fmaf(v.z, w.y, bi[c]);
         }
-        const float nyq = (D & 1u) == 0 ? fr[D / 2].x : 0.0f;
-        res[(size_t)y * S + x1] = (fr[0].x + 2.0f * s1 + ((x1 & 1u) ? -nyq : nyq)) * scale;
-        if (two)
-            res[(size_t)y * S + x2] = (fr[0].x + 2.0f * s2 + ((x2 & 1u) ? -nyq : nyq)) * scale;
+        j += k;
+        j = j >= D ? j - D : j;
+    }
+#pragma unroll
+    for (unsigned c = 0; c < kFinCols; c++) {
+        const float4 v = fold[c];
+        const float cr = ar[c] + v.x + ((k & 1u) ? -v.z : v.z), ci = ai[c] + v.y + ((k & 1u) ? -v.w : v.w);
+        lo[c] = make_float2(cr + br[c], ci - bi[c]);
+        hi[c] = make_float2(cr - br[c], ci + bi[c]);
+    }
+}
+
+// The column pass in place on spec: forward sums over y, filter and phase,
+// inverse sums over ky (the forward ones with results k and D - k exchanged).
+// CTA r tiles + t is the launch's group r, column tile t; shared memory: tw[D], the
+// folded columns, the columns' spectra.
+__global__ void __launch_bounds__(kFinThreads)
+avg_cols_kernel(AvgFinishArgs a)
+{
+    extern __shared__ __align__(16) float2 fsm[];
+    const unsigned rl = blockIdx.x / a.tiles, tile0 = blockIdx.x % a.tiles, r = a.r0 + rl;
+    const unsigned D = a.D, H = D / 2 + 1, K = (D - 1) / 2, tid = threadIdx.x;
+    if (a.total[r] == 0)
+        return;
+    const unsigned x0 = tile0 * kFinColumns, cols = min(kFinColumns, H - x0);
+    float2* tw = fsm;
+    float4* fold = reinterpret_cast<float4*>(fsm + ((D + 1) & ~1u)); // [K + 1][kFinColumns]
+    float2* g = reinterpret_cast<float2*>(fold + (K + 1) * kFinColumns); // [D][kFinColPitch]
+    float2* spec = a.spec + (size_t)rl * D * H;
+    auto fold_of = [&](float2 v1, float2 v2, unsigned y) {
+        return y > 0 ? make_float4(v1.x + v2.x, v1.y + v2.y, v1.x - v2.x, v1.y - v2.y)
+                     : make_float4(v1.x, v1.y, v2.x, v2.y);
+    };
+    auto partner = [&](unsigned y) { return y > 0 ? D - y : D / 2; }; // (D / 2: even sides only)
+    for (unsigned j = tid; j < D; j += blockDim.x)
+        tw[j] = a.tw[j];
+    const float2 zero = make_float2(0.0f, 0.0f);
+    for (unsigned e = tid; e < kFinColumns * (K + 1); e += blockDim.x) {
+        const unsigned y = e / kFinColumns, c = e % kFinColumns;
+        const bool in = c < cols, has2 = in && (y > 0 || D % 2 == 0);
+        fold[e] = fold_of(in ? spec[(size_t)y * H + x0 + c] : zero,
+                          has2 ? spec[(size_t)partner(y) * H + x0 + c] : zero, y);
     }
     __syncthreads();
-    for (size_t q = tid; q < npix; q += kFinishThreads)
-        if (GPUISAC_IN_BOUNDS(kChkAvgOut, (size_t)r * npix + q, (size_t)a.R * npix))
-            out[q] = res[(q / D) * S + q % D];
+    const unsigned tile = tid / H, k = tid % H;
+    const bool work = tile < kFinColumns / kFinCols;
+    const unsigned k2 = k == 0 ? 0 : D - k; // k's partner (itself at 0 and D / 2)
+    float2 lo[kFinCols], hi[kFinCols];
+    if (work) {
+        // The phase exp(-2 pi i (kx dx + ky dy) / D) is sincospi(kx px + ky py),
+        // px = -2 dx / D rounded to float once per group.
+        const double2 mn = a.mean[r];
+        const float px = a.center ? (float)(2.0 * mn.x / (double)D) : 0.0f;
+        const float py = a.center ? (float)(2.0 * mn.y / (double)D) : 0.0f;
+        const float kf = a.ff > 0.0f ? (float)(kPi / (2.0 * (double)a.ff * (double)a.fl)) : 0.0f;
+        dft_columns(fold + tile * kFinCols, tw, k, D, lo, hi);
+#pragma unroll
+        for (unsigned c = 0; c < kFinCols; c++) {
+            const unsigned kx = x0 + tile * kFinCols + c;
+            // the filter is the same at ky and D - ky
+            float hf = 1.0f;
+            if (a.fl > 0.0f) {
+                const float fx = (float)kx / (float)D, fy = (float)k / (float)D;
+                const float rr = sqrtf(fx * fx + fy * fy);
+                hf = a.ff > 0.0f ? 0.5f * (tanhf(kf * (rr + a.fl)) - tanhf(kf * (rr - a.fl)))
+                                 : (rr < a.fl ? 1.0f : (rr == a.fl ? 0.5f : 0.0f));
+            }
+            auto finish_term = [&](float2 v, int kys) {
+                float ps = 0.0f, pc = 1.0f;
+                if (a.center)
+                    sincospif(fmaf((float)kx, px, (float)kys * py), &ps, &pc);
+                return make_float2((v.x * pc - v.y * ps) * hf, (v.x * ps + v.y * pc) * hf);
+            };
+            g[k * kFinColPitch + tile * kFinCols + c] = finish_term(lo[c], (int)k);
+            if (k2 != k)
+                g[k2 * kFinColPitch + tile * kFinCols + c] = finish_term(hi[c], -(int)k);
+        }
+    }
+    __syncthreads();
+    for (unsigned e = tid; e < kFinColumns * (K + 1); e += blockDim.x) {
+        const unsigned y = e / kFinColumns, c = e % kFinColumns;
+        fold[e] = fold_of(g[y * kFinColPitch + c], y > 0 || D % 2 == 0 ? g[partner(y) * kFinColPitch + c] : zero, y);
+    }
+    __syncthreads();
+    if (!work)
+        return;
+    dft_columns(fold + tile * kFinCols, tw, k, D, lo, hi);
+#pragma unroll
+    for (unsigned c = 0; c < kFinCols; c++) {
+        const unsigned cc = tile * kFinCols + c;
+        if (cc < cols) {
+            spec[(size_t)k * H + x0 + cc] = hi[c];
+            if (k2 != k)
+                spec[(size_t)k2 * H + x0 + cc] = lo[c];
+        }
+    }
+}
+
+// inverse rows, half spectrum to real: CTA r tiles + t is the launch's group r, row
+// tile t.  Shared memory: tw[D], then per kx = 0..K the rows' real and imaginary
+// parts (kx = 0: the real parts at 0 and at D / 2).
+__global__ void __launch_bounds__(kFinThreads)
+avg_inverse_kernel(AvgFinishArgs a)
+{
+    extern __shared__ __align__(16) float2 fsm[];
+    const unsigned rl = blockIdx.x / a.tiles, tile0 = blockIdx.x % a.tiles, r = a.r0 + rl;
+    const unsigned D = a.D, H = D / 2 + 1, K = (D - 1) / 2, tid = threadIdx.x;
+    const unsigned y0 = tile0 * kFinRows, rows = min(kFinRows, D - y0);
+    const size_t npix = (size_t)D * D;
+    float* out = a.avg + (size_t)r * npix;
+    if (a.total[r] == 0)
+        return;
+    float2* tw = fsm;
+    float* es = reinterpret_cast<float*>(fsm + ((D + 1) & ~1u));
+    float* os = es + (K + 1) * kFinPitch;
+    const float2* spec = a.spec + (size_t)rl * D * H;
+    for (unsigned j = tid; j < D; j += blockDim.x)
+        tw[j] = a.tw[j];
+    for (unsigned e = tid; e < kFinRows * (K + 1); e += blockDim.x) {
+        const unsigned yy = e / (K + 1), kx = e % (K + 1);
+        float2 v = make_float2(0.0f, 0.0f);
+        if (yy < rows) {
+            const float2* row = spec + (size_t)(y0 + yy) * H;
+            v = row[kx];
+            if (kx == 0)
+                v.y = D % 2 == 0 ? row[D / 2].x : 0.0f;
+        }
+        es[kx * kFinPitch + yy] = v.x;
+        os[kx * kFinPitch + yy] = v.y;
+    }
+    __syncthreads();
+    const unsigned tile = tid / H, x = tid % H;
+    if (tile >= kFinRows / kFinTile)
+        return;
+    float sc[kFinTile], ss[kFinTile];
+    const float4* e4 = reinterpret_cast<const float4*>(es) + tile * (kFinTile / 4);
+    const float4* o4 = reinterpret_cast<const float4*>(os) + tile * (kFinTile / 4);
+#pragma unroll
+    for (unsigned i = 0; i < kFinTile; i++)
+        sc[i] = ss[i] = 0.0f;
+    unsigned j = x;
+    for (unsigned kx = 1; kx <= K; kx++) {
+        const float2 w = tw[j];
+        e4 += kFinPitch / 4, o4 += kFinPitch / 4;
+#pragma unroll
+        for (unsigned q = 0; q < kFinTile / 4; q++) {
+            const float4 e = e4[q], o = o4[q];
+            sc[4 * q] = fmaf(e.x, w.x, sc[4 * q]), ss[4 * q] = fmaf(o.x, w.y, ss[4 * q]);
+            sc[4 * q + 1] = fmaf(e.y, w.x, sc[4 * q + 1]), ss[4 * q + 1] = fmaf(o.y, w.y, ss[4 * q + 1]);
+            sc[4 * q + 2] = fmaf(e.z, w.x, sc[4 * q + 2]), ss[4 * q + 2] = fmaf(o.z, w.y, ss[4 * q + 2]);
+            sc[4 * q + 3] = fmaf(e.w, w.x, sc[4 * q + 3]), ss[4 * q + 3] = fmaf(o.w, w.y, ss[4 * q + 3]);
+        }
+        j += x;
+        j = j >= D ? j - D : j;
+    }
+    const float scale = 1.0f / (float)npix;
+#pragma unroll
+    for (unsigned i = 0; i < kFinTile; i++) {
+        const unsigned yy = tile * kFinTile + i;
+        if (yy >= rows)
+            break;
+        const float nyq = os[yy], base = es[yy] + ((x & 1u) ? -nyq : nyq);
+        const size_t q = (size_t)(y0 + yy) * D;
+        if (GPUISAC_IN_BOUNDS(kChkAvgOut, (size_t)r * npix + q + D - 1, (size_t)a.R * npix)) {
+            out[q + x] = (base + 2.0f * (sc[i] - ss[i])) * scale;
+            if (x > 0 && D - x != x)
+                out[q + D - x] = (base + 2.0f * (sc[i] + ss[i])) * scale;
+        }
+    }
 }
 
 template <typename T>
@@ -771,9 +911,10 @@ extern "C" int gpuisac_class_averages(const float* imgs, unsigned int n_img, uns
     const unsigned resident = (unsigned)std::max(1, sms * std::max(per_sm, 1));
     const unsigned piece = std::min(256u, std::max(8u, (P + 4 * resident - 1) / (4 * resident)));
     const size_t pieces_cap = (size_t)P / piece + R + 1;
-    const bool fin_smem = D <= kFinishSmemDim;
-    const size_t nspec = (size_t)D * ((D / 2 + 1) | 1u);
-    const size_t fin_smem_bytes = sizeof(float2) * (D + (fin_smem ? 2 * nspec : 0));
+    const bool spectra = fl > 0.0f || center;
+    const unsigned H = D / 2 + 1, K = (D - 1) / 2;
+    const unsigned fin_groups =
+        (unsigned)std::min<size_t>(R, std::max<size_t>(1, kFinSpecBytes / ((size_t)D * H * sizeof(float2))));
 
     AV_CK(w.cnt.ensure((size_t)n_chunks * R));
     AV_CK(w.total.ensure(R));
@@ -784,8 +925,8 @@ extern "C" int gpuisac_class_averages(const float* imgs, unsigned int n_img, uns
     AV_CK(w.order.ensure(P));
     AV_CK(w.mean.ensure(R));
     AV_CK(w.partial.ensure(pieces_cap * npix));
-    if (!fin_smem)
-        AV_CK(w.scratch.ensure((size_t)R * 2 * nspec));
+    if (spectra)
+        AV_CK(w.scratch.ensure((size_t)fin_groups * D * H));
     if (!w.h_err)
         AV_CK(cudaMallocHost(&w.h_err, kErrWords * sizeof(unsigned)));
     if (w.tw_dim != D) {
@@ -816,13 +957,28 @@ extern "C" int gpuisac_class_averages(const float* imgs, unsigned int n_img, uns
                   0, 0};
     ccf_test_settings(sa.test_stall, sa.wait_iters);
     sum_kernel<<<(unsigned)pieces_cap, sum_threads, sum_smem, st>>>(sa);
-    AvgFinishArgs fa{w.partial.p, w.pstart.p, w.total.p, w.mean.p, w.tw.p, fin_smem ? nullptr : w.scratch.p,
-                     averages, R, D, fl, ff, center};
-    if (fin_smem_bytes > 48 * 1024)
-        AV_CK(cudaFuncSetAttribute(avg_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)fin_smem_bytes));
-    avg_finish_kernel<<<R, kFinishThreads, fin_smem_bytes, st>>>(fa);
-    g_kernel_launches.fetch_add(8, std::memory_order_relaxed);
+    AvgFinishArgs fa{w.partial.p, w.pstart.p, w.total.p, w.mean.p, w.tw.p, w.scratch.p, averages, R, D, 0, 0, fl, ff,
+                     center};
+    unsigned fin_launches = 1;
+    fa.tiles = (unsigned)((npix + 255) / 256);
+    avg_mean_kernel<<<R * fa.tiles, 256, 0, st>>>(fa);
+    const unsigned fin_threads = (2 * H + 31) / 32 * 32;
+    const size_t tw_bytes = ((D + 1) & ~1u) * sizeof(float2);
+    const size_t row_smem = tw_bytes + 2 * sizeof(float) * (K + 1) * kFinPitch;
+    const size_t col_smem = tw_bytes + sizeof(float4) * (K + 1) * kFinColumns + sizeof(float2) * D * kFinColPitch;
+    const unsigned row_tiles = (D + kFinRows - 1) / kFinRows, col_tiles = (H + kFinColumns - 1) / kFinColumns;
+    for (unsigned r0 = 0; spectra && r0 < R; r0 += fin_groups) {
+        const unsigned n = std::min(fin_groups, R - r0);
+        fa.r0 = r0;
+        fa.tiles = row_tiles;
+        avg_rows_kernel<<<n * row_tiles, fin_threads, row_smem, st>>>(fa);
+        fa.tiles = col_tiles;
+        avg_cols_kernel<<<n * col_tiles, fin_threads, col_smem, st>>>(fa);
+        fa.tiles = row_tiles;
+        avg_inverse_kernel<<<n * row_tiles, fin_threads, row_smem, st>>>(fa);
+        fin_launches += 3;
+    }
+    g_kernel_launches.fetch_add(7 + fin_launches, std::memory_order_relaxed);
     AV_CK(cudaGetLastError());
     AV_CK(cudaMemcpyAsync(w.h_err, w.err.p, kErrWords * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     AV_CK(cudaStreamSynchronize(st));
