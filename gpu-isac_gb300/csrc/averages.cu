@@ -19,10 +19,9 @@
 //                            particle order
 //  6. avg_shift_kernel       one warp per group: mean shifts, parameters
 //  7. avg_sum_kernel         one CTA per piece (a run of one group's members):
-//                            each member image staged in shared memory by a
-//                            bulk copy (two buffers, the member's record
-//                            written beside it), every thread one column
-//                            and every G-th row of the output, the quadratic
+//                            each member image staged in shared memory by bulk
+//                            copies (two buffers), every thread one column of
+//                            two halves of the output, the quadratic
 //                            interpolation from shared memory, FP32 sums in
 //                            registers, one partial image per piece
 //  8. avg_mean_kernel        each group's pieces summed in order, times
@@ -49,6 +48,7 @@ namespace {
 constexpr unsigned kAvgChunk = 1024;      // particles per counting-sort chunk
 constexpr unsigned kSmemGroups = 16384;   // scatter: a chunk's group offsets in shared memory up to this
 constexpr unsigned kMaxDim = 256;         // image side limit
+constexpr unsigned kMinPiece = 2, kMaxPiece = 256; // members of a piece
 constexpr unsigned kStagedMaxDim = 160;   // member images staged in shared memory (two buffers) up to this
 constexpr double kPi = 3.141592653589793;
 
@@ -292,67 +292,129 @@ struct AvgSumArgs {
     const unsigned* pstart;
     float* partial;
     unsigned* err;
-    unsigned P, R, D, G, piece;
+    unsigned P, R, D, G, piece, pitch, half;
     unsigned test_stall, wait_iters; // failure-path tests only (gpuisac_test_stall_ccf)
 };
 
-// The interpolated value of output pixel (ixs, iy) of one member: the source
-// point from the rotation (float operations in the order of the restatement),
-// the pixel itself outside [0, D)^2, then the six-point quadratic rule with
-// periodic neighbours.  Indices stay in [0, D) for every input (a NaN or
-// infinite source point fails the range test).
-__device__ __forceinline__ float quadri_at(const float* __restrict__ src, int D, float xo, float yo)
+// the six pixels of the quadratic rule at one source point
+struct Six {
+    float f00, fp0, fm0, f0p, f0m, fpp; // offsets (0, 0), (+1, 0), (-1, 0), (0, +1), (0, -1), (+1, +1)
+};
+
+__device__ __forceinline__ Six six_at(const float* __restrict__ q, int ip, int im, int jp, int jm)
 {
-    const float fx = floorf(xo), fy = floorf(yo);
-    const int i = (int)fx, j = (int)fy;
-    const float dx = xo - fx, dy = yo - fy;
-    const int ip = i + 1 == D ? 0 : i + 1, im = i == 0 ? D - 1 : i - 1;
-    const int jp = j + 1 == D ? 0 : j + 1, jm = j == 0 ? D - 1 : j - 1;
-    const float f00 = src[j * D + i];
-    const float c1 = src[j * D + ip] - f00;
-    const float c2 = (c1 - f00 + src[j * D + im]) * 0.5f;
-    const float c3 = src[jp * D + i] - f00;
-    const float c4 = (c3 - f00 + src[jm * D + i]) * 0.5f;
-    const float c5 = src[jp * D + ip] - f00 - c1 - c3;
-    return f00 + dx * (c1 + (dx - 1.0f) * c2 + dy * c5) + dy * (c3 + (dy - 1.0f) * c4);
+    return {q[0], q[ip], q[im], q[jp], q[jm], q[jp + ip]};
 }
 
-constexpr int kRowsPerThread = 16; // output rows per thread and pass
+constexpr unsigned kSumTileX = 8, kSumTileY = 4; // a warp's pixels of the output
 
-__device__ __forceinline__ void accumulate(float (&acc)[kRowsPerThread], const float* __restrict__ src,
-                                           const AvgMember& b, unsigned ix, unsigned row0, unsigned G, unsigned D)
+__device__ __forceinline__ f32x2 add2_down(f32x2 a, f32x2 b)
 {
-    const float h = (float)(D >> 1), Df = (float)D;
+    f32x2 r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Adds one member's interpolated values to a thread's pixels of column ix: rows
+// row0 + p step < limit, p < ROWS, two at a time in packed halves (float operations in the
+// order of the restatement).
+//   x + 2^23 rounded down is 2^23 + floor(x) for x in [0, 2^23): its low bits are
+// the index and one subtraction gives the floor, where floorf and the conversion
+// each take a quarter-rate instruction.  Any other x (negative, infinite, NaN)
+// differs from 2^23 in its bits by more than D, as an unsigned number, so that one
+// comparison finds the points with all neighbours inside; a pair with another
+// point takes the general way.
+template <int ROWS>
+__device__ __forceinline__ void accumulate(f32x2 (&acc)[ROWS / 2], const float* __restrict__ src,
+                                           const AvgMember& b, unsigned ix, unsigned row0, unsigned limit,
+                                           unsigned step, unsigned D, unsigned pitch)
+{
+    const float h = (float)(D >> 1);
     const unsigned ixs = b.mirror ? (ix == 0 ? 0u : D - ix) : ix;
     const float x = __fsub_rn((float)ixs, __fadd_rn(h, b.sx));
     const float hy = __fadd_rn(h, b.sy);
     const float xc = __fmul_rn(x, b.c), xs = __fmul_rn(x, b.s);
+    const f32x2 xc2 = pack_f32x2(xc, xc), xs2 = pack_f32x2(xs, xs), hy2 = pack_f32x2(hy, hy), h2 = pack_f32x2(h, h);
+    const f32x2 two23 = pack_f32x2(8388608.0f, 8388608.0f), one = pack_f32x2(1.0f, 1.0f);
+    const f32x2 half = pack_f32x2(0.5f, 0.5f), down = pack_f32x2((float)(2 * step), (float)(2 * step));
+    f32x2 iy2 = pack_f32x2((float)row0, (float)(row0 + step));
+    const unsigned first = 0x4B000001u; // the bits of 2^23 + 1: index 1
+    const float* src1 = src + pitch + 1; // pixel (1, 1)
 #pragma unroll
-    for (int p = 0; p < kRowsPerThread; p++) {
-        const unsigned iy = row0 + (unsigned)p * G;
-        if (iy < D) {
-            const float y = __fsub_rn((float)iy, hy);
-            float xo = __fadd_rn(__fsub_rn(xc, __fmul_rn(y, b.s)), h);
-            float yo = __fadd_rn(__fadd_rn(xs, __fmul_rn(y, b.c)), h);
-            if (!(xo >= 0.0f && xo < Df && yo >= 0.0f && yo < Df)) {
-                xo = (float)ixs;
-                yo = (float)iy;
-            }
-            acc[p] += quadri_at(src, (int)D, xo, yo);
+    for (int p = 0; p < ROWS / 2; p++) {
+        const unsigned iy = row0 + 2u * (unsigned)p * step;
+        if (iy >= limit)
+            break;
+        const f32x2 y = sub2(iy2, hy2);
+        iy2 = add2(iy2, down);
+        // (the products by themselves: a packed one would be contracted into the sum)
+        const float2 yf = unpack_f32x2(y);
+        const f32x2 ys = pack_f32x2(__fmul_rn(yf.x, b.s), __fmul_rn(yf.y, b.s));
+        const f32x2 yc = pack_f32x2(__fmul_rn(yf.x, b.c), __fmul_rn(yf.y, b.c));
+        const f32x2 xo = add2(sub2(xc2, ys), h2), yo = add2(add2(xs2, yc), h2);
+        const f32x2 tx = add2_down(xo, two23), ty = add2_down(yo, two23);
+        const float2 fx = unpack_f32x2(tx), fy = unpack_f32x2(ty);
+        const unsigned ia = __float_as_uint(fx.x) - first, ib = __float_as_uint(fx.y) - first;
+        const unsigned ja = __float_as_uint(fy.x) - first, jb = __float_as_uint(fy.y) - first;
+        f32x2 dx = sub2(xo, sub2(tx, two23)), dy = sub2(yo, sub2(ty, two23));
+        Six a, c;
+        if (ia < D - 2u && ib < D - 2u && ja < D - 2u && jb < D - 2u) {
+            a = six_at(src1 + (ja * pitch + ia), 1, -1, (int)pitch, -(int)pitch);
+            c = six_at(src1 + (jb * pitch + ib), 1, -1, (int)pitch, -(int)pitch);
+        } else {
+            float2 dxs = unpack_f32x2(dx), dys = unpack_f32x2(dy);
+            // a point outside [0, D)^2 is the pixel itself; neighbours wrap
+            auto border = [&](unsigned i, unsigned j, unsigned iy_own, float& ddx, float& ddy) {
+                if (i >= D || j >= D) {
+                    i = ixs;
+                    j = iy_own;
+                    ddx = ddy = 0.0f;
+                }
+                const int Di = (int)D, wrap = (Di - 1) * (int)pitch;
+                return six_at(src + (j * pitch + i), i + 1 == D ? 1 - Di : 1, i == 0 ? Di - 1 : -1,
+                              j + 1 == D ? -wrap : (int)pitch, j == 0 ? wrap : -(int)pitch);
+            };
+            a = border(ia + 1u, ja + 1u, iy, dxs.x, dys.x);
+            c = border(ib + 1u, jb + 1u, min(iy + step, D - 1), dxs.y, dys.y); // (a row past the last is not stored)
+            dx = pack_f32x2(dxs.x, dxs.y), dy = pack_f32x2(dys.x, dys.y);
         }
+        const f32x2 f00 = pack_f32x2(a.f00, c.f00);
+        const f32x2 c1 = sub2(pack_f32x2(a.fp0, c.fp0), f00);
+        const f32x2 c2 = mul2(add2(sub2(c1, f00), pack_f32x2(a.fm0, c.fm0)), half);
+        const f32x2 c3 = sub2(pack_f32x2(a.f0p, c.f0p), f00);
+        const f32x2 c4 = mul2(add2(sub2(c3, f00), pack_f32x2(a.f0m, c.f0m)), half);
+        const f32x2 c5 = sub2(sub2(sub2(pack_f32x2(a.fpp, c.fpp), f00), c1), c3);
+        const f32x2 u = fma2(dy, c5, fma2(sub2(dx, one), c2, c1));
+        const f32x2 v = fma2(dy, fma2(sub2(dy, one), c4, c3), fma2(dx, u, f00));
+        acc[p] = add2(acc[p], v);
     }
 }
 
-// grid: an upper bound on the pieces; CTA t >= pieces returns.  Threads
-// D x G: thread (ix, g) sums output rows row0 + g + p G, p < 16, of column ix,
-// in passes of 16 G rows over the piece's members (one pass up to D = 128).
-template <bool STAGED>
-__global__ void __launch_bounds__(1024)
+// grid: an upper bound on the pieces; CTA t >= pieces returns.  Warps
+// ceil(D / 8) x G: warp (cb, g) has the tiles of four rows row0 + 4 (g + p G), p <
+// ROWS, the first half of them (`half` output rows) of columns 8 cb .. 8 cb + 7, the
+// second half of the columns half the image away (the outer columns have most of the
+// border's pixels; a warp's share of a member is then about the others'), in passes of
+// 2 half rows over the piece's members (one pass up to D = 128).  STAGED: the image
+// in shared memory with row length `pitch`.
+// What bounds it: issue and shared loads, six a pixel (without the border's branch
+// 238 us instead of 274 for 20,000 members of side 76, without any interpolation 83).
+// A warp's 8 x 4 pixels meet shared banks two deep at any angle where 32 of one row
+// met them 2.5 deep, and 4 deep when the row length is a multiple of 32.  Before (a
+// warp's pixels along rows, one at a time, floorf, pieces of P / (4 waves) members):
+// 20,000 of side 76 in 200 groups 295 us, now 275; 4,000 of 64 in 40 89 -> 64; 3,000
+// of 128 in 20 252 -> 141; 900 of 48 in 11 23 -> 12; 500 of 200 in 5 (read from global
+// memory) 304 -> 83.  Not kept: three CTAs of 10 warps an SM (64 registers, spills) 284,
+// four 299.
+template <bool STAGED, int ROWS, int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS)
 avg_sum_kernel(AvgSumArgs a)
 {
     extern __shared__ __align__(16) float sbuf[];
     __shared__ uint64_t bars[2];
-    __shared__ AvgMember mrec[2]; // the member whose image a buffer holds (written with the copy's issue)
+    // the piece's members (read one by one as their copies are issued, the warp that
+    // issues kept the others waiting at the end of each member)
+    __shared__ AvgMember mrec[STAGED ? kMaxPiece : 1];
     const unsigned t = blockIdx.x, R = a.R, D = a.D, G = a.G;
     const unsigned n_pieces = a.pstart[R];
     if (t >= n_pieces)
@@ -369,20 +431,32 @@ avg_sum_kernel(AvgSumArgs a)
     const unsigned r = lo;
     const unsigned k0 = a.start[r] + (t - a.pstart[r]) * a.piece;
     const unsigned k1 = min(a.start[r] + a.total[r], k0 + a.piece);
-    const unsigned tid = threadIdx.x, ix = tid % D, g = tid / D;
-    const size_t npix = (size_t)D * D;
+    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const unsigned blocks = (D + kSumTileX - 1) / kSumTileX, cb = warp / G;
+    const unsigned ix = cb * kSumTileX + lane % kSumTileX, iy0 = (warp % G) * kSumTileY + lane / kSumTileX;
+    const unsigned ix2 = (cb + blocks / 2) % blocks * kSumTileX + lane % kSumTileX; // the second half's column
+    const unsigned step = kSumTileY * G;
+    const size_t npix = (size_t)D * D, nbuf = (size_t)D * a.pitch;
     const uint32_t bytes = (uint32_t)(npix * sizeof(float));
     const uint32_t wlim = wait_tries(a.wait_iters);
-    auto issue = [&](unsigned k, unsigned buf) {
+    auto issue = [&](unsigned k, unsigned buf) { // by warp 0
         if (a.test_stall)
             return; // failure-path test: no copy, a wait that runs out
-        const AvgMember b = a.rec[a.order[k]];
-        mrec[buf] = b; // published to the other threads by the arrive below (release) and their wait (acquire)
-        if (GPUISAC_IN_BOUNDS(kChkAvgImg, b.img, a.P)) {
-            mbar_expect_tx(&bars[buf], bytes);
-            bulk_g2s(sbuf + buf * npix, a.imgs + (size_t)b.img * npix, bytes, &bars[buf]);
-        } else {
-            mbar_expect_tx(&bars[buf], 0);
+        const unsigned img_of = mrec[k - k0].img;
+        fence_proxy_async(); // the buffer's readers are done
+        if (lane == 0)
+            mbar_expect_tx(&bars[buf], img_of < a.P ? bytes : 0);
+        __syncwarp();
+        if (GPUISAC_IN_BOUNDS(kChkAvgImg, img_of, a.P)) {
+            const float* img = a.imgs + (size_t)img_of * npix;
+            float* dst = sbuf + buf * nbuf;
+            if (a.pitch == D) {
+                if (lane == 0)
+                    bulk_g2s(dst, img, bytes, &bars[buf]);
+            } else {
+                for (unsigned y = lane; y < D; y += 32)
+                    bulk_g2s(dst + y * a.pitch, img + (size_t)y * D, D * (uint32_t)sizeof(float), &bars[buf]);
+            }
         }
     };
     if (STAGED) {
@@ -391,17 +465,23 @@ avg_sum_kernel(AvgSumArgs a)
             mbar_init(&bars[1], 1);
             mbar_fence_init();
         }
+        for (unsigned k = k0 + tid; k < k1; k += blockDim.x)
+            mrec[k - k0] = a.rec[a.order[k]];
         __syncthreads();
     }
     unsigned u = 0; // members consumed: use u of buffer u & 1 completes phase (u >> 1) & 1
-    for (unsigned row0 = 0; row0 < D; row0 += kRowsPerThread * G) {
-        float acc[kRowsPerThread];
+    // (columns beyond the last are not stored)
+    auto add = [&](f32x2(&acc)[2][ROWS / 4], const float* src, const AvgMember& b, unsigned row0, unsigned pitch) {
+        accumulate<ROWS / 2>(acc[0], src, b, min(ix, D - 1), row0 + iy0, min(row0 + a.half, D), step, D, pitch);
+        accumulate<ROWS / 2>(acc[1], src, b, min(ix2, D - 1), row0 + a.half + iy0, D, step, D, pitch);
+    };
+    for (unsigned row0 = 0; row0 < D; row0 += 2 * a.half) {
+        f32x2 acc[2][ROWS / 4];
 #pragma unroll
-        for (int p = 0; p < kRowsPerThread; p++)
-            acc[p] = 0.0f;
+        for (int p = 0; p < ROWS / 4; p++)
+            acc[0][p] = acc[1][p] = 0;
         if (STAGED) {
-            if (tid == 0) {
-                fence_proxy_async(); // the previous pass read both buffers
+            if (warp == 0) {
                 issue(k0, u & 1u);
                 if (k0 + 1 < k1)
                     issue(k0 + 1, (u + 1) & 1u);
@@ -410,7 +490,7 @@ avg_sum_kernel(AvgSumArgs a)
                 const unsigned buf = u & 1u;
                 const bool ok = mbar_wait(&bars[buf], (u >> 1) & 1u, wlim);
                 if (ok)
-                    accumulate(acc, sbuf + buf * npix, mrec[buf], ix, row0 + g, G, D);
+                    add(acc, sbuf + buf * nbuf, mrec[k - k0], row0, a.pitch);
                 if (__syncthreads_or(!ok)) {
                     if (tid == 0) {
                         atomicAdd(a.err + kErrWait, 1u);
@@ -422,25 +502,25 @@ avg_sum_kernel(AvgSumArgs a)
                     }
                     return;
                 }
-                if (tid == 0 && k + 2 < k1) {
-                    fence_proxy_async();
+                if (warp == 0 && k + 2 < k1)
                     issue(k + 2, buf);
-                }
             }
         } else {
             for (unsigned k = k0; k < k1; k++) {
                 const AvgMember b = a.rec[a.order[k]];
                 if (GPUISAC_IN_BOUNDS(kChkAvgImg, b.img, a.P))
-                    accumulate(acc, a.imgs + (size_t)b.img * npix, b, ix, row0 + g, G, D);
+                    add(acc, a.imgs + (size_t)b.img * npix, b, row0, D);
             }
         }
         float* out = a.partial + (size_t)t * npix;
 #pragma unroll
-        for (int p = 0; p < kRowsPerThread; p++) {
-            const unsigned iy = row0 + g + (unsigned)p * G;
-            if (iy < D && GPUISAC_IN_BOUNDS(kChkAvgPartial, (size_t)t * npix + (size_t)iy * D + ix,
-                                            (size_t)n_pieces * npix))
-                out[(size_t)iy * D + ix] = acc[p];
+        for (int p = 0; p < ROWS; p++) {
+            const int hf = p / (ROWS / 2), ph = p % (ROWS / 2);
+            const unsigned iy = row0 + hf * a.half + iy0 + (unsigned)ph * step, col = hf ? ix2 : ix;
+            const float2 v = unpack_f32x2(acc[hf][ph / 2]);
+            if (col < D && iy < (hf ? D : min(row0 + a.half, D)) &&
+                GPUISAC_IN_BOUNDS(kChkAvgPartial, (size_t)t * npix + (size_t)iy * D + col, (size_t)n_pieces * npix))
+                out[(size_t)iy * D + col] = ph % 2 ? v.y : v.x;
         }
     }
 }
@@ -826,9 +906,11 @@ int fail(int code, const char* msg)
         }                                                                                              \
     } while (0)
 
-// threads D x G: G = ceil(D / 16) (one pass) up to D = 128, else as many
-// rows per pass as 1024 threads give
-unsigned sum_groups(unsigned D) { return D <= 128 ? (D + kRowsPerThread - 1) / kRowsPerThread : 1024 / D; }
+// The sum kernel: images up to side 80 by CTAs of ceil(D / 8) warps with 20 rows a
+// thread, three to an SM; larger ones with 16 rows a thread and two row groups (one
+// pass) up to side 128, one group above.
+constexpr unsigned kSumSmall = 80;
+unsigned sum_groups(unsigned D) { return D <= kSumSmall || D > 128 ? 1 : 2; }
 
 void release(AvgState& w)
 {
@@ -899,17 +981,34 @@ extern "C" int gpuisac_class_averages(const float* imgs, unsigned int n_img, uns
     const unsigned n_chunks = (P + kAvgChunk - 1) / kAvgChunk;
     // member images staged by bulk copies: whole rows of 16-byte multiples
     const bool staged = D % 2 == 0 && D <= kStagedMaxDim && (uintptr_t)imgs % 16 == 0;
-    void (*sum_kernel)(AvgSumArgs) = staged ? avg_sum_kernel<true> : avg_sum_kernel<false>;
-    const unsigned G = sum_groups(D), sum_threads = D * G;
-    const size_t sum_smem = staged ? 2 * sizeof(float) * npix : 0;
+    void (*sum_kernel)(AvgSumArgs) =
+        D <= kSumSmall ? (staged ? avg_sum_kernel<true, 20, 320, 2> : avg_sum_kernel<false, 20, 320, 2>)
+                       : (staged ? avg_sum_kernel<true, 16, 1024, 1> : avg_sum_kernel<false, 16, 1024, 1>);
+    // a row length that is a multiple of 16 floats puts a tile's rows on the same
+    // banks: such an image is staged with 4 more per row, row by row
+    const unsigned pitch = staged && D % 16 == 0 ? D + 4 : D;
+    const unsigned G = sum_groups(D), sum_threads = (D + kSumTileX - 1) / kSumTileX * G * 32;
+    // output rows of a half pass: pairs of tiles, as few as cover the image
+    const unsigned sum_rows = D <= kSumSmall ? 20 : 16, sum_tiles = (D + kSumTileY - 1) / kSumTileY;
+    const unsigned half = std::min(sum_rows / 2, (sum_tiles + 4 * G - 1) / (4 * G) * 2) * kSumTileY * G;
+    const size_t sum_smem = staged ? 2 * sizeof(float) * D * pitch : 0;
     int sms = 0, per_sm = 0;
     AV_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (sum_smem > 48 * 1024)
+    if (sum_smem + kMaxPiece * sizeof(AvgMember) + 64 > 48 * 1024) // (the static arrays count)
         AV_CK(cudaFuncSetAttribute(sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sum_smem));
     AV_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sum_kernel, (int)sum_threads, sum_smem));
-    // pieces of about P / (4 waves of resident CTAs) members, 8..256
-    const unsigned resident = (unsigned)std::max(1, sms * std::max(per_sm, 1));
-    const unsigned piece = std::min(256u, std::max(8u, (P + 4 * resident - 1) / (4 * resident)));
+    // members of a piece: whole waves of resident CTAs if the groups are of equal
+    // size (what the assignment makes; with others only the last wave is less full), a
+    // wave's time taken as its members and two more for the start
+    const unsigned resident = (unsigned)std::max(1, sms * std::max(per_sm, 1)), group = (P + R - 1) / R;
+    unsigned piece = kMinPiece;
+    unsigned long long best = ~0ull;
+    for (unsigned c = kMinPiece; c <= kMaxPiece; c++) {
+        const unsigned long long n = (unsigned long long)R * ((group + c - 1) / c);
+        const unsigned long long cost = (n + resident - 1) / resident * (c + 2);
+        if (cost < best)
+            best = cost, piece = c;
+    }
     const size_t pieces_cap = (size_t)P / piece + R + 1;
     const bool spectra = fl > 0.0f || center;
     const unsigned H = D / 2 + 1, K = (D - 1) / 2;
@@ -954,7 +1053,7 @@ extern "C" int gpuisac_class_averages(const float* imgs, unsigned int n_img, uns
     avg_shift_kernel<<<(R + 7) / 8, 256, 0, st>>>(w.rec.p, w.order.p, w.start.p, w.total.p, R, w.mean.p,
                                                   reinterpret_cast<float2*>(shifts), reinterpret_cast<float4*>(params));
     AvgSumArgs sa{imgs, w.rec.p, w.order.p, w.start.p, w.total.p, w.pstart.p, w.partial.p, w.err.p, P, R, D, G, piece,
-                  0, 0};
+                  pitch, half, 0, 0};
     ccf_test_settings(sa.test_stall, sa.wait_iters);
     sum_kernel<<<(unsigned)pieces_cap, sum_threads, sum_smem, st>>>(sa);
     AvgFinishArgs fa{w.partial.p, w.pstart.p, w.total.p, w.mean.p, w.tw.p, w.scratch.p, averages, R, D, 0, 0, fl, ff,
