@@ -16,7 +16,8 @@
 //           group that received proposals keeps its maxasi best pairs, its
 //           threshold becomes the maxasi-th best pair key, and the rest are
 //           unplaced again;
-//   end:    when a round turns nobody away.  Every group then holds maxasi
+//   end:    when a round turns nobody away (every round and what follows run in one
+//           cooperative grid, up to 1,024 rounds a launch).  Every group then holds maxasi
 //           particles; the one with the lowest threshold is the group the host
 //           algorithm closes last, and the leftover particles join it.
 // The result also comes out as the host function's list: each group's members
@@ -40,13 +41,26 @@
 namespace gpuisac {
 namespace {
 
-constexpr unsigned kRows = 8;         // row slices of d per particle in the proposal scan
-constexpr unsigned kSelThreads = 256; // threads of a group's selection / ranking CTA
-constexpr unsigned kSmallSel = 1024;  // groups up to this many candidates select in shared memory
-constexpr unsigned kSparseDiv = 8;    // a round with at most nima / 8 particles to place uses the list form
-constexpr unsigned kErrNaN = 1u, kErrInternal = 2u;
+constexpr unsigned kThreads = 256;   // 8 warps: a group's selection, 32 particles x 8 row slices, ...
+constexpr unsigned kRows = 8;        // row slices of d per particle in the proposal scan
+// groups up to this many candidates select by counting in shared memory, others by
+// digits: c^2 / 256 steps against two or three passes over c and 256 counters (20,000
+// particles in 20 groups: 582 us in all when 1,024 candidates still counted, 181 now)
+constexpr unsigned kSmallSel = 128;
+constexpr unsigned kSparseDiv = 8;   // a round with at most nima / 8 particles to place uses the list form
+// CTAs of the cooperative grid per SM: two meet faster (20,000 particles x 200 groups:
+// 222 us against 238), four read the peaks of many particles faster (100,000 x 500: 614
+// against 792)
+constexpr unsigned kCtasPerSm = 2, kCtasPerSmWide = 4;
+constexpr unsigned kWideTiles = 8; // tiles of 32 particles per SM from which on four
+constexpr unsigned kMaxRounds = 1024; // per launch (a launch goes on where the last one stopped)
+constexpr unsigned kWaitTries = 1u << 26; // of a grid barrier: tens of seconds
+constexpr unsigned kErrNaN = 1u, kErrInternal = 2u, kErrWait = 4u;
 
-enum { kScNext = 0, kScErr = 1, kScLast = 2, kScLeft = 3, kScCount = 4 };
+// kScNext: particles turned away; kScTotal: bucketed members of a round;
+// kScRounds: rounds done; kScBar: arrivals at the grid barrier
+enum { kScNext = 0, kScErr, kScLast, kScLeft, kScTotal, kScRounds, kScBar = 32, kScCount };
+constexpr unsigned kScWords = 32; // 64-bit words they take (the barrier's line apart, and nothing else on theirs)
 
 __device__ __forceinline__ uint64_t pair_key(float v, uint32_t l)
 {
@@ -55,187 +69,155 @@ __device__ __forceinline__ uint64_t pair_key(float v, uint32_t l)
     return ((uint64_t)u << 32) | (uint64_t)(0xFFFFFFFFu - l);
 }
 
+// One call's arrays.  Those the kernel writes are read by plain loads after a grid
+// barrier (no read-only path).
+struct Assign {
+    const float* d;
+    size_t pitch;
+    unsigned nref, nima, maxasi, extra;
+    bool first;  // nobody has proposed yet
+    int* belongsto;
+    int* out;    // the list, or NULL
+    uint64_t *theta, *pkey, *bk;
+    unsigned *cnt, *touched, *off, *fill, *bp, *list, *sc;
+    unsigned char* redo;
+    int* assign;
+    unsigned wait_tries;
+};
+
+// All CTAs of the (cooperative) grid meet: what each wrote before is seen by all
+// after.  False when the wait ran out in any of them that this one heard of: the
+// caller returns (every other wait of the launch runs out as well).
+__device__ bool grid_meet(const Assign& a, unsigned& target)
+{
+    __shared__ bool s_ok;
+    __syncthreads();
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        unsigned *bar = a.sc + kScBar, seen = 0, tries = 0;
+        __threadfence();
+        atomicAdd(bar, 1u);
+        while (true) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+            if ((int)(seen - target) >= 0 || ++tries > a.wait_tries)
+                break;
+            __nanosleep(20);
+        }
+        s_ok = (int)(seen - target) >= 0;
+        if (!s_ok)
+            atomicOr(a.sc + kScErr, kErrWait);
+        __threadfence();
+    }
+    __syncthreads();
+    return s_ok;
+}
+
+__device__ __forceinline__ void propose_to(const Assign& a, unsigned p, int bg, uint64_t best)
+{
+    a.assign[p] = bg;
+    a.pkey[p] = best;
+    if (bg >= 0) {
+        atomicAdd(a.cnt + bg, 1u);
+        a.touched[bg] = 1u;
+    }
+}
+
 // Each unplaced particle's best pair among the groups whose threshold it
-// beats.  Block = 32 consecutive particles x kRows row slices; the lanes of a
-// warp read one row of d for the block's unplaced particles, so that a round
-// with few of them touches only the 32-byte sectors they share; a block with
-// none returns at once.  redo = NULL: every particle (the first round);
-// otherwise redo[p] = 1 marks the particles turned away last round (cleared
-// here).
-__global__ void __launch_bounds__(32 * kRows)
-propose_kernel(const float* __restrict__ d, size_t pitch, unsigned nref, unsigned nima,
-               unsigned char* __restrict__ redo, const uint64_t* __restrict__ theta, int* __restrict__ assign,
-               uint64_t* __restrict__ pkey, unsigned* __restrict__ cnt, unsigned* __restrict__ touched,
-               unsigned* __restrict__ err)
+// beats.  Tile = 32 consecutive particles x kRows row slices; the lanes of a
+// warp read one row of d for the tile's unplaced particles, so that a round
+// with few of them touches only the 32-byte sectors they share; a tile with
+// none is passed over.  all: every particle (the first round); otherwise
+// redo[p] = 1 marks the particles turned away last round (cleared here).
+__device__ void propose_scan(const Assign& a, bool all)
 {
     __shared__ uint64_t s_key[kRows][32];
     __shared__ int s_grp[kRows][32];
-    const unsigned x = threadIdx.x, y = threadIdx.y;
-    const unsigned p = blockIdx.x * 32 + x;
-    const bool live = p < nima && (!redo || redo[p]);
-    if (!__syncthreads_or(live))
-        return;
-    if (live && redo && y == 0)
-        redo[p] = 0;
-    uint64_t best = 0;
-    int bg = -1;
-    bool nan = false;
-    if (live) {
-        const float* col = d + p;
+    const unsigned x = threadIdx.x & 31u, y = threadIdx.x >> 5;
+    for (unsigned tile = blockIdx.x; tile < (a.nima + 31) / 32; tile += gridDim.x) {
+        const unsigned p = tile * 32 + x;
+        const bool live = p < a.nima && (all || a.redo[p]);
+        if (!__syncthreads_or(live))
+            continue;
+        if (live && !all && y == 0)
+            a.redo[p] = 0;
+        uint64_t best = 0;
+        int bg = -1;
+        bool nan = false;
+        if (live) {
+            const float* col = a.d + p;
 #pragma unroll 4
-        for (unsigned g = y; g < nref; g += kRows) {
-            const float v = __ldg(col + (size_t)g * pitch);
-            nan |= (v != v);
-            const uint64_t k = pair_key(v, g * nima + p);
-            if (k > best && k > __ldg(theta + g)) {
-                best = k;
-                bg = (int)g;
+            for (unsigned g = y; g < a.nref; g += kRows) {
+                const float v = __ldg(col + (size_t)g * a.pitch);
+                nan |= (v != v);
+                const uint64_t k = pair_key(v, g * a.nima + p);
+                if (k > best && k > a.theta[g]) {
+                    best = k;
+                    bg = (int)g;
+                }
             }
         }
-    }
-    if (nan)
-        atomicOr(err, kErrNaN);
-    s_key[y][x] = best;
-    s_grp[y][x] = bg;
-    __syncthreads();
-    if (y == 0 && live) {
+        if (nan)
+            atomicOr(a.sc + kScErr, kErrNaN);
+        s_key[y][x] = best;
+        s_grp[y][x] = bg;
+        __syncthreads();
+        if (y == 0 && live) {
 #pragma unroll
-        for (unsigned r = 1; r < kRows; r++)
-            if (s_key[r][x] > best) {
-                best = s_key[r][x];
-                bg = s_grp[r][x];
-            }
-        assign[p] = bg;
-        pkey[p] = best;
-        if (bg >= 0) {
-            atomicAdd(cnt + bg, 1u);
-            touched[bg] = 1u;
+            for (unsigned r = 1; r < kRows; r++)
+                if (s_key[r][x] > best) {
+                    best = s_key[r][x];
+                    bg = s_grp[r][x];
+                }
+            propose_to(a, p, bg, best);
         }
+        __syncthreads();
     }
 }
 
 // The list form of the proposal scan, for rounds with few particles to
 // place: one warp per particle of list[0..n), its lanes striding over the
 // rows of the particle's column, the best pair found by a warp reduction.
-__global__ void __launch_bounds__(256)
-propose_list_kernel(const float* __restrict__ d, size_t pitch, unsigned nref, unsigned nima,
-                    const unsigned* __restrict__ list, unsigned n, unsigned char* __restrict__ redo,
-                    const uint64_t* __restrict__ theta, int* __restrict__ assign, uint64_t* __restrict__ pkey,
-                    unsigned* __restrict__ cnt, unsigned* __restrict__ touched, unsigned* __restrict__ err)
+__device__ void propose_listed(const Assign& a, unsigned n)
 {
     const unsigned lane = threadIdx.x & 31;
-    const unsigned i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (i >= n)
-        return;
-    const unsigned p = list[i];
-    uint64_t best = 0;
-    int bg = -1;
-    bool nan = false;
-    const float* col = d + p;
+    for (unsigned i = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); i < n; i += gridDim.x * (kThreads / 32)) {
+        const unsigned p = a.list[i];
+        uint64_t best = 0;
+        int bg = -1;
+        bool nan = false;
+        const float* col = a.d + p;
 #pragma unroll 4
-    for (unsigned g = lane; g < nref; g += 32) {
-        const float v = __ldg(col + (size_t)g * pitch);
-        nan |= (v != v);
-        const uint64_t k = pair_key(v, g * nima + p);
-        if (k > best && k > __ldg(theta + g)) {
-            best = k;
-            bg = (int)g;
-        }
-    }
-#pragma unroll
-    for (unsigned o = 16; o > 0; o >>= 1) {
-        const uint64_t ok = __shfl_xor_sync(0xFFFFFFFFu, best, o);
-        const int og = __shfl_xor_sync(0xFFFFFFFFu, bg, o);
-        if (ok > best) {
-            best = ok;
-            bg = og;
-        }
-    }
-    if (__any_sync(0xFFFFFFFFu, nan) && lane == 0)
-        atomicOr(err, kErrNaN);
-    if (lane == 0) {
-        redo[p] = 0;
-        assign[p] = bg;
-        pkey[p] = best;
-        if (bg >= 0) {
-            atomicAdd(cnt + bg, 1u);
-            touched[bg] = 1u;
-        }
-    }
-}
-
-// Exclusive scan of the member counts of the groups that received proposals
-// (one CTA of 1024 threads); clears the fill counters and the next round's
-// list length.
-__global__ void __launch_bounds__(1024)
-offsets_kernel(unsigned nref, const unsigned* __restrict__ cnt, const unsigned* __restrict__ touched,
-               unsigned* __restrict__ off, unsigned* __restrict__ fill, unsigned* __restrict__ n_next)
-{
-    __shared__ unsigned s_warp[32];
-    __shared__ unsigned s_carry;
-    const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        s_carry = 0;
-        *n_next = 0;
-    }
-    __syncthreads();
-    for (unsigned b = 0; b < nref; b += 1024) {
-        const unsigned g = b + threadIdx.x;
-        const unsigned v = (g < nref && touched[g]) ? cnt[g] : 0u;
-        unsigned s = v;
-#pragma unroll
-        for (unsigned o = 1; o < 32; o <<= 1) {
-            const unsigned t = __shfl_up_sync(0xFFFFFFFFu, s, o);
-            if (lane >= o)
-                s += t;
-        }
-        if (lane == 31)
-            s_warp[w] = s;
-        __syncthreads();
-        if (w == 0) {
-            unsigned ws = s_warp[lane];
-#pragma unroll
-            for (unsigned o = 1; o < 32; o <<= 1) {
-                const unsigned t = __shfl_up_sync(0xFFFFFFFFu, ws, o);
-                if (lane >= o)
-                    ws += t;
+        for (unsigned g = lane; g < a.nref; g += 32) {
+            const float v = __ldg(col + (size_t)g * a.pitch);
+            nan |= (v != v);
+            const uint64_t k = pair_key(v, g * a.nima + p);
+            if (k > best && k > a.theta[g]) {
+                best = k;
+                bg = (int)g;
             }
-            s_warp[lane] = ws;
         }
-        __syncthreads();
-        const unsigned incl = s + (w ? s_warp[w - 1] : 0u);
-        if (g < nref) {
-            off[g] = s_carry + incl - v;
-            fill[g] = 0;
+#pragma unroll
+        for (unsigned o = 16; o > 0; o >>= 1) {
+            const uint64_t ok = __shfl_xor_sync(0xFFFFFFFFu, best, o);
+            const int og = __shfl_xor_sync(0xFFFFFFFFu, bg, o);
+            if (ok > best) {
+                best = ok;
+                bg = og;
+            }
         }
-        __syncthreads();
-        if (threadIdx.x == 1023)
-            s_carry += incl;
-        __syncthreads();
+        if (__any_sync(0xFFFFFFFFu, nan) && lane == 0)
+            atomicOr(a.sc + kScErr, kErrNaN);
+        if (lane == 0) {
+            a.redo[p] = 0;
+            propose_to(a, p, bg, best);
+        }
     }
-}
-
-// Members of the groups that received proposals, bucketed by group.
-__global__ void __launch_bounds__(256)
-scatter_kernel(unsigned nima, const int* __restrict__ assign, const uint64_t* __restrict__ pkey,
-               const unsigned* __restrict__ touched, const unsigned* __restrict__ off, unsigned* __restrict__ fill,
-               unsigned* __restrict__ bp, uint64_t* __restrict__ bk)
-{
-    const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= nima)
-        return;
-    const int g = assign[p];
-    if (g < 0 || !touched[g])
-        return;
-    const unsigned s = off[g] + atomicAdd(fill + g, 1u);
-    bp[s] = p;
-    bk[s] = pkey[p];
 }
 
 // The k-th largest of c distinct keys (1 <= k <= c), by a radix select over
 // the 8-bit digits from the top, in one CTA; stops early once one key is left
 // in the selected bucket.
-__device__ uint64_t kth_largest(const uint64_t* __restrict__ keys, unsigned c, unsigned k)
+__device__ uint64_t kth_largest(const uint64_t* keys, unsigned c, unsigned k)
 {
     __shared__ unsigned hist[256];
     __shared__ uint64_t s_prefix, s_found;
@@ -252,17 +234,30 @@ __device__ uint64_t kth_largest(const uint64_t* __restrict__ keys, unsigned c, u
                 atomicAdd(&hist[(unsigned)(v >> shift) & 255u], 1u);
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned acc = 0;
-            int b = 255;
-            for (; b > 0; b--) {
-                if (acc + hist[b] >= kk)
-                    break;
-                acc += hist[b];
+        if (threadIdx.x < 32) {
+            // lane l has bins 255 - 8 l down to 248 - 8 l; the bin that holds the kk-th
+            // largest is in the first lane whose sum from the top reaches kk
+            const unsigned top = 255u - 8u * threadIdx.x;
+            unsigned own = 0;
+#pragma unroll
+            for (unsigned i = 0; i < 8; i++)
+                own += hist[top - i];
+            unsigned acc = own;
+#pragma unroll
+            for (unsigned o = 1; o < 32; o <<= 1) {
+                const unsigned up = __shfl_up_sync(0xFFFFFFFFu, acc, o);
+                if (threadIdx.x >= o)
+                    acc += up;
             }
-            s_prefix = prefix | ((uint64_t)b << shift);
-            s_k = kk - acc;
-            s_single = hist[b] == 1u;
+            if (acc >= kk && acc - own < kk) {
+                acc -= own;
+                unsigned b = top;
+                while (acc + hist[b] < kk)
+                    acc += hist[b--];
+                s_prefix = prefix | ((uint64_t)b << shift);
+                s_k = kk - acc;
+                s_single = hist[b] == 1u;
+            }
         }
         __syncthreads();
         prefix = s_prefix;
@@ -284,7 +279,7 @@ __device__ uint64_t kth_largest(const uint64_t* __restrict__ keys, unsigned c, u
 
 // The k-th largest of c <= kSmallSel distinct keys: the one with exactly
 // k - 1 larger keys, counted against a copy in shared memory.
-__device__ uint64_t kth_largest_small(const uint64_t* __restrict__ keys, unsigned c, unsigned k)
+__device__ uint64_t kth_largest_small(const uint64_t* keys, unsigned c, unsigned k)
 {
     __shared__ uint64_t s_keys[kSmallSel];
     __shared__ uint64_t s_found;
@@ -294,6 +289,7 @@ __device__ uint64_t kth_largest_small(const uint64_t* __restrict__ keys, unsigne
     for (unsigned i = threadIdx.x; i < c; i += blockDim.x) {
         const uint64_t v = s_keys[i];
         unsigned larger = 0;
+#pragma unroll 8
         for (unsigned j = 0; j < c; j++)
             larger += s_keys[j] > v;
         if (larger == k - 1)
@@ -306,148 +302,189 @@ __device__ uint64_t kth_largest_small(const uint64_t* __restrict__ keys, unsigne
 // One CTA per group: a group with proposals and at least maxasi members keeps
 // its maxasi best, takes the maxasi-th best key as its threshold and turns
 // the others away: marked in redo and appended to list (they propose again
-// next round); n_next counts them.
-__global__ void __launch_bounds__(kSelThreads)
-select_kernel(unsigned maxasi, const unsigned* __restrict__ off, const unsigned* __restrict__ bp,
-              const uint64_t* __restrict__ bk, unsigned* __restrict__ cnt, unsigned* __restrict__ touched,
-              uint64_t* __restrict__ theta, int* __restrict__ assign, unsigned char* __restrict__ redo,
-              unsigned* __restrict__ list, unsigned* __restrict__ n_next)
+// next round); kScNext counts them.
+__device__ void select_best(const Assign& a, unsigned g)
 {
-    const unsigned g = blockIdx.x;
-    const unsigned t = touched[g], c = cnt[g];
+    const unsigned t = a.touched[g], c = a.cnt[g];
     __syncthreads();
     if (!t)
         return;
     if (threadIdx.x == 0)
-        touched[g] = 0;
-    if (c < maxasi)
+        a.touched[g] = 0;
+    if (c < a.maxasi)
         return;
-    const unsigned base = off[g];
-    const uint64_t kth = c <= kSmallSel ? kth_largest_small(bk + base, c, maxasi) : kth_largest(bk + base, c, maxasi);
-    if (c > maxasi)
-        for (unsigned i = threadIdx.x; i < c; i += blockDim.x)
-            if (bk[base + i] < kth) {
-                const unsigned p = bp[base + i];
-                assign[p] = -1;
-                redo[p] = 1;
-                list[atomicAdd(n_next, 1u)] = p;
+    const unsigned base = a.off[g];
+    const uint64_t* bk = a.bk + base;
+    const uint64_t kth = c <= kSmallSel ? kth_largest_small(bk, c, a.maxasi) : kth_largest(bk, c, a.maxasi);
+    if (c > a.maxasi)
+        for (unsigned i = threadIdx.x; i < c; i += kThreads)
+            if (bk[i] < kth) {
+                const unsigned p = a.bp[base + i];
+                a.assign[p] = -1;
+                a.redo[p] = 1;
+                a.list[atomicAdd(a.sc + kScNext, 1u)] = p;
             }
     if (threadIdx.x == 0) {
-        theta[g] = kth;
-        cnt[g] = maxasi;
+        a.theta[g] = kth;
+        a.cnt[g] = a.maxasi;
     }
 }
 
-// The group that closed last (lowest threshold); checks that every group
-// holds maxasi members.
-__global__ void __launch_bounds__(1024)
-last_group_kernel(unsigned nref, unsigned maxasi, const uint64_t* __restrict__ theta,
-                  const unsigned* __restrict__ cnt, unsigned* __restrict__ sc)
+// The group that closed last (lowest threshold), found by every CTA for itself;
+// the first checks that every group holds maxasi members.
+__device__ unsigned last_group(const Assign& a)
 {
-    __shared__ uint64_t s_key[1024];
-    __shared__ unsigned s_grp[1024];
+    __shared__ uint64_t s_key[kThreads];
+    __shared__ unsigned s_grp[kThreads];
     uint64_t best = ~0ull;
     unsigned bg = 0;
-    for (unsigned g = threadIdx.x; g < nref; g += 1024) {
-        if (cnt[g] != maxasi || theta[g] == 0)
-            atomicOr(sc + kScErr, kErrInternal);
-        if (theta[g] < best) {
-            best = theta[g];
+    for (unsigned g = threadIdx.x; g < a.nref; g += kThreads) {
+        const uint64_t t = a.theta[g];
+        if (blockIdx.x == 0 && (a.cnt[g] != a.maxasi || t == 0))
+            atomicOr(a.sc + kScErr, kErrInternal);
+        if (t < best) {
+            best = t;
             bg = g;
         }
     }
     s_key[threadIdx.x] = best;
     s_grp[threadIdx.x] = bg;
     __syncthreads();
-    for (unsigned h = 512; h > 0; h >>= 1) {
+    for (unsigned h = kThreads / 2; h > 0; h >>= 1) {
         if (threadIdx.x < h && s_key[threadIdx.x + h] < s_key[threadIdx.x]) {
             s_key[threadIdx.x] = s_key[threadIdx.x + h];
             s_grp[threadIdx.x] = s_grp[threadIdx.x + h];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        sc[kScLast] = s_grp[0];
-        sc[kScLeft] = 0;
-    }
+    return s_grp[0];
 }
 
-// belongsto; a leftover particle joins the last group (its pair key with that
-// group ranks it among the leftovers) and is tagged with group index nref.
-__global__ void __launch_bounds__(256)
-belong_kernel(const float* __restrict__ d, size_t pitch, unsigned nref, unsigned nima, int* __restrict__ assign,
-              uint64_t* __restrict__ pkey, int* __restrict__ belongsto, unsigned* __restrict__ sc)
-{
-    const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= nima)
-        return;
-    int g = assign[p];
-    if (g < 0) {
-        const unsigned last = sc[kScLast];
-        pkey[p] = pair_key(d[(size_t)last * pitch + p], last * nima + p);
-        assign[p] = (int)nref;
-        atomicAdd(sc + kScLeft, 1u);
-        g = (int)last;
-    }
-    if (belongsto)
-        belongsto[p] = g;
-}
-
-// Members bucketed by final group: group g at g*maxasi, the leftovers at
-// nref*maxasi (fill has nref+1 counters).
-__global__ void __launch_bounds__(256)
-scatter_final_kernel(unsigned nref, unsigned nima, unsigned maxasi, unsigned extra, const int* __restrict__ assign,
-                     const uint64_t* __restrict__ pkey, unsigned* __restrict__ fill, unsigned* __restrict__ bp,
-                     uint64_t* __restrict__ bk, unsigned* __restrict__ sc)
-{
-    const unsigned p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= nima)
-        return;
-    const unsigned g = (unsigned)assign[p];
-    const unsigned cap = g < nref ? maxasi : extra;
-    const unsigned j = atomicAdd(fill + g, 1u);
-    if (g > nref || j >= cap) {
-        atomicOr(sc + kScErr, kErrInternal);
-        return;
-    }
-    const unsigned s = g * maxasi + j;
-    bp[s] = p;
-    bk[s] = pkey[p];
-}
-
-// Rank of each member within its group by counting the larger keys: CTA
-// (g, chunk) places members chunk*256 .. +255 of group g (g = nref: the
+// Rank of each member within its group by counting the larger keys: chunk
+// `chunk` places members chunk*256 .. +255 of group g (g = nref: the
 // leftovers) at their rank.
-__global__ void __launch_bounds__(kSelThreads)
-rank_kernel(unsigned nref, unsigned maxasi, unsigned extra, const unsigned* __restrict__ bp,
-            const uint64_t* __restrict__ bk, int* __restrict__ out, const unsigned* __restrict__ sc)
+__device__ void rank_chunk(const Assign& a, unsigned g, unsigned chunk)
 {
-    __shared__ uint64_t tile[kSelThreads];
-    const unsigned g = blockIdx.x;
-    const unsigned c = g < nref ? maxasi : extra;
-    const unsigned base = g * maxasi;
-    const unsigned i = blockIdx.y * kSelThreads + threadIdx.x;
-    if (blockIdx.y * kSelThreads >= c) {
-        if (g == nref && blockIdx.y == 0 && threadIdx.x == 0)
-            out[nref * maxasi + extra] = (int)sc[kScLast];
-        return;
-    }
+    __shared__ uint64_t tile[kThreads];
+    const unsigned c = g < a.nref ? a.maxasi : a.extra;
+    const unsigned base = g * a.maxasi, i = chunk * kThreads + threadIdx.x;
     const bool live = i < c;
-    const uint64_t ki = live ? bk[base + i] : 0;
+    const uint64_t ki = live ? a.bk[base + i] : 0;
     unsigned r = 0;
-    for (unsigned j0 = 0; j0 < c; j0 += kSelThreads) {
+    for (unsigned j0 = 0; j0 < c; j0 += kThreads) {
         __syncthreads();
         if (j0 + threadIdx.x < c)
-            tile[threadIdx.x] = bk[base + j0 + threadIdx.x];
+            tile[threadIdx.x] = a.bk[base + j0 + threadIdx.x];
         __syncthreads();
-        const unsigned m = min(kSelThreads, c - j0);
+        const unsigned m = min(kThreads, c - j0);
+#pragma unroll 8
         for (unsigned j = 0; j < m; j++)
             r += tile[j] > ki;
     }
     if (live)
-        out[base + r] = (int)bp[base + i];
-    if (g == nref && blockIdx.y == 0 && threadIdx.x == 0)
-        out[nref * maxasi + extra] = (int)sc[kScLast];
+        a.out[base + r] = (int)a.bp[base + i];
+}
+
+// The rounds and what follows them, in one cooperative grid that meets between
+// steps.  What bounds it: the meetings (four a round) and the steps' dependent
+// loads.  As four kernels a round with a read of the count after each, launches and
+// reads were most of the time: 20,000 particles x 200 groups (9 rounds) 376 us, now
+// 233; 3,000 x 76 (7) 274 -> 135; 300 x 7 (4) 179 -> 82; 100,000 x 500 (10) 661 ->
+// 579.  The count read after every third or fourth such round: 311 to 362 us.
+__global__ void __launch_bounds__(kThreads)
+assign_kernel(Assign a)
+{
+    const unsigned t0 = blockIdx.x * kThreads + threadIdx.x, nt = gridDim.x * kThreads;
+    unsigned target = 0;
+    for (unsigned round = 0;; round++) {
+        const bool all = a.first && round == 0;
+        // (changed next after the meeting that follows the proposals)
+        const unsigned n = all ? a.nima : __ldcg(a.sc + kScNext);
+        if (n == 0)
+            break;
+        if (round == kMaxRounds)
+            return;
+        if (!all && n <= a.nima / kSparseDiv)
+            propose_listed(a, n);
+        else
+            propose_scan(a, all);
+        if (!grid_meet(a, target) || (__ldcg(a.sc + kScErr) & kErrNaN))
+            return;
+        // room for the members of the groups that received proposals, in any order
+        for (unsigned g = t0; g < a.nref; g += nt)
+            if (a.touched[g]) {
+                a.off[g] = atomicAdd(a.sc + kScTotal, a.cnt[g]);
+                a.fill[g] = 0;
+            }
+        if (t0 == 0) {
+            a.sc[kScNext] = 0;
+            a.sc[kScRounds]++;
+        }
+        if (!grid_meet(a, target))
+            return;
+        // the members, bucketed by group
+        for (unsigned p = t0; p < a.nima; p += nt) {
+            const int g = a.assign[p];
+            if (g >= 0 && a.touched[g]) {
+                const unsigned s = a.off[g] + atomicAdd(a.fill + g, 1u);
+                a.bp[s] = p;
+                a.bk[s] = a.pkey[p];
+            }
+        }
+        if (!grid_meet(a, target))
+            return;
+        if (t0 == 0)
+            a.sc[kScTotal] = 0;
+        for (unsigned g = blockIdx.x; g < a.nref; g += gridDim.x)
+            select_best(a, g);
+        if (!grid_meet(a, target))
+            return;
+    }
+
+    // belongsto; a leftover particle joins the last group (its pair key with that
+    // group ranks it among the leftovers) and is tagged with group index nref
+    const unsigned last = last_group(a);
+    if (t0 == 0)
+        a.sc[kScLast] = last;
+    for (unsigned g = t0; g <= a.nref; g += nt)
+        a.fill[g] = 0;
+    for (unsigned p = t0; p < a.nima; p += nt) {
+        int g = a.assign[p];
+        if (g < 0) {
+            a.pkey[p] = pair_key(a.d[(size_t)last * a.pitch + p], last * a.nima + p);
+            a.assign[p] = (int)a.nref;
+            atomicAdd(a.sc + kScLeft, 1u);
+            g = (int)last;
+        }
+        if (a.belongsto)
+            a.belongsto[p] = g;
+    }
+    if (!a.out || !grid_meet(a, target))
+        return;
+    // members bucketed by final group: group g at g*maxasi, the leftovers at
+    // nref*maxasi
+    for (unsigned p = t0; p < a.nima; p += nt) {
+        const unsigned g = (unsigned)a.assign[p];
+        const unsigned cap = g < a.nref ? a.maxasi : a.extra;
+        const unsigned j = g <= a.nref ? atomicAdd(a.fill + g, 1u) : cap;
+        if (j >= cap) {
+            atomicOr(a.sc + kScErr, kErrInternal);
+            continue;
+        }
+        const unsigned s = g * a.maxasi + j;
+        a.bp[s] = p;
+        a.bk[s] = a.pkey[p];
+    }
+    if (!grid_meet(a, target) || (__ldcg(a.sc + kScErr) & kErrInternal))
+        return;
+    const unsigned chunks = (a.maxasi + kThreads - 1) / kThreads, chunks_left = (a.extra + kThreads - 1) / kThreads;
+    const unsigned long long items = (unsigned long long)a.nref * chunks + chunks_left;
+    for (unsigned long long i = blockIdx.x; i < items; i += gridDim.x) {
+        const unsigned g = (unsigned)min(i / chunks, (unsigned long long)a.nref);
+        rank_chunk(a, g, (unsigned)(i - (unsigned long long)g * chunks));
+    }
+    if (t0 == 0)
+        a.out[(size_t)a.nref * a.maxasi + a.extra] = (int)last;
 }
 
 template <typename T>
@@ -471,9 +508,9 @@ struct Buf {
 
 struct AssignState {
     std::mutex mu;
-    Buf<uint64_t> theta, pkey, bk;
-    Buf<unsigned> cnt, touched, off, fill, bp, list, sc;
-    Buf<unsigned char> redo;
+    Buf<uint64_t> zeroed; // sc, theta, cnt, touched, redo: what a call starts from zero
+    Buf<uint64_t> pkey, bk;
+    Buf<unsigned> off, fill, bp, list;
     Buf<int> assign;
     Buf<float> d_host_copy;
     Buf<int> ids_host_copy;
@@ -506,7 +543,7 @@ int check_args(const float* d, unsigned long long pitch, unsigned nref, unsigned
         return fail(2, "assign_groups: nref * nima must stay below 2^32");
     if (pitch < nima)
         return fail(2, "assign_groups: d_pitch smaller than nima");
-    if ((nima / nref + kSelThreads - 1) / kSelThreads > 65535u)
+    if ((nima / nref + kThreads - 1) / kThreads > 65535u)
         return fail(2, "assign_groups: groups of more than 16,776,960 particles");
     return 0;
 }
@@ -516,76 +553,56 @@ int assign_locked(const float* d, size_t pitch, unsigned nref, unsigned nima, in
 {
     AssignState& w = g_asg;
     const unsigned maxasi = nima / nref, extra = nima % nref;
-    A_CK(w.theta.ensure(nref));
-    A_CK(w.cnt.ensure(nref));
-    A_CK(w.touched.ensure(nref));
+    const size_t zero_words = kScWords + 2 * (size_t)nref + ((size_t)nima + 7) / 8;
+    A_CK(w.zeroed.ensure(zero_words));
+    unsigned* const sc = reinterpret_cast<unsigned*>(w.zeroed.p);
+    uint64_t* const theta = w.zeroed.p + kScWords;
+    unsigned *const cnt = reinterpret_cast<unsigned*>(theta + nref), *const touched = cnt + nref;
+    unsigned char* const redo = reinterpret_cast<unsigned char*>(theta + 2 * (size_t)nref);
     A_CK(w.off.ensure(nref));
     A_CK(w.fill.ensure(nref + 1));
     A_CK(w.assign.ensure(nima));
     A_CK(w.pkey.ensure(nima));
     A_CK(w.bp.ensure(nima));
     A_CK(w.bk.ensure(nima));
-    A_CK(w.redo.ensure(nima));
     A_CK(w.list.ensure(nima));
-    A_CK(w.sc.ensure(kScCount));
     if (!w.h_sc)
         A_CK(cudaHostAlloc(&w.h_sc, kScCount * sizeof(unsigned), cudaHostAllocDefault));
 
-    A_CK(cudaMemsetAsync(w.theta.p, 0, nref * sizeof(uint64_t), st));
-    A_CK(cudaMemsetAsync(w.cnt.p, 0, nref * sizeof(unsigned), st));
-    A_CK(cudaMemsetAsync(w.touched.p, 0, nref * sizeof(unsigned), st));
-    A_CK(cudaMemsetAsync(w.sc.p, 0, kScCount * sizeof(unsigned), st));
+    A_CK(cudaMemsetAsync(w.zeroed.p, 0, zero_words * sizeof(uint64_t), st));
 
-    A_CK(cudaMemsetAsync(w.redo.p, 0, nima, st));
-
+    int dev = 0, sms = 0, per_sm = 0;
+    A_CK(cudaGetDevice(&dev));
+    A_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    A_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, assign_kernel, (int)kThreads, 0));
+    const unsigned tiles = (nima + 31) / 32;
+    const unsigned want = tiles >= kWideTiles * (unsigned)sms ? kCtasPerSmWide : kCtasPerSm;
+    // no more CTAs than the widest step has work for
+    const unsigned grid = std::min((unsigned)sms * std::min((unsigned)std::max(per_sm, 1), want), std::max(tiles, nref));
+    Assign a{d, pitch, nref, nima, maxasi, extra, true, belongsto, id_list_long, theta, w.pkey.p, w.bk.p,
+             cnt, touched, w.off.p, w.fill.p, w.bp.p, w.list.p, sc, redo, w.assign.p, kWaitTries};
     const unsigned long long max_rounds = (unsigned long long)nref * nima + 1;
-    unsigned rounds = 0, turned = nima;
+    unsigned rounds = 0;
     for (;;) {
-        // the list written by the previous round's selection is read here,
-        // before this round's selection rewrites it
-        if (rounds > 0 && turned <= nima / kSparseDiv)
-            propose_list_kernel<<<(turned + 7) / 8, 256, 0, st>>>(d, pitch, nref, nima, w.list.p, turned, w.redo.p,
-                                                                  w.theta.p, w.assign.p, w.pkey.p, w.cnt.p,
-                                                                  w.touched.p, w.sc.p + kScErr);
-        else
-            propose_kernel<<<(nima + 31) / 32, dim3(32, kRows), 0, st>>>(d, pitch, nref, nima,
-                                                                          rounds ? w.redo.p : nullptr, w.theta.p,
-                                                                          w.assign.p, w.pkey.p, w.cnt.p,
-                                                                          w.touched.p, w.sc.p + kScErr);
-        offsets_kernel<<<1, 1024, 0, st>>>(nref, w.cnt.p, w.touched.p, w.off.p, w.fill.p, w.sc.p + kScNext);
-        scatter_kernel<<<(nima + 255) / 256, 256, 0, st>>>(nima, w.assign.p, w.pkey.p, w.touched.p, w.off.p,
-                                                           w.fill.p, w.bp.p, w.bk.p);
-        select_kernel<<<nref, kSelThreads, 0, st>>>(maxasi, w.off.p, w.bp.p, w.bk.p, w.cnt.p, w.touched.p,
-                                                     w.theta.p, w.assign.p, w.redo.p, w.list.p, w.sc.p + kScNext);
-        g_kernel_launches.fetch_add(4, std::memory_order_relaxed);
-        A_CK(cudaGetLastError());
-        A_CK(cudaMemcpyAsync(w.h_sc, w.sc.p, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        void* args[] = {&a};
+        A_CK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(assign_kernel), dim3(grid), dim3(kThreads), args,
+                                         0, st));
+        g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+        A_CK(cudaMemcpyAsync(w.h_sc, sc, kScCount * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
         A_CK(cudaStreamSynchronize(st));
-        rounds++;
+        rounds = w.h_sc[kScRounds];
+        if (w.h_sc[kScErr] & kErrWait)
+            return fail(1, "assign_groups: a grid barrier timed out (bounded wait ran out)");
         if (w.h_sc[kScErr] & kErrNaN)
             return fail(2, "assign_groups: d holds a NaN peak");
-        turned = w.h_sc[kScNext];
+        const unsigned turned = w.h_sc[kScNext];
         if (turned == 0)
             break;
         if (turned > nima || rounds >= max_rounds)
             return fail(1, "assign_groups: the proposal rounds did not settle (internal error)");
+        a.first = false;
+        A_CK(cudaMemsetAsync(sc + kScBar, 0, sizeof(unsigned), st));
     }
-
-    last_group_kernel<<<1, 1024, 0, st>>>(nref, maxasi, w.theta.p, w.cnt.p, w.sc.p);
-    belong_kernel<<<(nima + 255) / 256, 256, 0, st>>>(d, pitch, nref, nima, w.assign.p, w.pkey.p, belongsto, w.sc.p);
-    g_kernel_launches.fetch_add(2, std::memory_order_relaxed);
-    if (id_list_long) {
-        A_CK(cudaMemsetAsync(w.fill.p, 0, (nref + 1) * sizeof(unsigned), st));
-        scatter_final_kernel<<<(nima + 255) / 256, 256, 0, st>>>(nref, nima, maxasi, extra, w.assign.p, w.pkey.p,
-                                                                 w.fill.p, w.bp.p, w.bk.p, w.sc.p);
-        const unsigned chunks = (std::max(std::max(maxasi, extra), 1u) + kSelThreads - 1) / kSelThreads;
-        rank_kernel<<<dim3(nref + 1, chunks), kSelThreads, 0, st>>>(nref, maxasi, extra, w.bp.p, w.bk.p,
-                                                                   id_list_long, w.sc.p);
-        g_kernel_launches.fetch_add(2, std::memory_order_relaxed);
-    }
-    A_CK(cudaGetLastError());
-    A_CK(cudaMemcpyAsync(w.h_sc, w.sc.p, kScCount * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    A_CK(cudaStreamSynchronize(st));
     if ((w.h_sc[kScErr] & kErrInternal) || w.h_sc[kScLeft] != extra)
         return fail(1, "assign_groups: inconsistent group sizes (internal error)");
     if (rounds_out)
@@ -605,8 +622,8 @@ void assign_clear()
         b.p = nullptr;
         b.n = 0;
     };
-    drop(w.theta), drop(w.pkey), drop(w.bk), drop(w.cnt), drop(w.touched), drop(w.off), drop(w.fill);
-    drop(w.bp), drop(w.list), drop(w.sc), drop(w.redo), drop(w.assign), drop(w.d_host_copy);
+    drop(w.zeroed), drop(w.pkey), drop(w.bk), drop(w.off), drop(w.fill);
+    drop(w.bp), drop(w.list), drop(w.assign), drop(w.d_host_copy);
     drop(w.ids_host_copy);
     if (w.h_sc)
         cudaFreeHost(w.h_sc);
