@@ -1001,9 +1001,11 @@ extern "C" int gpuisac_class_averages(const float* imgs, unsigned int n_img, uns
     // size (what the assignment makes; with others only the last wave is less full), a
     // wave's time taken as its members and two more for the start
     const unsigned resident = (unsigned)std::max(1, sms * std::max(per_sm, 1)), group = (P + R - 1) / R;
-    unsigned piece = kMinPiece;
+    // (pieces of fewer than 8 only where their partial images stay few)
+    const unsigned least = P / kMinPiece + R <= 4 * resident ? kMinPiece : 8u;
+    unsigned piece = least;
     unsigned long long best = ~0ull;
-    for (unsigned c = kMinPiece; c <= kMaxPiece; c++) {
+    for (unsigned c = least; c <= kMaxPiece; c++) {
         const unsigned long long n = (unsigned long long)R * ((group + c - 1) / c);
         const unsigned long long cost = (n + resident - 1) / resident * (c + 2);
         if (cost < best)
