@@ -316,9 +316,14 @@ ccf_peak_tmem_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned rin
 // at 29 rings 1.18 -> 1.07).  On the way: two references per group in one team
 // 40.5 (four FFT warps wait on their own latency), two teams 36.4, halves 33.9.
 // The pair's best so far (`bests`) spares the transforms below it the index
-// search: 33.9 -> 33.2 ms (32 groups' search 35.4 -> 34.8).
+// search: 33.9 -> 33.2 ms (32 groups' search 35.4 -> 34.8).  The references on their
+// way to tensor memory loaded five ring pairs at a time through row pointers: 33.2 ->
+// 31.5 ms (pairs one at a time through the pointers 33.0, two 31.7, three 31.9, four
+// 31.8; 61 rings 8.40 -> 7.94; the learned search of one-particle items, 4,000 x 16 and
+// 200 x 200, 9.5 -> 7.2).
 // Not kept: packed FMAs in the contraction (bit-identical; 35.7 against 33.9),
 // the staging area refilled in parts of a row as they are summed (47).
+constexpr unsigned kRefBatch = 5; // ring pairs of the references a thread loads at once
 constexpr int kWsBarC = 1;      // contraction side, item changes
 constexpr int kWsBarCH = 2;     // + half: 2, 3 (one half of the contraction side)
 constexpr int kWsBarFull = 4;   // + 2 buffer + half: 4 .. 7
@@ -485,19 +490,36 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
             if (tid == 0)
                 next_item[ii & 3u] = w.item_counter ? gridDim.x + atomicAdd(w.item_counter, 1u) : item + gridDim.x;
             // this item's references -> tensor memory (both halves read every ring)
-            for (unsigned j = 2 * half; j < nrp; j += 2 * (NC / 128)) {
+            // (kRefBatch ring pairs' loads in flight: this is pure latency, an
+            // eighth of the time of an item of one particle with one at a time)
+            {
+                const float2* rp[QT];
 #pragma unroll
-                for (int jj = 0; jj < 2; jj++) {
-                    float v[8];
+                for (int q = 0; q < QT; q++)
+                    rp[q] = q0 + q < grp.n_ref
+                                ? grp.ref_sp + (size_t)ref_row(grp, q0 + q) * ring_num * kSlots + k
+                                : nullptr;
+                constexpr unsigned kStep = 2 * (NC / 128);
+                for (unsigned j0 = 2 * half; j0 < nrp; j0 += kStep * kRefBatch) {
+                    float v[kRefBatch][2][8];
 #pragma unroll
-                    for (int q = 0; q < QT; q++) {
-                        float2 uv = make_float2(0.f, 0.f);
-                        if (j + jj < ring_num && q0 + q < grp.n_ref)
-                            uv = __ldg(&grp.ref_sp[((size_t)ref_row(grp, q0 + q) * ring_num + j + jj) * kSlots + k]);
-                        v[2 * q] = uv.x;
-                        v[2 * q + 1] = uv.y;
+                    for (unsigned i = 0; i < 2 * kRefBatch; i++) {
+                        const unsigned j = j0 + kStep * (i / 2) + i % 2;
+#pragma unroll
+                        for (int q = 0; q < QT; q++) {
+                            float2 uv = make_float2(0.f, 0.f);
+                            if (j < ring_num && rp[q])
+                                uv = __ldg(rp[q] + (size_t)j * kSlots);
+                            v[i / 2][i % 2][2 * q] = uv.x;
+                            v[i / 2][i % 2][2 * q + 1] = uv.y;
+                        }
                     }
-                    tmem_st8(tmem + (j + jj) * 8, v);
+#pragma unroll
+                    for (unsigned i = 0; i < 2 * kRefBatch; i++) {
+                        const unsigned j = j0 + kStep * (i / 2) + i % 2;
+                        if (j < nrp)
+                            tmem_st8(tmem + j * 8, v[i / 2][i % 2]);
+                    }
                 }
             }
             tmem_wait_st();
