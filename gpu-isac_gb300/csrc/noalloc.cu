@@ -7,7 +7,7 @@
 // after start-up), or code that must not pay the implicit device-wide
 // synchronisation cudaMalloc / cudaFree can cause in the middle of its stream
 // work.  They pass their inputs and outputs; the work space this pipeline
-// needs (the polar template, twiddles and shift tables, the reference
+// needs (the polar directions, twiddles and shift tables, the reference
 // spectra, and one chunk of particle spectra at a time) lives in one
 // file-scope device array built into the library.
 #include <cuda_runtime.h>
