@@ -3,12 +3,18 @@
 // (both K-major), converted to BF16 while they are staged, FP32 accumulate in
 // tensor memory, FP32 out.
 //
-// One CTA of 128 threads per 128 x 128 tile of C: for every 64-wide K slice
+// One CTA of 256 threads per 128 x 128 tile of C: for every 64-wide K slice
 // the threads stage A's and B's slices in shared memory in the canonical
 // no-swizzle K-major layout (8-row x 16-byte core matrices), one elected
 // thread issues four tcgen05.mma (K = 16 each) and commits them to an
-// mbarrier; the accumulator (128 lanes x 128 FP32 columns) is read back with
-// tcgen05.ld for the epilogue.
+// mbarrier, and the next slices are loaded into registers while these are
+// multiplied; the accumulator (128 lanes x 128 FP32 columns) is read back with
+// tcgen05.ld for the epilogue, four columns a store where C's rows allow it.
+// What bounds it: the loads' latency (the two layers and the scores of 4,000
+// particles at 49 shifts, M = 196,000: N x K = 256 x 560, 128 x 256, 200 x 128).
+// 681, 235, 256 us with 128 threads that loaded a slice, waited for its products
+// and stored C one column at a time; 355, 107, 109 us now (without the
+// bound of three CTAs 376, 114, 113; four, with spills, 447, 123, 126).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -20,6 +26,8 @@ namespace gpuisac {
 namespace {
 
 constexpr int kTM = 128, kTN = 128, kTK = 64;
+constexpr int kThreads = 256;
+constexpr int kPerThread = kTM * (kTK / 4) / kThreads; // float4 of a slice per thread
 constexpr uint32_t kTcCols = 128; // tensor-memory columns of the accumulator
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -67,19 +75,29 @@ __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity)
     return false;
 }
 
-// stage rows [r0, r0+128) x k [k0, k0+64) of X [rows][K] (pitch ld) as BF16;
-// rows / k beyond the matrix read zero
-__device__ __forceinline__ void stage_slice(unsigned char* dst, const float* __restrict__ X, long rows, int K,
+// rows [r0, r0+128) x k [k0, k0+64) of X [rows][K] (pitch ld), this thread's
+// quarter-rows of them; rows / k beyond the matrix read zero
+__device__ __forceinline__ void load_slice(float4 (&v)[kPerThread], const float* __restrict__ X, long rows, int K,
                                            long ld, long r0, int k0)
 {
-    for (int e = threadIdx.x; e < kTM * (kTK / 4); e += blockDim.x) {
-        const int row = e / (kTK / 4), kq = e % (kTK / 4);
+#pragma unroll
+    for (int i = 0; i < kPerThread; i++) {
+        const int e = threadIdx.x + i * kThreads, row = e / (kTK / 4), kq = e % (kTK / 4);
         const long gr = r0 + row;
         const int gk = k0 + 4 * kq;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (gr < rows && gk < K)
-            v = __ldg(reinterpret_cast<const float4*>(X + gr * ld + gk));
-        __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+            v[i] = __ldg(reinterpret_cast<const float4*>(X + gr * ld + gk));
+    }
+}
+
+// the same in shared memory as BF16
+__device__ __forceinline__ void store_slice(unsigned char* dst, const float4 (&v)[kPerThread])
+{
+#pragma unroll
+    for (int i = 0; i < kPerThread; i++) {
+        const int e = threadIdx.x + i * kThreads, row = e / (kTK / 4), kq = e % (kTK / 4);
+        __nv_bfloat162 lo = __floats2bfloat162_rn(v[i].x, v[i].y), hi = __floats2bfloat162_rn(v[i].z, v[i].w);
         uint2 packed;
         packed.x = *reinterpret_cast<uint32_t*>(&lo);
         packed.y = *reinterpret_cast<uint32_t*>(&hi);
@@ -87,7 +105,7 @@ __device__ __forceinline__ void stage_slice(unsigned char* dst, const float* __r
     }
 }
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kThreads, 3)
 gemm_tc_kernel(int M, int N, int K, float alpha, const float* __restrict__ A, long lda, const float* __restrict__ B,
                long ldb, const float* __restrict__ bias, int relu, float* __restrict__ C, long ldc,
                unsigned* __restrict__ err)
@@ -116,9 +134,12 @@ gemm_tc_kernel(int M, int N, int K, float alpha, const float* __restrict__ A, lo
 
     uint32_t phase = 0;
     bool ok = true;
+    float4 va[kPerThread], vb[kPerThread];
+    load_slice(va, A, M, K, lda, m0, 0);
+    load_slice(vb, B, N, K, ldb, n0, 0);
     for (int k0 = 0; k0 < K; k0 += kTK) {
-        stage_slice(sa, A, M, K, lda, m0, k0);
-        stage_slice(sb, B, N, K, ldb, n0, k0);
+        store_slice(sa, va);
+        store_slice(sb, vb);
         // the generic-proxy writes above become visible to the tensor cores
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
@@ -139,6 +160,10 @@ gemm_tc_kernel(int M, int N, int K, float alpha, const float* __restrict__ A, lo
                              saddr(&bar))
                          : "memory");
         }
+        if (k0 + kTK < K) {
+            load_slice(va, A, M, K, lda, m0, k0 + kTK);
+            load_slice(vb, B, N, K, ldb, n0, k0 + kTK);
+        }
         // the slices are read by the tensor cores until the commit lands
         ok = bar_wait(&bar, phase) && ok;
         phase ^= 1u;
@@ -148,11 +173,13 @@ gemm_tc_kernel(int M, int N, int K, float alpha, const float* __restrict__ A, lo
     if (!ok && tid == 0)
         atomicExch(err, 1u);
 
-    // epilogue: warp w holds rows 32w..32w+31 (lane = row), 16 columns per load
-    const long row = m0 + warp * 32 + lane;
-    const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
+    // epilogue: warp w holds rows 32 (w % 4) .. + 31 (lane = row) of one half of the
+    // columns, 16 per load
+    const long row = m0 + (warp & 3) * 32 + lane;
+    const uint32_t taddr = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const bool wide = ldc % 4 == 0 && ((uintptr_t)C & 15) == 0 && N % 4 == 0;
 #pragma unroll 1
-    for (int c0 = 0; c0 < kTN; c0 += 16) {
+    for (int c0 = (warp >> 2) * (kTN / 2), c1 = c0 + kTN / 2; c0 < c1; c0 += 16) {
         uint32_t r[16];
         asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
                      "%12, %13, %14, %15}, [%16];"
@@ -163,16 +190,27 @@ gemm_tc_kernel(int M, int N, int K, float alpha, const float* __restrict__ A, lo
                      : "memory");
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (row < M && K > 0) {
+            float v[16];
 #pragma unroll
             for (int i = 0; i < 16; i++) {
                 const long n = n0 + c0 + i;
-                if (n < N) {
-                    float v = alpha * __uint_as_float(r[i]);
-                    if (bias)
-                        v += bias[n];
-                    if (relu)
-                        v = fmaxf(v, 0.f);
-                    C[row * ldc + n] = v;
+                v[i] = alpha * __uint_as_float(r[i]);
+                if (bias && n < N)
+                    v[i] += bias[n];
+                if (relu)
+                    v[i] = fmaxf(v[i], 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < 16; i += 4) {
+                const long n = n0 + c0 + i;
+                if (wide) {
+                    if (n < N)
+                        *reinterpret_cast<float4*>(C + row * ldc + n) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                } else {
+#pragma unroll
+                    for (int h = 0; h < 4; h++)
+                        if (n + h < N)
+                            C[row * ldc + n + h] = v[i + h];
                 }
             }
         }
@@ -202,7 +240,7 @@ extern "C" int gpuisac_nn_gemm_bf16(int M, int N, int K, float alpha, const floa
     if ((M + kTM - 1) / kTM > 65535)
         return 2;
     dim3 grid((N + kTN - 1) / kTN, (M + kTM - 1) / kTM);
-    gemm_tc_kernel<<<grid, 128, 0, (cudaStream_t)stream>>>(M, N, K, alpha, A, lda, B, ldb, bias, relu, C, ldc, err);
+    gemm_tc_kernel<<<grid, kThreads, 0, (cudaStream_t)stream>>>(M, N, K, alpha, A, lda, B, ldb, bias, relu, C, ldc, err);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
