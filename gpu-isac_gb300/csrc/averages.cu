@@ -886,6 +886,7 @@ struct AvgState {
     Buf<double2> mean;
     Buf<float> partial;
     Buf<float2> scratch, tw;
+    std::vector<float2> h_tw;
     unsigned tw_dim = 0;
     unsigned* h_err = nullptr; // pinned
 } g_avg;
@@ -1031,11 +1032,14 @@ extern "C" int gpuisac_class_averages(const float* imgs, unsigned int n_img, uns
     if (!w.h_err)
         AV_CK(cudaMallocHost(&w.h_err, kErrWords * sizeof(unsigned)));
     if (w.tw_dim != D) {
-        std::vector<float2> tw(D);
+        // (read until the stream is synchronised below: kept in the state, copied on
+        // the caller's stream)
+        w.tw_dim = 0;
+        w.h_tw.resize(D);
         for (unsigned j = 0; j < D; j++)
-            tw[j] = make_float2((float)cos(2.0 * kPi * j / D), (float)sin(2.0 * kPi * j / D));
+            w.h_tw[j] = make_float2((float)cos(2.0 * kPi * j / D), (float)sin(2.0 * kPi * j / D));
         AV_CK(w.tw.ensure(D));
-        AV_CK(cudaMemcpy(w.tw.p, tw.data(), D * sizeof(float2), cudaMemcpyHostToDevice));
+        AV_CK(cudaMemcpyAsync(w.tw.p, w.h_tw.data(), D * sizeof(float2), cudaMemcpyHostToDevice, st));
         w.tw_dim = D;
     }
 

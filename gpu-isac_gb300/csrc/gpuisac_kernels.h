@@ -59,7 +59,7 @@ struct TexStack {
     size_t d_objs_n = 0;
     unsigned n = 0, dim = 0, batch = 0, tex = 0, n_batches = 0;
     int device = -1;
-    cudaError_t prepare(const StackDesc& st);
+    cudaError_t prepare(const StackDesc& st, cudaStream_t stream);
     cudaError_t fill(const StackDesc& st, cudaStream_t stream);
     cudaError_t build(const StackDesc& st, cudaStream_t stream);
     // build(), or -- when it fails (no memory for the copy, say) -- nothing:

@@ -428,13 +428,19 @@ extern "C" int gpuisac_multi_ref_align_groups_device(const AlignConfig* cfg, con
         h[5] = rows;
         h[6] = lut_first;
     }
-    G_CK(cudaMemcpy(S.tw.p, geo.tw.data(), kRingLen * sizeof(float2), cudaMemcpyHostToDevice));
-    G_CK(cudaMemcpy(S.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice));
-    G_CK(cudaMemcpy(S.shifts_f.p, geo.shifts_f.data(), Sn * sizeof(float2), cudaMemcpyHostToDevice));
-    G_CK(cudaMemcpy(S.shifts_i.p, geo.shifts_i.data(), Sn * sizeof(int2), cudaMemcpyHostToDevice));
+    // (uploads on the caller's stream: a copy on the legacy default stream may
+    // still be on its way when a kernel of a non-blocking stream reads)
     const int2 zero = make_int2(0, 0);
-    G_CK(cudaMemcpy(S.zero.p, &zero, sizeof(int2), cudaMemcpyHostToDevice));
-    G_CK(cudaMemcpy(dt, ht.data(), L.bytes, cudaMemcpyHostToDevice));
+    const StreamJoin join{st};
+    auto up = [&](void* dst, const void* src, size_t bytes) {
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    };
+    G_CK(up(S.tw.p, geo.tw.data(), kRingLen * sizeof(float2)));
+    G_CK(up(S.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2)));
+    G_CK(up(S.shifts_f.p, geo.shifts_f.data(), Sn * sizeof(float2)));
+    G_CK(up(S.shifts_i.p, geo.shifts_i.data(), Sn * sizeof(int2)));
+    G_CK(up(S.zero.p, &zero, sizeof(int2)));
+    G_CK(up(dt, ht.data(), L.bytes));
     S.stats.plan_ms = ms_since(t_call);
 
     // ---- the recorded sequence for this shape, or a new recording ----
@@ -512,8 +518,8 @@ extern "C" int gpuisac_multi_ref_align_groups_device(const AlignConfig* cfg, con
     G_CK(cudaMemsetAsync(S.err.p, 0, sizeof(unsigned), st));
     G_CK(cudaGraphLaunch(S.recs[ri].exec, st));
     g_kernel_launches.fetch_add(S.stats.graph_launches, std::memory_order_relaxed);
-    G_CK(cudaStreamSynchronize(st));
     unsigned flag = 0;
-    G_CK(cudaMemcpy(&flag, S.err.p, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    G_CK(cudaMemcpyAsync(&flag, S.err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    G_CK(cudaStreamSynchronize(st));
     return flag ? fail(1, "a kernel timed out waiting for its own asynchronous copies") : 0;
 }

@@ -21,6 +21,13 @@ struct NvtxRange {
     NvtxRange& operator=(const NvtxRange&) = delete;
 };
 
+// Synchronises a stream on every way out of a call, before the host memory goes
+// that copies on it may still read (declared after that memory).
+struct StreamJoin {
+    cudaStream_t stream;
+    ~StreamJoin() { cudaStreamSynchronize(stream); }
+};
+
 // Spectra held at a time by the sessions that run init / clear cycles
 // (pre-alignment, multigroup).
 constexpr size_t kSpectraBytes = (size_t)1 << 30;

@@ -59,6 +59,14 @@ struct Buf {
     }
 };
 
+// Copies of a call go through its own stream: one on the legacy default stream may
+// still be on its way when a kernel of a non-blocking stream reads, and does not
+// wait for what that stream writes.
+cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st)
+{
+    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+}
+
 struct PropState {
     std::mutex mu;
     Buf<float2> tw, dirs, shifts_f, ref_sp, sbj_sp;
@@ -107,17 +115,20 @@ extern "C" int gpuisac_align_proposals_device(const AlignConfig* cfg, const floa
     P_CK(S.ref_sp.ensure(row_elems * geo.R));
     P_CK(S.table.ensure(n_sel));
     const int2 zero = make_int2(0, 0);
-    P_CK(cudaMemcpy(S.tw.p, geo.tw.data(), kRingLen * sizeof(float2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.shifts_f.p, geo.shifts_f.data(), Sn * sizeof(float2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.shifts_i.p, geo.shifts_i.data(), Sn * sizeof(int2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.zero.p, &zero, sizeof(int2), cudaMemcpyHostToDevice));
+    std::vector<CcfGroup> table(n_sel);
+    const StreamJoin join{st};
+    P_CK(upload(S.tw.p, geo.tw.data(), kRingLen * sizeof(float2), st));
+    P_CK(upload(S.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), st));
+    P_CK(upload(S.shifts_f.p, geo.shifts_f.data(), Sn * sizeof(float2), st));
+    P_CK(upload(S.shifts_i.p, geo.shifts_i.data(), Sn * sizeof(int2), st));
+    P_CK(upload(S.zero.p, &zero, sizeof(int2), st));
     P_CK(cudaMemsetAsync(S.err.p, 0, sizeof(unsigned), st));
 
     // selected particles (host copy of the list, for the per-particle groups)
     std::vector<unsigned> sel(n_sel);
     if (part_idx) {
-        P_CK(cudaMemcpy(sel.data(), part_idx, n_sel * sizeof(unsigned), cudaMemcpyDeviceToHost));
+        P_CK(cudaMemcpyAsync(sel.data(), part_idx, n_sel * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        P_CK(cudaStreamSynchronize(st));
         for (unsigned i = 0; i < n_sel; i++)
             if (sel[i] >= geo.P)
                 return fail(2, "particle index outside the stack");
@@ -129,7 +140,8 @@ extern "C" int gpuisac_align_proposals_device(const AlignConfig* cfg, const floa
     // every proposal must name a reference of the stack (the kernels trust them)
     {
         std::vector<unsigned> prop((size_t)n_sel * k);
-        P_CK(cudaMemcpy(prop.data(), proposals, prop.size() * sizeof(unsigned), cudaMemcpyDeviceToHost));
+        P_CK(cudaMemcpyAsync(prop.data(), proposals, prop.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        P_CK(cudaStreamSynchronize(st));
         for (unsigned v : prop)
             if (v >= geo.R)
                 return fail(2, "proposal names a reference outside the stack");
@@ -145,7 +157,6 @@ extern "C" int gpuisac_align_proposals_device(const AlignConfig* cfg, const floa
 
     // one group per selected particle: 1 particle x its k references
     const unsigned tiles = (k + qt - 1) / qt;
-    std::vector<CcfGroup> table(n_sel);
     size_t free_b = 0, total_b = 0;
     P_CK(cudaMemGetInfo(&free_b, &total_b));
     const size_t per_part = row_elems * Sn * sizeof(float2);
@@ -187,9 +198,9 @@ extern "C" int gpuisac_align_proposals_device(const AlignConfig* cfg, const floa
         w.item_counter = S.err.p + 1;
         P_CK(launch_ccf_peak_work(w, variant, S.tw.p, NR, Sn, S.shifts_f.p, S.err.p, st));
     }
-    P_CK(cudaStreamSynchronize(st)); // the host table must outlive its copies
     unsigned flag = 0;
-    P_CK(cudaMemcpy(&flag, S.err.p, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    P_CK(cudaMemcpyAsync(&flag, S.err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    P_CK(cudaStreamSynchronize(st)); // (the host table and the uploads' sources must outlive their copies)
     return flag ? fail(1, "a kernel timed out waiting for its own asynchronous copies") : 0;
 }
 
@@ -316,11 +327,14 @@ extern "C" int gpuisac_learned_align_device(const AlignConfig* cfg, const float*
     P_CK(S.err.ensure(2)); // the timeout flag and the CCF kernel's work counter
     P_CK(S.ref_sp.ensure(row_elems * R));
     const int2 zero = make_int2(0, 0);
-    P_CK(cudaMemcpy(S.tw.p, geo.tw.data(), kRingLen * sizeof(float2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.shifts_f.p, geo.shifts_f.data(), Sn * sizeof(float2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.shifts_i.p, geo.shifts_i.data(), Sn * sizeof(int2), cudaMemcpyHostToDevice));
-    P_CK(cudaMemcpy(S.zero.p, &zero, sizeof(int2), cudaMemcpyHostToDevice));
+    std::vector<CcfGroup> table;
+    std::vector<unsigned> fbl;
+    const StreamJoin join{st};
+    P_CK(upload(S.tw.p, geo.tw.data(), kRingLen * sizeof(float2), st));
+    P_CK(upload(S.dirs.p, geo.dirs.data(), geo.dirs.size() * sizeof(float2), st));
+    P_CK(upload(S.shifts_f.p, geo.shifts_f.data(), Sn * sizeof(float2), st));
+    P_CK(upload(S.shifts_i.p, geo.shifts_i.data(), Sn * sizeof(int2), st));
+    P_CK(upload(S.zero.p, &zero, sizeof(int2), st));
     P_CK(cudaMemsetAsync(S.err.p, 0, sizeof(unsigned), st));
 
     // reference spectra for the search (reference basis, every reference)
@@ -363,8 +377,8 @@ extern "C" int gpuisac_learned_align_device(const AlignConfig* cfg, const float*
     StackDesc sbjs{sbj, P, D, geo.sbj_batch, tex};
     if (texture_unit_enabled())
         sbj_tx = S.sbj_tex.try_build(sbjs, st);
-    std::vector<CcfGroup> table(chunk);
-    std::vector<unsigned> flags(chunk), fbl;
+    table.resize(chunk);
+    std::vector<unsigned> flags(chunk);
     unsigned long long n_pairs = 0;
     float4* bparam = reinterpret_cast<float4*>(best_param);
     const unsigned tiles_k = (k + qt - 1) / qt, tiles_all = (R + qt - 1) / qt;
@@ -493,6 +507,7 @@ extern "C" int gpuisac_learned_align_device(const AlignConfig* cfg, const float*
     if (pairs)
         *pairs = n_pairs;
     unsigned flag = 0;
-    P_CK(cudaMemcpy(&flag, S.err.p, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    P_CK(cudaMemcpyAsync(&flag, S.err.p, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    P_CK(cudaStreamSynchronize(st));
     return flag ? fail(1, "a kernel timed out waiting for its own asynchronous copies") : 0;
 }

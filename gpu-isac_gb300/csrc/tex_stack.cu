@@ -269,11 +269,11 @@ const unsigned long long* TexStack::try_build(const StackDesc& st, cudaStream_t 
 
 cudaError_t TexStack::build(const StackDesc& st, cudaStream_t stream)
 {
-    cudaError_t e = prepare(st);
+    cudaError_t e = prepare(st, stream);
     return e != cudaSuccess ? e : fill(st, stream);
 }
 
-cudaError_t TexStack::prepare(const StackDesc& st)
+cudaError_t TexStack::prepare(const StackDesc& st, cudaStream_t stream)
 {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -314,7 +314,11 @@ cudaError_t TexStack::prepare(const StackDesc& st)
             return e;
         d_objs_n = n_seg;
     }
-    e = cudaMemcpy(d_objs, objs.data(), n_seg * sizeof(unsigned long long), cudaMemcpyHostToDevice);
+    // (on the stream whose kernels read them: a copy on the legacy default stream may
+    // still be on its way for a non-blocking one)
+    e = cudaMemcpyAsync(d_objs, objs.data(), n_seg * sizeof(unsigned long long), cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess)
+        e = cudaStreamSynchronize(stream);
     if (e != cudaSuccess)
         return e;
     n = st.n;
