@@ -451,12 +451,13 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
         const uint32_t row_bytes = ring_num * kSlots * sizeof(float2);
         // this half's part of the shift group of rows v0..v0+NSI-1 of stream t of
         // the item whose particles start at p0 and number np
-        const uint32_t wlim = wait_tries(w.wait_iters);
-        // returns whether copies were issued
-        auto issue = [&](const CcfGroup& gg, unsigned p0, unsigned np, unsigned t, unsigned v0) -> bool {
+        const uint32_t wlim = w.test_stall == kTestLate ? 0u : wait_tries(w.wait_iters);
+        unsigned issued = 0; // shift groups copied (lead thread): the n-th completes phase n of the barrier
+        auto issue = [&](const CcfGroup& gg, unsigned p0, unsigned np, unsigned t, unsigned v0) {
             const float2* sp = gg.sbj_sp;
-            if (w.test_stall)
-                return false;
+            if (w.test_stall == kTestStall)
+                return;
+            issued++;
             size_t at[SPT];
             bool in[SPT];
             unsigned nv = 0;
@@ -480,11 +481,9 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
                 if (in[i] && GPUISAC_IN_BOUNDS(kChkCcfRow, at[i] + (size_t)ring_num * kSlots - 1,
                                                (size_t)gg.n_part * n_shift * ring_num * kSlots))
                     bulk_g2s(sbuf + (size_t)(SPT * half + i) * nrp * kSlots, sp + at[i], row_bytes, bar);
-            return true;
         };
-        bool pending = false; // lead thread: copies in flight
         if (lead)
-            pending = issue(grp, pb, pe - pb, 0, 0);
+            issue(grp, pb, pe - pb, 0, 0);
         unsigned it = 0, ii = 0;
         while (true) {
             if (tid == 0)
@@ -542,8 +541,6 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
                     // ---- wait for this half's spectra (bounded) ----
                     if (!failed) {
                         const bool ok = mbar_wait(bar, phase, wlim);
-                        if (ok && lead)
-                            pending = false;
                         failed = !nbar_and(kWsBarCH + half, NCH, ok);
                     }
                     phase ^= 1u;
@@ -612,9 +609,9 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
                     tmem_fence_after();
                     if (lead && !failed) {
                         if (nj < ng0)
-                            pending = issue(grp, pb, np, nt, nj * NSI);
+                            issue(grp, pb, np, nt, nj * NSI);
                         else if (has_next)
-                            pending = issue(ngrp, npb, npe - npb, 0, 0);
+                            issue(ngrp, npb, npe - npb, 0, 0);
                     }
                     // ---- hand the pair spectra to the FFT side ----
                     float2* zb = zbuf + (size_t)b * NP * kPairStride;
@@ -653,8 +650,8 @@ ccf_peak_ws_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned ring_
         }
         if (failed && lead) {
             atomicExch(err, 1u);
-            if (pending)
-                mbar_wait(bar, phase, wlim); // let copies in flight land before leaving (bounded)
+            if (issued) // the half's last copies land before the CTA ends (bounded)
+                mbar_wait(bar, (issued - 1) & 1u);
         }
     } else {
         // ================= FFT / peak side =================
@@ -1145,5 +1142,11 @@ cudaError_t launch_ccf_peak(const float2* sbj_sp, const float2* ref_sp, const fl
 extern "C" void gpuisac_test_stall_ccf(unsigned int wait_iters)
 {
     gpuisac::g_test_wait_iters.store(wait_iters);
-    gpuisac::g_test_stall.store(wait_iters ? 1u : 0u);
+    gpuisac::g_test_stall.store(wait_iters ? gpuisac::kTestStall : 0u);
+}
+
+extern "C" void gpuisac_test_late_ccf(int on)
+{
+    gpuisac::g_test_wait_iters.store(on ? 64u : 0u);
+    gpuisac::g_test_stall.store(on ? gpuisac::kTestLate : 0u);
 }

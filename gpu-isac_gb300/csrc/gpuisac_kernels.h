@@ -250,9 +250,11 @@ struct CcfWork {
     unsigned ppc;     // particles per work item
     unsigned max_ref; // most references of any group (0: not known); 1 selects the one-reference contraction
     unsigned max_part; // most particles of any group (0: not known); 1 (or ppc = 1) selects the split-shift streams
-    // failure-path tests only (gpuisac_test_stall_ccf): the kernels that stage
-    // with bulk copies issue none, and their bounded waits give up after
-    // wait_iters tries (0: the default, about a second)
+    // failure-path tests only.  kTestStall (gpuisac_test_stall_ccf): the kernels
+    // that stage with bulk copies issue none, and their bounded waits give up
+    // after wait_iters tries (0: the default, about a second).  kTestLate
+    // (gpuisac_test_late_ccf): the warp-specialised kernel issues its copies and
+    // its waits for them give up without a try; the others stall.
     unsigned test_stall;
     unsigned wait_iters;
 };
@@ -263,6 +265,7 @@ struct CcfWork {
 void contraction_force(int mode);
 
 // the failure-path test settings every CCF launch carries (both 0 normally)
+enum : unsigned { kTestStall = 1, kTestLate = 2 };
 void ccf_test_settings(unsigned& stall, unsigned& wait_iters);
 
 enum { kCcfGeneral = 0, kCcfTmem = 1, kCcfWs = 2 };

@@ -49,7 +49,7 @@ EXPORTS = (
     "gpuisac_nn_softmax_xent", "gpuisac_nn_adam", "gpuisac_nn_topk", "gpuisac_nn_col_stats", "gpuisac_nn_loss_grad",
     "gpuisac_nn_affine_cols", "gpuisac_nn_group_max", "gpuisac_learned_align_device", "gpuisac_autotune_ccf",
     "gpuisac_ccf_tile_name", "gpuisac_nn_gemm_bf16", "gpuisac_assign_groups_device", "gpuisac_assign_groups",
-    "gpuisac_ref_free_averages", "gpuisac_set_contraction", "gpuisac_get_contraction", "gpuisac_test_stall_ccf", "gpuisac_normalize_mask",
+    "gpuisac_ref_free_averages", "gpuisac_set_contraction", "gpuisac_get_contraction", "gpuisac_test_stall_ccf", "gpuisac_test_late_ccf", "gpuisac_normalize_mask",
     "gpuisac_split_plan", "gpuisac_groups_stats", "gpuisac_checked_failures", "gpuisac_class_averages",
     "gpuisac_test_fail_alloc",
 )
@@ -209,6 +209,8 @@ def load(path: str | None = None) -> ctypes.CDLL:
     L.gpuisac_get_contraction.restype = ctypes.c_int
     L.gpuisac_test_stall_ccf.argtypes = [ctypes.c_uint]
     L.gpuisac_test_stall_ccf.restype = None
+    L.gpuisac_test_late_ccf.argtypes = [ctypes.c_int]
+    L.gpuisac_test_late_ccf.restype = None
     L.gpuisac_test_fail_alloc.argtypes = [ctypes.c_uint]
     L.gpuisac_test_fail_alloc.restype = None
     L.gpuisac_normalize_mask.argtypes = [ctypes.c_void_p, ctypes.c_uint, ctypes.c_uint, ctypes.c_void_p, ctypes.c_int,

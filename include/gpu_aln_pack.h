@@ -216,6 +216,10 @@ int gpuisac_multi_ref_align_device(const AlignConfig *cfg, const float *sbj, con
  * most 20 us, so that the call comes back with error code 1 ("timed out") and
  * the context stays usable; 0 restores normal operation. */
 void gpuisac_test_stall_ccf(unsigned int wait_iters);
+/* The same for copies that come too late: while on, the warp-specialised CCF
+ * kernel issues its copies and gives up each wait for them without a try, with
+ * the copies still in flight (the other kernels behave as stalled). */
+void gpuisac_test_late_ccf(int on);
 /* No counterpart in the reference (whose cudaMalloc failures exit the
  * process): failure-path tests only -- the next n device allocations of the
  * alignment's work space fail as if the device were out of memory, so that
