@@ -17,7 +17,8 @@
 //           threshold becomes the maxasi-th best pair key, and the rest are
 //           unplaced again;
 //   end:    when a round turns nobody away (every round and what follows run in one
-//           cooperative grid, up to 1,024 rounds a launch).  Every group then holds maxasi
+//           cooperative grid, up to 1,024 rounds a launch, or, where the steps are long,
+//           each step as a launch of its own).  Every group then holds maxasi
 //           particles; the one with the lowest threshold is the group the host
 //           algorithm closes last, and the leftover particles join it.
 // The result also comes out as the host function's list: each group's members
@@ -365,7 +366,7 @@ __device__ unsigned last_group(const Assign& a)
 // leftovers) at their rank.
 __device__ void rank_chunk(const Assign& a, unsigned g, unsigned chunk)
 {
-    __shared__ uint64_t tile[kThreads];
+    __shared__ ulonglong2 tile[kThreads / 2];
     const unsigned c = g < a.nref ? a.maxasi : a.extra;
     const unsigned base = g * a.maxasi, i = chunk * kThreads + threadIdx.x;
     const bool live = i < c;
@@ -373,76 +374,65 @@ __device__ void rank_chunk(const Assign& a, unsigned g, unsigned chunk)
     unsigned r = 0;
     for (unsigned j0 = 0; j0 < c; j0 += kThreads) {
         __syncthreads();
-        if (j0 + threadIdx.x < c)
-            tile[threadIdx.x] = a.bk[base + j0 + threadIdx.x];
+        reinterpret_cast<uint64_t*>(tile)[threadIdx.x] = j0 + threadIdx.x < c ? a.bk[base + j0 + threadIdx.x] : 0;
         __syncthreads();
-        const unsigned m = min(kThreads, c - j0);
+        const unsigned m = (min(kThreads, c - j0) + 1) / 2; // (a zero past the last is no larger key)
 #pragma unroll 8
-        for (unsigned j = 0; j < m; j++)
-            r += tile[j] > ki;
+        for (unsigned j = 0; j < m; j++) {
+            const ulonglong2 k = tile[j];
+            r += k.x > ki;
+            r += k.y > ki;
+        }
     }
     if (live)
         a.out[base + r] = (int)a.bp[base + i];
 }
 
-// The rounds and what follows them, in one cooperative grid that meets between
-// steps.  What bounds it: the meetings (four a round) and the steps' dependent
-// loads.  As four kernels a round with a read of the count after each, launches and
-// reads were most of the time: 20,000 particles x 200 groups (9 rounds) 376 us, now
-// 233; 3,000 x 76 (7) 274 -> 135; 300 x 7 (4) 179 -> 82; 100,000 x 500 (10) 661 ->
-// 579.  The count read after every third or fourth such round: 311 to 362 us.
-__global__ void __launch_bounds__(kThreads)
-assign_kernel(Assign a)
+// ---- the steps of a round, and of what follows the rounds; every CTA of the grid takes
+// its share ----
+
+// room for the members of the groups that received proposals, in any order
+__device__ void make_room(const Assign& a)
 {
     const unsigned t0 = blockIdx.x * kThreads + threadIdx.x, nt = gridDim.x * kThreads;
-    unsigned target = 0;
-    for (unsigned round = 0;; round++) {
-        const bool all = a.first && round == 0;
-        // (changed next after the meeting that follows the proposals)
-        const unsigned n = all ? a.nima : __ldcg(a.sc + kScNext);
-        if (n == 0)
-            break;
-        if (round == kMaxRounds)
-            return;
-        if (!all && n <= a.nima / kSparseDiv)
-            propose_listed(a, n);
-        else
-            propose_scan(a, all);
-        if (!grid_meet(a, target) || (__ldcg(a.sc + kScErr) & kErrNaN))
-            return;
-        // room for the members of the groups that received proposals, in any order
-        for (unsigned g = t0; g < a.nref; g += nt)
-            if (a.touched[g]) {
-                a.off[g] = atomicAdd(a.sc + kScTotal, a.cnt[g]);
-                a.fill[g] = 0;
-            }
-        if (t0 == 0) {
-            a.sc[kScNext] = 0;
-            a.sc[kScRounds]++;
+    for (unsigned g = t0; g < a.nref; g += nt)
+        if (a.touched[g]) {
+            a.off[g] = atomicAdd(a.sc + kScTotal, a.cnt[g]);
+            a.fill[g] = 0;
         }
-        if (!grid_meet(a, target))
-            return;
-        // the members, bucketed by group
-        for (unsigned p = t0; p < a.nima; p += nt) {
-            const int g = a.assign[p];
-            if (g >= 0 && a.touched[g]) {
-                const unsigned s = a.off[g] + atomicAdd(a.fill + g, 1u);
-                a.bp[s] = p;
-                a.bk[s] = a.pkey[p];
-            }
-        }
-        if (!grid_meet(a, target))
-            return;
-        if (t0 == 0)
-            a.sc[kScTotal] = 0;
-        for (unsigned g = blockIdx.x; g < a.nref; g += gridDim.x)
-            select_best(a, g);
-        if (!grid_meet(a, target))
-            return;
+    if (t0 == 0) {
+        a.sc[kScNext] = 0;
+        a.sc[kScRounds]++;
     }
+}
 
-    // belongsto; a leftover particle joins the last group (its pair key with that
-    // group ranks it among the leftovers) and is tagged with group index nref
+// their members, bucketed by group
+__device__ void bucket_members(const Assign& a)
+{
+    const unsigned t0 = blockIdx.x * kThreads + threadIdx.x, nt = gridDim.x * kThreads;
+    for (unsigned p = t0; p < a.nima; p += nt) {
+        const int g = a.assign[p];
+        if (g >= 0 && a.touched[g]) {
+            const unsigned s = a.off[g] + atomicAdd(a.fill + g, 1u);
+            a.bp[s] = p;
+            a.bk[s] = a.pkey[p];
+        }
+    }
+}
+
+__device__ void select_groups(const Assign& a)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        a.sc[kScTotal] = 0;
+    for (unsigned g = blockIdx.x; g < a.nref; g += gridDim.x)
+        select_best(a, g);
+}
+
+// belongsto; a leftover particle joins the last group (its pair key with that
+// group ranks it among the leftovers) and is tagged with group index nref
+__device__ void join_groups(const Assign& a)
+{
+    const unsigned t0 = blockIdx.x * kThreads + threadIdx.x, nt = gridDim.x * kThreads;
     const unsigned last = last_group(a);
     if (t0 == 0)
         a.sc[kScLast] = last;
@@ -459,10 +449,13 @@ assign_kernel(Assign a)
         if (a.belongsto)
             a.belongsto[p] = g;
     }
-    if (!a.out || !grid_meet(a, target))
-        return;
-    // members bucketed by final group: group g at g*maxasi, the leftovers at
-    // nref*maxasi
+}
+
+// members bucketed by final group: group g at g*maxasi, the leftovers at
+// nref*maxasi
+__device__ void bucket_final(const Assign& a)
+{
+    const unsigned t0 = blockIdx.x * kThreads + threadIdx.x, nt = gridDim.x * kThreads;
     for (unsigned p = t0; p < a.nima; p += nt) {
         const unsigned g = (unsigned)a.assign[p];
         const unsigned cap = g < a.nref ? a.maxasi : a.extra;
@@ -475,16 +468,108 @@ assign_kernel(Assign a)
         a.bp[s] = p;
         a.bk[s] = a.pkey[p];
     }
-    if (!grid_meet(a, target) || (__ldcg(a.sc + kScErr) & kErrInternal))
-        return;
+}
+
+__device__ void rank_members(const Assign& a)
+{
     const unsigned chunks = (a.maxasi + kThreads - 1) / kThreads, chunks_left = (a.extra + kThreads - 1) / kThreads;
     const unsigned long long items = (unsigned long long)a.nref * chunks + chunks_left;
     for (unsigned long long i = blockIdx.x; i < items; i += gridDim.x) {
         const unsigned g = (unsigned)min(i / chunks, (unsigned long long)a.nref);
         rank_chunk(a, g, (unsigned)(i - (unsigned long long)g * chunks));
     }
-    if (t0 == 0)
-        a.out[(size_t)a.nref * a.maxasi + a.extra] = (int)last;
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        a.out[(size_t)a.nref * a.maxasi + a.extra] = (int)a.sc[kScLast];
+}
+
+// The rounds and what follows them, in one cooperative grid that meets between
+// steps.  What bounds it: the meetings (four a round) and the steps' dependent
+// loads.  As four kernels a round with a read of the count after each, launches and
+// reads were most of the time: 20,000 particles x 200 groups (9 rounds) 376 us, now
+// 233; 3,000 x 76 (7) 274 -> 135; 300 x 7 (4) 179 -> 82; 100,000 x 500 (10) 661 ->
+// 579.  The count read after every third or fourth such round: 311 to 362 us.
+__global__ void __launch_bounds__(kThreads)
+assign_kernel(Assign a)
+{
+    unsigned target = 0;
+    for (unsigned round = 0;; round++) {
+        const bool all = a.first && round == 0;
+        // (changed next after the meeting that follows the proposals)
+        const unsigned n = all ? a.nima : __ldcg(a.sc + kScNext);
+        if (n == 0)
+            break;
+        if (round == kMaxRounds)
+            return;
+        if (!all && n <= a.nima / kSparseDiv)
+            propose_listed(a, n);
+        else
+            propose_scan(a, all);
+        if (!grid_meet(a, target) || (__ldcg(a.sc + kScErr) & kErrNaN))
+            return;
+        make_room(a);
+        if (!grid_meet(a, target))
+            return;
+        bucket_members(a);
+        if (!grid_meet(a, target))
+            return;
+        select_groups(a);
+        if (!grid_meet(a, target))
+            return;
+    }
+    join_groups(a);
+    if (!a.out || !grid_meet(a, target))
+        return;
+    bucket_final(a);
+    if (!grid_meet(a, target) || (__ldcg(a.sc + kScErr) & kErrInternal))
+        return;
+    rank_members(a);
+}
+
+// The same steps a launch each, with a read of the count after every round: a step
+// then has as many CTAs as it has work for, with the registers of its own code, where
+// the cooperative grid's two to four CTAs an SM (all steps' registers, every CTA in
+// every meeting) take many groups and tiles one after another.
+enum { kStepScan, kStepListed, kStepRoom, kStepBucket, kStepSelect, kStepJoin, kStepFinal, kStepRank };
+
+template <int STEP>
+__global__ void __launch_bounds__(kThreads)
+assign_step_kernel(Assign a, unsigned n)
+{
+    if constexpr (STEP == kStepScan)
+        propose_scan(a, a.first);
+    else if constexpr (STEP == kStepListed)
+        propose_listed(a, n);
+    else if constexpr (STEP == kStepRoom)
+        make_room(a);
+    else if constexpr (STEP == kStepBucket)
+        bucket_members(a);
+    else if constexpr (STEP == kStepSelect)
+        select_groups(a);
+    else if constexpr (STEP == kStepJoin)
+        join_groups(a);
+    else if constexpr (STEP == kStepFinal)
+        bucket_final(a);
+    else if (!(__ldcg(a.sc + kScErr) & kErrInternal))
+        rank_members(a);
+}
+
+// Whether the steps run as launches of their own.  Long reads: many pairs, or many
+// particles.  Many groups: a selection per group, unless the rounds place few
+// particles each, and a scan of all of them per tile, the more so when the
+// cooperative grid's CTAs have a second tile each.  us in all, cooperative grid / own
+// launches (random peaks, particles x groups):
+//   300,000 x 200   792 /   805    500,000 x 200 1,534 / 1,434  1,000,000 x 1,000 4,807 / 3,213
+//   300,000 x 100   836 /   882  1,000,000 x 100 3,507 / 3,227    600,000 x 50    2,581 / 2,468
+//    10,000 x 2,000 776 /   798     13,000 x 2,000   926 / 790     20,000 x 3,000 1,706 / 991
+//     9,000 x 3,000 1,074 / 1,173   11,750 x 2,500 1,626 / 1,010   40,000 x 40,000 35,457 / 27,163
+//     6,000 x 6,000 2,376 / 2,467   12,000 x 6,000 3,167 / 2,417
+//    50,000 x 1,000 673 /   755    100,000 x 1,000   937 / 876
+bool steps_apart(unsigned nref, unsigned nima, unsigned sms)
+{
+    const unsigned long long pairs = (unsigned long long)nref * nima;
+    const bool second_tile = nima > 32 * kCtasPerSm * sms;
+    return nima > 400000u || pairs > 80000000ull || (nref > 1000u && pairs > 36000000ull) ||
+           (nref >= 2000u && second_tile && pairs > 22000000ull);
 }
 
 template <typename T>
@@ -582,12 +667,29 @@ int assign_locked(const float* d, size_t pitch, unsigned nref, unsigned nima, in
     Assign a{d, pitch, nref, nima, maxasi, extra, true, belongsto, id_list_long, theta, w.pkey.p, w.bk.p,
              cnt, touched, w.off.p, w.fill.p, w.bp.p, w.list.p, sc, redo, w.assign.p, kWaitTries};
     const unsigned long long max_rounds = (unsigned long long)nref * nima + 1;
-    unsigned rounds = 0;
-    for (;;) {
-        void* args[] = {&a};
-        A_CK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(assign_kernel), dim3(grid), dim3(kThreads), args,
-                                         0, st));
+    unsigned rounds = 0, turned = nima;
+    const bool apart = steps_apart(nref, nima, (unsigned)sms);
+    auto step = [&](auto kernel, unsigned ctas, unsigned n) {
+        kernel<<<std::max(ctas, 1u), kThreads, 0, st>>>(a, n);
         g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    };
+    const unsigned per_particle = (nima + kThreads - 1) / kThreads;
+    for (;;) {
+        if (apart) {
+            if (!a.first && turned <= nima / kSparseDiv)
+                step(assign_step_kernel<kStepListed>, (turned + 7) / 8, turned);
+            else
+                step(assign_step_kernel<kStepScan>, tiles, 0);
+            step(assign_step_kernel<kStepRoom>, (nref + kThreads - 1) / kThreads, 0);
+            step(assign_step_kernel<kStepBucket>, per_particle, 0);
+            step(assign_step_kernel<kStepSelect>, nref, 0);
+            A_CK(cudaGetLastError());
+        } else {
+            void* args[] = {&a};
+            A_CK(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(assign_kernel), dim3(grid), dim3(kThreads),
+                                             args, 0, st));
+            g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+        }
         A_CK(cudaMemcpyAsync(w.h_sc, sc, kScCount * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
         A_CK(cudaStreamSynchronize(st));
         rounds = w.h_sc[kScRounds];
@@ -595,13 +697,24 @@ int assign_locked(const float* d, size_t pitch, unsigned nref, unsigned nima, in
             return fail(1, "assign_groups: a grid barrier timed out (bounded wait ran out)");
         if (w.h_sc[kScErr] & kErrNaN)
             return fail(2, "assign_groups: d holds a NaN peak");
-        const unsigned turned = w.h_sc[kScNext];
+        turned = w.h_sc[kScNext];
         if (turned == 0)
             break;
         if (turned > nima || rounds >= max_rounds)
             return fail(1, "assign_groups: the proposal rounds did not settle (internal error)");
         a.first = false;
-        A_CK(cudaMemsetAsync(sc + kScBar, 0, sizeof(unsigned), st));
+        if (!apart)
+            A_CK(cudaMemsetAsync(sc + kScBar, 0, sizeof(unsigned), st));
+    }
+    if (apart) {
+        step(assign_step_kernel<kStepJoin>, std::min(per_particle, 8u * (unsigned)sms), 0);
+        if (id_list_long) {
+            step(assign_step_kernel<kStepFinal>, per_particle, 0);
+            step(assign_step_kernel<kStepRank>, nref * ((maxasi + kThreads - 1) / kThreads) + 1, 0);
+        }
+        A_CK(cudaGetLastError());
+        A_CK(cudaMemcpyAsync(w.h_sc, sc, kScCount * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+        A_CK(cudaStreamSynchronize(st));
     }
     if ((w.h_sc[kScErr] & kErrInternal) || w.h_sc[kScLeft] != extra)
         return fail(1, "assign_groups: inconsistent group sizes (internal error)");
