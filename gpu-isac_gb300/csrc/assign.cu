@@ -55,7 +55,11 @@ constexpr unsigned kSparseDiv = 8;   // a round with at most nima / 8 particles 
 constexpr unsigned kCtasPerSm = 2, kCtasPerSmWide = 4;
 constexpr unsigned kWideTiles = 8; // tiles of 32 particles per SM from which on four
 constexpr unsigned kMaxRounds = 1024; // per launch (a launch goes on where the last one stopped)
-constexpr unsigned kWaitTries = 1u << 26; // of a grid barrier: tens of seconds
+// tries of a grid barrier's wait, 0.23 us each.  At the first meeting of a launch CTAs
+// may not have started (another stream's kernels hold their SMs): 15 seconds.  From then
+// on all run, and no step of a call that takes this form lasts more than milliseconds:
+// one second, as the other kernels' waits.
+constexpr unsigned kStartTries = 1u << 26, kWaitTries = 1u << 22;
 constexpr unsigned kErrNaN = 1u, kErrInternal = 2u, kErrWait = 4u;
 
 // kScNext: particles turned away; kScTotal: bucketed members of a round;
@@ -83,7 +87,8 @@ struct Assign {
     unsigned *cnt, *touched, *off, *fill, *bp, *list, *sc;
     unsigned char* redo;
     int* assign;
-    unsigned wait_tries;
+    unsigned start_tries, wait_tries;
+    unsigned stall; // failure-path tests only (gpuisac_test_stall_ccf): every meeting waits for one arrival too many
 };
 
 // All CTAs of the (cooperative) grid meet: what each wrote before is seen by all
@@ -96,15 +101,16 @@ __device__ bool grid_meet(const Assign& a, unsigned& target)
     target += gridDim.x;
     if (threadIdx.x == 0) {
         unsigned *bar = a.sc + kScBar, seen = 0, tries = 0;
+        const unsigned want = target + a.stall, limit = target == gridDim.x ? a.start_tries : a.wait_tries;
         __threadfence();
         atomicAdd(bar, 1u);
         while (true) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-            if ((int)(seen - target) >= 0 || ++tries > a.wait_tries)
+            if ((int)(seen - want) >= 0 || ++tries > limit)
                 break;
             __nanosleep(20);
         }
-        s_ok = (int)(seen - target) >= 0;
+        s_ok = (int)(seen - want) >= 0;
         if (!s_ok)
             atomicOr(a.sc + kScErr, kErrWait);
         __threadfence();
@@ -665,7 +671,11 @@ int assign_locked(const float* d, size_t pitch, unsigned nref, unsigned nima, in
     // no more CTAs than the widest step has work for
     const unsigned grid = std::min((unsigned)sms * std::min((unsigned)std::max(per_sm, 1), want), std::max(tiles, nref));
     Assign a{d, pitch, nref, nima, maxasi, extra, true, belongsto, id_list_long, theta, w.pkey.p, w.bk.p,
-             cnt, touched, w.off.p, w.fill.p, w.bp.p, w.list.p, sc, redo, w.assign.p, kWaitTries};
+             cnt, touched, w.off.p, w.fill.p, w.bp.p, w.list.p, sc, redo, w.assign.p, kStartTries, kWaitTries, 0};
+    unsigned test_stall = 0, test_tries = 0;
+    ccf_test_settings(test_stall, test_tries);
+    if (test_stall)
+        a.stall = 1, a.start_tries = a.wait_tries = test_tries;
     const unsigned long long max_rounds = (unsigned long long)nref * nima + 1;
     unsigned rounds = 0, turned = nima;
     const bool apart = steps_apart(nref, nima, (unsigned)sms);

@@ -214,7 +214,8 @@ int gpuisac_multi_ref_align_device(const AlignConfig *cfg, const float *sbj, con
  * kernels of the tensor-core contraction and the averaging step's sum kernel)
  * issue no copies and give up each bounded wait after wait_iters tries of at
  * most 20 us, so that the call comes back with error code 1 ("timed out") and
- * the context stays usable; 0 restores normal operation. */
+ * the context stays usable; the group assignment's cooperative grid waits at its
+ * barrier for an arrival that never comes, as often.  0 restores normal operation. */
 void gpuisac_test_stall_ccf(unsigned int wait_iters);
 /* The same for copies that come too late: while on, the warp-specialised CCF
  * kernel issues its copies and gives up each wait for them without a try, with
