@@ -117,7 +117,7 @@ extern "C" int gpuisac_autotune_ccf(const AlignConfig* cfg, const float* sbj, co
             ms = std::min(ms, t);
         }
         char b[96];
-        snprintf(b, sizeof(b), "%s%s %.3f ms", rep.empty() ? "" : "; ", tile_text(cand[i]).c_str(), ms);
+        snprintf(b, sizeof(b), "%s%s %.3f ms", rep.empty() ? "" : "; ", tile_text(ccf_tile_launched()).c_str(), ms);
         rep += b;
         if (ms < best_ms) {
             best_ms = ms;
@@ -134,5 +134,11 @@ extern "C" int gpuisac_autotune_ccf(const AlignConfig* cfg, const float* sbj, co
 extern "C" int gpuisac_ccf_tile_name(unsigned int ring_num, unsigned int n_shift, char* buf, size_t len)
 {
     copy_text(tile_text(ccf_tile(ring_num, n_shift, true)), buf, len);
+    return 0;
+}
+
+extern "C" int gpuisac_ccf_launched_name(char* buf, size_t len)
+{
+    copy_text(tile_text(ccf_tile_launched()), buf, len);
     return 0;
 }

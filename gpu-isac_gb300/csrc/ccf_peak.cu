@@ -945,6 +945,7 @@ std::mutex g_tile_mu;
 std::map<std::pair<unsigned, unsigned>, CcfTile> g_tiles;
 std::atomic<unsigned> g_tile_gen{0};
 thread_local const CcfTile* t_forced = nullptr;
+thread_local CcfTile t_launched{kCcfGeneral, 8, 0};
 } // namespace
 
 void ccf_tile_record(unsigned ring_num, unsigned n_shift, const CcfTile& t)
@@ -965,6 +966,8 @@ bool ccf_tile_lookup(unsigned ring_num, unsigned n_shift, CcfTile& t)
 }
 
 void ccf_tile_force(const CcfTile* t) { t_forced = t; }
+
+CcfTile ccf_tile_launched() { return t_launched; }
 
 bool ccf_tile_allows_tmem(unsigned ring_num) { return ring_num <= kTmaMaxRings; }
 
@@ -1045,27 +1048,26 @@ cudaError_t launch_ccf_peak_work(const CcfWork& w_in, int variant, const float2*
         if (e != cudaSuccess)
             return e;
     }
+    t_launched = CcfTile{variant, 8, w.ppc};
     if (variant == kCcfWs) {
-        const bool four = ccf_tile(ring_num, n_shift, true).ws_warps == 4;
         const bool one_ref = w.max_ref == 1;
+        const bool four = !one_ref && ccf_tile(ring_num, n_shift, true).ws_warps == 4;
+        // items of one particle: its shifts as the two streams (8 contraction
+        // warps; a tile of 4 keeps them)
+        const bool split = !one_ref && !four && (w.ppc == 1 || w.max_part == 1);
         cudaError_t e;
-        if (ring_num <= kTmaMaxRings) {
-            if (one_ref)
-                e = launch_ws<8, 4, 1>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
-            else if (w.ppc == 1 || w.max_part == 1)
-                e = launch_ws<8, 4, 4, true>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
-            else
-                e = four ? launch_ws<4, 4, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
-                         : launch_ws<8, 4, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
-        } else {
-            if (one_ref)
-                e = launch_ws<8, 2, 1>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
-            else if (w.ppc == 1 || w.max_part == 1)
-                e = launch_ws<8, 2, 4, true>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
-            else
-                e = four ? launch_ws<4, 2, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
-                         : launch_ws<8, 2, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
-        }
+        if (four)
+            t_launched.ws_warps = 4;
+        if (ring_num <= kTmaMaxRings)
+            e = one_ref ? launch_ws<8, 4, 1>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
+                : split ? launch_ws<8, 4, 4, true>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
+                : four  ? launch_ws<4, 4, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
+                        : launch_ws<8, 4, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
+        else
+            e = one_ref ? launch_ws<8, 2, 1>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
+                : split ? launch_ws<8, 2, 4, true>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
+                : four  ? launch_ws<4, 2, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream)
+                        : launch_ws<8, 2, 4>(w, grid, twiddle, ring_num, n_shift, shifts_f, err, stream);
         if (e != cudaSuccess)
             return e;
     } else if (variant == kCcfTmem) {
@@ -1093,9 +1095,12 @@ cudaError_t launch_ccf_peak_work(const CcfWork& w_in, int variant, const float2*
 
 // The tile's particles per work item, or fewer where that leaves items for less
 // than four rounds of the SMs (an 8 x 4 alignment is one item of 8 particles on
-// one SM otherwise: 145 us, 40 as 8 items).
+// one SM otherwise: 145 us, 40 as 8 items).  A tile that the autotuner forces is run
+// as it is: its candidates differ in this number.
 unsigned ccf_particles_per_item(const CcfTile& tile, size_t particle_tiles)
 {
+    if (t_forced)
+        return tile.ppc;
     const size_t share = particle_tiles / (4 * (size_t)persistent_grid(~0u, 1));
     return (unsigned)std::min<size_t>(tile.ppc, std::max<size_t>(1, share));
 }

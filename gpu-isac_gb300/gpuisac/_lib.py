@@ -48,7 +48,7 @@ EXPORTS = (
     "gpuisac_nn_relu_backward", "gpuisac_nn_colsum", "gpuisac_nn_l2norm", "gpuisac_nn_l2norm_backward",
     "gpuisac_nn_softmax_xent", "gpuisac_nn_adam", "gpuisac_nn_topk", "gpuisac_nn_col_stats", "gpuisac_nn_loss_grad",
     "gpuisac_nn_affine_cols", "gpuisac_nn_group_max", "gpuisac_learned_align_device", "gpuisac_autotune_ccf",
-    "gpuisac_ccf_tile_name", "gpuisac_nn_gemm_bf16", "gpuisac_assign_groups_device", "gpuisac_assign_groups",
+    "gpuisac_ccf_tile_name", "gpuisac_ccf_launched_name", "gpuisac_nn_gemm_bf16", "gpuisac_assign_groups_device", "gpuisac_assign_groups",
     "gpuisac_ref_free_averages", "gpuisac_set_contraction", "gpuisac_get_contraction", "gpuisac_test_stall_ccf", "gpuisac_test_late_ccf", "gpuisac_normalize_mask",
     "gpuisac_split_plan", "gpuisac_groups_stats", "gpuisac_checked_failures", "gpuisac_class_averages",
     "gpuisac_test_fail_alloc",
@@ -156,6 +156,8 @@ def load(path: str | None = None) -> ctypes.CDLL:
     L.gpuisac_autotune_ccf.restype = ci
     L.gpuisac_ccf_tile_name.argtypes = [cu, cu, ctypes.c_char_p, ctypes.c_size_t]
     L.gpuisac_ccf_tile_name.restype = ci
+    L.gpuisac_ccf_launched_name.argtypes = [ctypes.c_char_p, ctypes.c_size_t]
+    L.gpuisac_ccf_launched_name.restype = ci
     L.gpuisac_nn_affine_cols.argtypes = [vp, cl, ci, vp, vp, vp]
     L.gpuisac_nn_group_max.argtypes = [vp, cl, ci, ci, vp, vp]
     L.gpuisac_learned_align_device.argtypes = [aln_cfg_ptr, vp, vp, vp, ctypes.POINTER(GpuisacProposalNet), vp, cu,

@@ -323,3 +323,10 @@ def ccf_tile_name(ring_num: int, n_shift: int) -> str:
     buf = ctypes.create_string_buffer(64)
     _lib.load().gpuisac_ccf_tile_name(ring_num, n_shift, buf, len(buf))
     return buf.value.decode()
+
+
+def ccf_launched_name() -> str:
+    """The tile shape this thread's last CCF launch ran with."""
+    buf = ctypes.create_string_buffer(64)
+    _lib.load().gpuisac_ccf_launched_name(buf, len(buf))
+    return buf.value.decode()

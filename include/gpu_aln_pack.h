@@ -361,13 +361,17 @@ int gpuisac_learned_align_device(const AlignConfig *cfg, const float *sbj, const
  * through gpuisac_multi_ref_align_device and keeps the fastest for cfg's ring
  * count and shift count for the rest of the process; every candidate gives
  * bit-identical results.  report (optional) receives one line: each
- * candidate's time and the choice.  Blocks until done.  Returns 0 or an error
+ * candidate as it ran with its time, and the choice.  Blocks until done.  Returns 0 or an error
  * code. */
 int gpuisac_autotune_ccf(const AlignConfig *cfg, const float *sbj, const float *ref, unsigned int n_sample,
                          char *report, size_t report_len, void *stream);
 /* No counterpart in the reference.  The tile shape the CCF launches of this
  * ring count and shift count use, as text ("ws8/ppc8"). */
 int gpuisac_ccf_tile_name(unsigned int ring_num, unsigned int n_shift, char *buf, size_t len);
+/* The same text for the shape that the calling thread's last CCF launch ran
+ * with: a launch of few work items takes fewer particles per item than its
+ * tile names, one of a single reference 8 contraction warps. */
+int gpuisac_ccf_launched_name(char *buf, size_t len);
 
 /* ---- learned reference proposal (no counterpart in the reference): kernels
  * of a small embedding network, all on caller-owned row-major FP32 device
