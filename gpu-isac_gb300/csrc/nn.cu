@@ -357,6 +357,63 @@ __global__ void __launch_bounds__(256) gemm_kernel(const __grid_constant__ GemmG
     }
 }
 
+// One product with a short K and nothing added: 64 x 64 tiles, K steps of 16 through one
+// buffer, 4 x 4 outputs per thread, the same order of k.  There is no K loop to hide
+// behind, so what counts is how many tiles an SM has at a time: 48 registers and 9 KB
+// against 80 and 35, and no zeros summed up to a step of 32 or 64.
+constexpr int kShortT = 64, kShortK = 16;
+
+__global__ void __launch_bounds__(256)
+gemm_short_kernel(int M, int N, int K, float alpha, const float* __restrict__ A, long sam, long sak,
+                  const float* __restrict__ B, long sbk, long sbn, float beta, float* __restrict__ C, long ldc)
+{
+    __shared__ float As[kShortK][kShortT + 4];
+    __shared__ float Bs[kShortK][kShortT + 4];
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int m0 = (int)blockIdx.y * kShortT, n0 = (int)blockIdx.x * kShortT;
+    float acc[4][4] = {};
+    for (int k0 = 0; k0 < K; k0 += kShortK) {
+        for (int e = threadIdx.x; e < kShortK * kShortT; e += 256) {
+            const int kk = e / kShortT, o = e % kShortT, gk = k0 + kk;
+            As[kk][o] = m0 + o < M && gk < K ? A[(long)(m0 + o) * sam + (long)gk * sak] : 0.f;
+        }
+        for (int e = threadIdx.x; e < kShortK * kShortT; e += 256) {
+            const int kk = e / kShortT, o = e % kShortT, gk = k0 + kk;
+            Bs[kk][o] = n0 + o < N && gk < K ? B[(long)gk * sbk + (long)(n0 + o) * sbn] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int kk = 0; kk < kShortK; kk++) {
+            float a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                a[i] = As[kk][ty * 4 + i];
+                b[i] = Bs[kk][tx * 4 + i];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int gm = m0 + ty * 4 + i;
+        if (gm >= M)
+            continue;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int gn = n0 + tx * 4 + j;
+            if (gn >= N)
+                continue;
+            float* c = C + (long)gm * ldc + gn;
+            *c = alpha * acc[i][j] + (beta != 0.f ? beta * *c : 0.f);
+        }
+    }
+}
+
 // ---------------------------------------------------------------- elementwise
 // Y[i][j] += b[j]; optionally ReLU
 __global__ void bias_act_kernel(float* __restrict__ Y, const float* __restrict__ b, long rows, int cols, int relu)
@@ -540,6 +597,23 @@ cudaError_t launch_gemms(GemmGroup& g, cudaStream_t st)
     };
     int t = 64;
     long tiles = count(t);
+    // A product by itself with a short K: us here / in 64 x 64 tiles with two buffers,
+    // columns x K at 300,000 rows: 8 x 8 37 / 82, 200 x 16 164 / 290, 64 x 24 66 / 83,
+    // 64 x 32 114 / 89, 8 x 32 81 / 84, 64 x 40 94 / 118 (of its second 32 most are zeros),
+    // 8 x 48 91 / 113, 200 x 48 402 / 421, 8 x 64 142 / 118; small products to K = 16 13.9 /
+    // 15.0, 500 x 200 x 24 16.4 / 15.0.
+    const GemmProblem& p0 = g.p[0];
+    const int K = p0.part[0].K;
+    const bool plain = g.n == 1 && p0.part[1].K == 0 && !p0.bias && !p0.mask && !g.cs[0].dY && !g.cs[1].dY;
+    const int rows = (p0.M + kShortT - 1) / kShortT;
+    if (plain && rows <= 65535 &&
+        (K <= 16 || (tiles >= device_sms() && (K <= 24 || (K <= 48 && (K > 32 || p0.N <= 32)))))) {
+        const GemmPart& q = p0.part[0];
+        gemm_short_kernel<<<dim3((unsigned)p0.tiles_n, (unsigned)rows), 256, 0, st>>>(
+            p0.M, p0.N, K, p0.alpha, q.A, q.sam, q.sak, q.B, q.sbk, q.sbn, p0.beta, p0.C, p0.ldc);
+        g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+        return cudaGetLastError();
+    }
     if (tiles < device_sms())
         tiles = count(t = 32);
     long grid = tiles;
