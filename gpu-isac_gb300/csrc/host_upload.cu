@@ -31,10 +31,14 @@
 namespace gpuisac {
 namespace {
 
-// (16 MB of pinned memory for 16 workers: pinning costs about 35 us a MB, and
-// gpu_clear gives it back, so every init / clear cycle pays for it; with 2 MB
-// slots it was 2.1 ms of an alignment of 2,000 particles)
-constexpr size_t kSlotBytes = 512u << 10;
+// Bytes a worker stages at a time (two slots each).  Pinning costs about 35 us a MB, and
+// gpu_clear gives it back, so every init / clear cycle pays for it: small uploads take
+// 16 MB for 16 workers, large ones 32, whose fewer and longer copies are worth more.
+// Session init (device memory, pinning and upload), ms, with slots of 512 KB / 1 MB / 2 MB:
+// 92 MB 2.66 / 2.98 / 4.08, 231 MB 4.50 / 4.42 / 5.49, 1.16 GB 15.85 / 13.80 / 14.78, 2.3 GB
+// 29.7 / 25.6 / 26.1.
+constexpr size_t kSlotBytes = 512u << 10, kLargeSlotBytes = 1u << 20;
+constexpr size_t kLargeUpload = (size_t)256 << 20;
 constexpr unsigned kMaxWorkers = 16;
 
 struct Staging {
@@ -81,12 +85,13 @@ cudaError_t upload_host_images(const float* const* imgs, unsigned n, size_t img_
         (void)cudaGetLastError(); // pageable pointers may report an error on older drivers
     }
 
-    const size_t n_pieces = (total + kSlotBytes - 1) / kSlotBytes;
+    const size_t slot_bytes = total < kLargeUpload ? kSlotBytes : kLargeSlotBytes;
+    const size_t n_pieces = (total + slot_bytes - 1) / slot_bytes;
     unsigned hw = std::thread::hardware_concurrency();
     const unsigned T = (unsigned)std::min<size_t>(std::min(kMaxWorkers, std::max(1u, hw)), n_pieces);
 
     std::lock_guard<std::mutex> lk(g_stage.mu);
-    const size_t need = (size_t)2 * T * kSlotBytes;
+    const size_t need = (size_t)2 * T * slot_bytes;
     if (g_stage.bytes < need) {
         if (g_stage.h)
             cudaFreeHost(g_stage.h);
@@ -120,9 +125,9 @@ cudaError_t upload_host_images(const float* const* imgs, unsigned n, size_t img_
         size_t k = 0;
         for (size_t p = t; p < n_pieces && first_err.load(std::memory_order_relaxed) == 0; p += T, k++) {
             const unsigned slot = 2 * t + (unsigned)(k & 1);
-            unsigned char* stage = g_stage.h + (size_t)slot * kSlotBytes;
+            unsigned char* stage = g_stage.h + (size_t)slot * slot_bytes;
             cudaError_t r = cudaEventSynchronize(ev[slot]); // the slot's previous copy has left
-            const size_t x0 = p * kSlotBytes, x1 = std::min(total, x0 + kSlotBytes);
+            const size_t x0 = p * slot_bytes, x1 = std::min(total, x0 + slot_bytes);
             if (r == cudaSuccess) {
                 for (size_t x = x0; x < x1;) {
                     const size_t i = x / bytes, within = x - i * bytes;
