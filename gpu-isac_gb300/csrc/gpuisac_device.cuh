@@ -375,9 +375,9 @@ __device__ __forceinline__ void ifft256_two(Cx2 (&x)[16], void* ws, const float2
 // The division by N is Markstein's (P. Markstein, "Computation of elementary
 // functions on the IBM RISC System/6000 processor", 1990): with y = RN(1 / N)
 // and q0 = RN(m y), the remainder e = m - q0 N is exact in an FMA and
-// RN(q0 + e y) is the correctly rounded m / N -- checked for every 24-bit m
-// and every N up to the largest ring count (tests/test_ring_offsets.py holds
-// the template's own values).
+// RN(q0 + e y) is the correctly rounded m / N: tests/test_ring_division.py for
+// every 24-bit m and every N up to the largest ring count,
+// tests/test_ring_offsets.py for the template's own values.
 struct RingScale {
     float2 n, neg_n, y; // (N, N), (-N, -N), (RN(1 / N), RN(1 / N))
     __device__ __forceinline__ explicit RingScale(unsigned ring_num)
