@@ -634,6 +634,7 @@ int check_args(const float* d, unsigned long long pitch, unsigned nref, unsigned
         return fail(2, "assign_groups: nref * nima must stay below 2^32");
     if (pitch < nima)
         return fail(2, "assign_groups: d_pitch smaller than nima");
+    // (the list ranks members by comparing all of a group with all: 40 s at that size)
     if ((nima / nref + kThreads - 1) / kThreads > 65535u)
         return fail(2, "assign_groups: groups of more than 16,776,960 particles");
     return 0;

@@ -647,7 +647,6 @@ bool split_plan(unsigned ring_num, unsigned n_shift, unsigned n_ref, SplitPlan& 
     p.zw = p.block | 1u; // odd row length: the FFT's column reads hit distinct banks
     p.kg = (ring_num + 7) / 8;
     p.rga = (2 * p.block + 7) / 8;
-    p.rounds = 1;
     p.fft_groups = zfft_groups(p.block);
     const size_t cap = std::min<size_t>((size_t)smem_optin_max(), 227 * 1024);
     // references per tile: as many as N = 2 x refs <= 256 allows with at

@@ -74,6 +74,8 @@ Carve carve(const HostGeometry& g)
     c.off_tw = c.off_err + 256;
     c.off_zero = c.off_tw + up256(kRingLen * sizeof(float2));
     c.off_dirs = c.off_zero + up256(sizeof(int2));
+    // (room for every ring's offsets, of which the directions of one are used: the
+    // workloads that fit, and those refused, stay the ones callers have planned for)
     c.off_sf = c.off_dirs + up256((size_t)g.NR * kRingLen * sizeof(float2));
     c.off_si = c.off_sf + up256((size_t)g.S * sizeof(float2));
     c.off_ref = c.off_si + up256((size_t)g.S * sizeof(int2));
