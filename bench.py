@@ -928,11 +928,10 @@ def precision_vs_fp64(dev, n=256, R=200):
 
 
 def spectra_roofline(w, P, steps, spec_ms, spec_launches, hbm_peak, peak_kind, out_bytes_per_row):
-    """resample + FFT stage: images read once per shift row, spectra (or
-    operands) written"""
+    """resample + FFT stage: images read once, spectra (or operands) written"""
     S = w["n_shifts"]
     spec_avg_ms = spec_ms / max(spec_launches, 1)
-    spec_bytes = (P * w["img_dim"] ** 2 * 4 * S + P * S * out_bytes_per_row) * steps / max(spec_launches, 1)
+    spec_bytes = (P * w["img_dim"] ** 2 * 4 + P * S * out_bytes_per_row) * steps / max(spec_launches, 1)
     return {"avg_launch_ms": spec_avg_ms, "bytes_per_launch": spec_bytes,
             "achieved_gbs": spec_bytes / (spec_avg_ms / 1000.0) / 1e9 if spec_avg_ms else None,
             "hbm_peak_gbs": hbm_peak, "hbm_peak_kind": peak_kind}

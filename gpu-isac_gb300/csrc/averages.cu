@@ -914,7 +914,7 @@ int fail(int code, const char* msg)
     } while (0)
 
 // The sum kernel: images up to side 80 by CTAs of ceil(D / 8) warps with 20 rows a
-// thread, three to an SM; larger ones with 16 rows a thread and two row groups (one
+// thread, two to an SM at side 76 (96 registers); larger ones with 16 rows a thread and two row groups (one
 // pass) up to side 128, one group above.
 constexpr unsigned kSumSmall = 80;
 unsigned sum_groups(unsigned D) { return D <= kSumSmall || D > 128 ? 1 : 2; }

@@ -307,8 +307,8 @@ ccf_peak_tmem_kernel(CcfWork w, const float2* __restrict__ twiddle, unsigned rin
 // pair spectra through two shared-memory buffers guarded by named barriers
 // (FULL: contraction -> FFT, EMPTY: FFT -> contraction).
 //
-// What bounds it: issue and FMA throughput of the CUDA cores (issue 62 %, FMA
-// pipe 52 %; scalar FMAs on three distinct registers reach 97 of 128 per cycle
+// What bounds it: issue and FMA throughput of the CUDA cores (issue 69 %, FMA
+// pipe 59 %; scalar FMAs on three distinct registers reach 97 of 128 per cycle
 // and SM at best), 3,000 x 200 at 35 rings and 49 shifts: contraction alone
 // 25.5 ms, FFT side alone 19.8, without the copies 32.7, all of it 33.8 (37.4
 // with one team transforming one reference per group and the contraction side

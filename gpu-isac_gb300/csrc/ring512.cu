@@ -207,10 +207,10 @@ polar_spectra512_kernel(StackDesc st, const float2* __restrict__ dirs, const flo
 // stages deep.  Sums run ring by ring in order.
 //
 // What bounds it: FP32 FMA issue (62.5k FMA a pair at 61 rings; the FMA pipe is
-// active 56 % of the cycles, two warps a scheduler, one packed FMA per two
-// cycles) beside shared memory at 12 x 8 bytes per 128 FMAs and thread.  The row is 125 KB at 61 rings, too large to keep a reference
-// and a shift group on the SM with the pairs' spectra as the 256-sample kernel
-// does; one CTA per (particle, reference), re-reading every shift row for each
+// active 60 % of the cycles, issue 56 %, two warps a scheduler, one packed FMA
+// per two cycles) beside shared memory at 12 x 8 bytes per 128 FMAs and thread.
+// The row is 125 KB at 61 rings, too large to keep a reference and a shift group
+// on the SM with the pairs' spectra as the 256-sample kernel does; one CTA per (particle, reference), re-reading every shift row for each
 // reference with four accumulators a thread, was bound by the latency of those
 // reads (issue 13 %).  Contraction, FFT and search of 300 x 60 pairs, 61
 // rings, 25 shifts: 13.4 -> 2.15 ms; 100 x 200, 81 shifts: 41.0 -> 7.2 ms.
